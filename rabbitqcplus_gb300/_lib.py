@@ -38,6 +38,7 @@ GPU_CU_SOURCES = [
     "k_store.cu",
     "k_tables.cu",
     "k_sort.cu",
+    "k_align.cu",
     "k_correct.cu",
     "k_learned.cu",
     "care_capi.cu",

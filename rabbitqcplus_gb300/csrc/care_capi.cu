@@ -188,8 +188,8 @@ struct GraphSig {
 
 // One batch pipeline of the batched driver: its buffers, stream and graph.
 struct BatchSet {
-    DevBuf rawCount, cand, ncand, paired, aln, fid, fshift, forient, fweight, flen, nfinal, uoff, scanTmp, cursor,
-        work, colFeat, colMeta, colCount, order, orderScratch, bigScratch, perm;
+    DevBuf rawCount, cand, ncand, paired, aln, fid, fshift, forient, fweight, flen, nfinal, cursor, work, colFeat,
+        colMeta, colCount, order, orderScratch, bigScratch, units;
     cudaStream_t stream = nullptr;
     cudaEvent_t joined = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -201,8 +201,7 @@ struct BatchSet {
         if (joined) cudaEventDestroy(joined);
         joined = nullptr;
         for (DevBuf* b : {&rawCount, &cand, &ncand, &paired, &aln, &fid, &fshift, &forient, &fweight, &flen, &nfinal,
-                          &uoff, &scanTmp, &cursor, &work, &colFeat, &colMeta, &colCount, &order, &orderScratch,
-                          &bigScratch, &perm})
+                          &cursor, &work, &colFeat, &colMeta, &colCount, &order, &orderScratch, &bigScratch, &units})
             b->release();
         if (stream) cudaStreamDestroy(stream);
         stream = nullptr;
@@ -229,7 +228,7 @@ struct cg_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    cudaEvent_t st0 = nullptr, st1 = nullptr, st1b = nullptr, st2 = nullptr, st3 = nullptr;  // stage boundaries
+    cudaEvent_t st0 = nullptr, st1 = nullptr, st2 = nullptr, st3 = nullptr;  // stage boundaries
     std::string err;
 
     // appended reads, one device chunk per cg_append_reads call (uploaded by
@@ -248,10 +247,6 @@ struct cg_ctx {
     uint64_t n = 0;
     int lmax = 0, pitch = 0, wp = 0, k = 20, nmaps = 48, maxValuesPerKey = 75;
     DevBuf enc, len, hilo, qual, ambig, sig;
-    // strand bits of every read's minima in maps 0-15 (u16 [N]) and the read
-    // ids in those maps' buckets tagged with them: fewer than 2^31 reads
-    DevBuf strand;
-    bool strandTags = false;
     std::vector<MapTable> maps;    // views into tableSlabs
     std::vector<DevBuf> tableSlabs;
     TablesArg tables{};
@@ -263,9 +258,10 @@ struct cg_ctx {
 
     // batch buffers
     DevBuf qrange, rawCount, cand, ncand, paired, aln, fid, fshift, forient, fweight, flen, nfinal, flags, out, counters;
-    DevBuf scanTmp, uoff, msaOrder, orderScratch, bigScratch, perm, lenRange, laneWork;
+    DevBuf scanTmp, msaOrder, orderScratch, bigScratch, units, lenRange;
     uint32_t* hPinned = nullptr;  // 2 words: total raw, max raw
-    bool lenVaries = false;       // reads of different lengths: candidates aligned in length order
+    unsigned long long* hCounters = nullptr;  // pinned copy of the counters (read_counters)
+    bool lenVaries = false;       // reads of different lengths
 
     // batched driver
     BatchSet sets[kMaxSets];
@@ -281,7 +277,8 @@ struct cg_ctx {
     bool haveMlp = false;
     bool collecting = false;  // cg_get_columns: record the columns, do not score them
     float minLogit = 0.0f;    // logit of threshold_anchor
-    unsigned long long timeoutsSeen = 0;  // classifier blocks whose MMA wait ran out, already reported
+    // alignment and classifier blocks whose tensor-core wait ran out, already reported
+    unsigned long long alignTimeoutsSeen = 0, timeoutsSeen = 0;
 
     // forest classifier (CG_CORR_FOREST)
     DevBuf forestNodes, treeOffsets;
@@ -431,7 +428,7 @@ int build_store(cg_ctx* c) {
     const int lmax = c->appendLmax;
     c->lmax = std::max(lmax, 1);
     c->pitch = (c->lmax + 15) / 16;
-    c->wp = (c->lmax + 31) / 32 + 1;
+    c->wp = align_plane_words(align_words(c->lmax));
     c->k = c->o.kmerlength == 0 ? (lmax < 160 ? 20 : 32) : c->o.kmerlength;  // dispatch_care_correct_cpu.cpp:81-95
     c->nmaps = c->o.num_hash_functions;
     {
@@ -446,7 +443,7 @@ int build_store(cg_ctx* c) {
     CG_CUDA(c, c->enc.ensure(n * c->pitch * sizeof(uint32_t)));
     CG_CUDA(c, c->len.ensure(n * sizeof(uint16_t)));
     CG_CUDA(c, c->ambig.ensure(n));
-    CG_CUDA(c, c->hilo.ensure(n * 4 * (uint64_t)c->wp * sizeof(uint32_t)));
+    CG_CUDA(c, c->hilo.ensure(n * 2 * (uint64_t)c->wp * sizeof(uint32_t)));
     if (q) CG_CUDA(c, c->qual.ensure(n * (uint64_t)c->lmax));
     CG_CUDA(c, cudaMemsetAsync(c->enc.p, 0, n * c->pitch * sizeof(uint32_t), c->stream));
     if (q) CG_CUDA(c, cudaMemsetAsync(c->qual.p, 0, n * (uint64_t)c->lmax, c->stream));
@@ -492,13 +489,7 @@ int build_tables(cg_ctx* c) {
     const uint64_t n = c->n;
     CG_CUDA(c, c->sig.ensure(n * c->nmaps * sizeof(unsigned long long)));
     StoreArg st = store_arg(c);
-    c->strandTags = n <= 0x7fffffffull;
-    uint16_t* strand = nullptr;
-    if (c->strandTags) {
-        CG_CUDA(c, c->strand.ensure((size_t)n * sizeof(uint16_t)));
-        strand = c->strand.as<uint16_t>();
-    }
-    CG_CUDA(c, launch_signatures(st, c->k, c->nmaps, c->sig.as<unsigned long long>(), strand, c->stream));
+    CG_CUDA(c, launch_signatures(st, c->k, c->nmaps, c->sig.as<unsigned long long>(), c->stream));
     if (n > 0x40000000ull) return fail(c, CG_ERR_UNSUPPORTED, "too many reads for one table (%llu)",
                                        (unsigned long long)n);
     // The maps are built in waves of up to kTableStreams maps, one stream and
@@ -572,7 +563,7 @@ int build_tables(cg_ctx* c) {
             const unsigned long long* keys = c->sig.as<unsigned long long>() + (uint64_t)h * n;
             cudaError_t e = radix_sort_pairs(keys, n, bits, l.keys.as<unsigned long long>(), l.ids.as<uint32_t>(),
                                              l.keysAlt.as<unsigned long long>(), l.idsAlt.as<uint32_t>(),
-                                             l.sortTmp.p, l.stream, h < 16 ? strand : nullptr, h);
+                                             l.sortTmp.p, l.stream);
             if (e == cudaSuccess) e = launch_run_heads(l.keys.as<unsigned long long>(), n, l.runOf.as<uint32_t>(),
                                                        l.stream);
             if (e == cudaSuccess) e = scan_exclusive_u32(l.runOf.as<uint32_t>(), n + 1, l.scanTmp.p, l.stream);
@@ -625,8 +616,7 @@ int build_tables(cg_ctx* c) {
                                                       l.runOf.as<uint32_t>(), l.start.as<uint32_t>(),
                                                       hRuns[h], l.packed.as<unsigned long long>(),
                                                       c->maxValuesPerKey, mt.values, mt.slots,
-                                                      (uint32_t)(mt.cap - 1), l.stream, rawAll,
-                                                      strand ? 0x7fffffffu : 0xffffffffu);
+                                                      (uint32_t)(mt.cap - 1), l.stream, rawAll);
             if (!cuda(e, "build")) break;
             c->stats.table_keys += mt.keys;
             c->stats.table_values += mt.nvalues;
@@ -655,9 +645,17 @@ int build_tables(cg_ctx* c) {
     CG_CUDA(c, e);
     c->tables.nmaps = c->nmaps;
     c->tables.maxValuesPerKey = c->maxValuesPerKey;
-    c->tables.strand = strand;
     return CG_OK;
 }
+
+int sm_count(cg_ctx* c) {
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess) sms = 1;
+    return std::max(sms, 1);
+}
+
+// units a batch of `count` anchors and `raw` raw ids can have
+size_t unit_slots(int count, uint64_t raw) { return (size_t)count + raw / kAlignUnit + 1; }
 
 BatchArg batch_arg(cg_ctx* c, uint64_t first, int count) {
     BatchArg b{};
@@ -677,8 +675,9 @@ BatchArg batch_arg(cg_ctx* c, uint64_t first, int count) {
     b.fweight = c->fweight.as<float>();
     b.flen = c->flen.as<uint16_t>();
     b.nfinal = c->nfinal.as<uint32_t>();
-    b.perm = c->lenVaries || c->strandTags ? c->perm.as<uint32_t>() : nullptr;
-    b.lenOrder = c->lenVaries;
+    b.units = c->units.as<uint2>();
+    b.unitCursor = b.rawCount + count + 2;  // cleared with the raw counts
+    b.unitCount = b.rawCount + count + 3;
     b.flags = c->flags.as<uint8_t>();
     b.out = c->out.as<char>();
     b.outPitch = c->lmax;
@@ -718,10 +717,11 @@ int run_candidates(cg_ctx* c, uint64_t first, int count) {
     const StoreArg st = store_arg(c);
     CG_CUDA(c, cudaEventRecord(c->st0, c->stream));
     CG_CUDA(c, c->qrange.ensure((size_t)count * c->nmaps * sizeof(uint2)));
-    CG_CUDA(c, c->rawCount.ensure((size_t)(count + 2) * sizeof(uint32_t)));
+    CG_CUDA(c, c->rawCount.ensure((size_t)(count + 4) * sizeof(uint32_t)));
     CG_CUDA(c, c->ncand.ensure((size_t)count * sizeof(uint32_t)));
+    CG_CUDA(c, c->nfinal.ensure((size_t)count * sizeof(uint32_t)));
     CG_CUDA(c, c->scanTmp.ensure(scan_tmp_bytes(count + 1)));
-    CG_CUDA(c, cudaMemsetAsync(c->rawCount.p, 0, (size_t)(count + 2) * sizeof(uint32_t), c->stream));
+    CG_CUDA(c, cudaMemsetAsync(c->rawCount.p, 0, (size_t)(count + 4) * sizeof(uint32_t), c->stream));
     BatchArg b = batch_arg(c, first, count);
     CG_CUDA(c, launch_query_count(st, c->tables, c->params, b, c->stream));
     CG_CUDA(c, scan_exclusive_u32(b.rawCount, (size_t)count + 1, c->scanTmp.p, c->stream));
@@ -733,7 +733,7 @@ int run_candidates(cg_ctx* c, uint64_t first, int count) {
     const uint32_t maxRaw = c->hPinned[1];
     const size_t cap = std::max<uint64_t>(total, 1);
     CG_CUDA(c, c->cand.ensure(cap * sizeof(uint32_t)));
-    if (c->lenVaries || c->strandTags) CG_CUDA(c, c->perm.ensure(cap * sizeof(uint32_t)));
+    CG_CUDA(c, c->units.ensure(unit_slots(count, total) * sizeof(uint2)));
     CG_CUDA(c, c->paired.ensure(cap));
     CG_CUDA(c, c->aln.ensure(cap * sizeof(uint2)));
     CG_CUDA(c, c->fid.ensure(cap * sizeof(uint32_t)));
@@ -754,7 +754,6 @@ int run_batch(cg_ctx* c, uint64_t first, int count, uint8_t* hFlags, char* hOut,
     int rc = run_candidates(c, first, count);
     if (rc != CG_OK) return rc;
     const StoreArg st = store_arg(c);
-    CG_CUDA(c, c->nfinal.ensure((size_t)count * sizeof(uint32_t)));
     CG_CUDA(c, c->flags.ensure((size_t)count));
     CG_CUDA(c, c->out.ensure((size_t)count * c->lmax));
     const bool learned = c->params.correctionType == CG_CORR_LEARNED;
@@ -771,23 +770,10 @@ int run_batch(cg_ctx* c, uint64_t first, int count, uint8_t* hFlags, char* hOut,
         CG_CUDA(c, launch_pair_flags(b, c->stream));
         c->stats.kernel_launches += 1;
     }
-    // dense candidate numbering for the thread-per-candidate alignment
-    CG_CUDA(c, c->uoff.ensure((size_t)(count + 1) * sizeof(uint32_t)));
-    CG_CUDA(c, cudaMemsetAsync(c->uoff.as<uint32_t>() + count, 0, sizeof(uint32_t), c->stream));
-    CG_CUDA(c, cudaMemcpyAsync(c->uoff.p, b.ncand, (size_t)count * sizeof(uint32_t), cudaMemcpyDeviceToDevice,
-                               c->stream));
-    CG_CUDA(c, scan_exclusive_u32(c->uoff.as<uint32_t>(), (size_t)count + 1, c->scanTmp.p, c->stream));
-    CG_CUDA(c, cudaMemcpyAsync(c->hPinned + 2, c->uoff.as<uint32_t>() + count, sizeof(uint32_t),
-                               cudaMemcpyDeviceToHost, c->stream));
-    CG_CUDA(c, cudaStreamSynchronize(c->stream));
-    c->stats.kernel_launches += scan_launches(count + 1) + 1;
-    // the alignment's warps take their candidates from a counter (deferred
-    // second orientations are then scanned in full warps)
-    CG_CUDA(c, c->laneWork.ensure(sizeof(unsigned int)));
-    CG_CUDA(c, cudaMemsetAsync(c->laneWork.p, 0, sizeof(unsigned int), c->stream));
-    b.laneWork = c->laneWork.as<unsigned int>();
     CG_CUDA(c, cudaEventRecord(c->st1, c->stream));
-    CG_CUDA(c, launch_align_filter(st, c->params, b, c->uoff.as<uint32_t>(), c->hPinned[2], c->st1b, c->stream));
+    const size_t blocks = std::min<size_t>(unit_slots(count, c->hPinned[0]),
+                                           (size_t)sm_count(c) * align_occupancy(st));
+    CG_CUDA(c, launch_align(st, c->params, b, c->lenVaries, (unsigned)blocks, c->stream));
     CG_CUDA(c, cudaEventRecord(c->st2, c->stream));
     CG_CUDA(c, c->msaOrder.ensure((size_t)count * sizeof(uint32_t)));
     CG_CUDA(c, c->orderScratch.ensure(32 * sizeof(unsigned int)));
@@ -806,21 +792,19 @@ int run_batch(cg_ctx* c, uint64_t first, int count, uint8_t* hFlags, char* hOut,
         c->stats.kernel_launches += 1;
     }
     CG_CUDA(c, cudaEventRecord(c->st3, c->stream));
-    c->stats.kernel_launches += 3;
+    c->stats.kernel_launches += 2;
     c->stats.align_launches += 1;
     c->stats.msa_launches += 1;
     CG_CUDA(c, cudaMemcpyAsync(hFlags, b.flags, (size_t)count, c->outKind, c->stream));
     CG_CUDA(c, cudaMemcpy2DAsync(hOut, outPitch, b.out, (size_t)c->lmax, std::min<size_t>(outPitch, c->lmax),
                                  (size_t)count, c->outKind, c->stream));
     CG_CUDA(c, cudaEventSynchronize(c->st3));
-    float t01 = 0, t11 = 0, t12 = 0, t23 = 0;
+    float t01 = 0, t12 = 0, t23 = 0;
     cudaEventElapsedTime(&t01, c->st0, c->st1);
-    cudaEventElapsedTime(&t11, c->st1, c->st1b);
-    cudaEventElapsedTime(&t12, c->st1b, c->st2);
+    cudaEventElapsedTime(&t12, c->st1, c->st2);
     cudaEventElapsedTime(&t23, c->st2, c->st3);
     c->stats.seconds_candidates += t01 / 1000.0;
-    c->stats.seconds_align += t11 / 1000.0;
-    c->stats.seconds_filter += t12 / 1000.0;
+    c->stats.seconds_align += t12 / 1000.0;
     c->stats.seconds_msa += t23 / 1000.0;
     return CG_OK;
 }
@@ -854,8 +838,7 @@ BatchArg set_arg(cg_ctx* c, BatchSet& s, int count) {
     b.fweight = s.fweight.as<float>();
     b.flen = s.flen.as<uint16_t>();
     b.nfinal = s.nfinal.as<uint32_t>();
-    b.perm = c->lenVaries || c->strandTags ? s.perm.as<uint32_t>() : nullptr;
-    b.lenOrder = c->lenVaries;
+    b.units = s.units.as<uint2>();
     b.flags = c->flagsRange.as<uint8_t>();
     b.out = c->outRange.as<char>();
     b.outPitch = c->lmax;
@@ -863,6 +846,8 @@ BatchArg set_arg(cg_ctx* c, BatchSet& s, int count) {
     b.cursor = s.cursor.as<unsigned long long>();
     b.rangeOff = c->rangeOff.as<unsigned long long>();
     b.work = s.work.as<unsigned int>();
+    b.unitCursor = b.work + 1;
+    b.unitCount = b.work + 2;
     if (c->params.correctionType == CG_CORR_LEARNED) set_columns(b, s.colFeat, s.colMeta, s.colCount, count);
     b.order = s.order.as<uint32_t>();
     return b;
@@ -874,11 +859,9 @@ int ensure_set(cg_ctx* c, BatchSet& s, int count, uint64_t capRaw) {
     const size_t n = (size_t)count;
     CG_CUDA(c, s.rawCount.ensure((n + 2) * sizeof(uint32_t)));
     CG_CUDA(c, s.ncand.ensure(n * sizeof(uint32_t)));
-    CG_CUDA(c, s.uoff.ensure((n + 1) * sizeof(uint32_t)));
     CG_CUDA(c, s.nfinal.ensure(n * sizeof(uint32_t)));
-    CG_CUDA(c, s.scanTmp.ensure(scan_tmp_bytes(n + 1)));
+    CG_CUDA(c, s.units.ensure(unit_slots(count, capRaw) * sizeof(uint2)));
     CG_CUDA(c, s.cand.ensure(capRaw * sizeof(uint32_t)));
-    if (c->lenVaries || c->strandTags) CG_CUDA(c, s.perm.ensure(capRaw * sizeof(uint32_t)));
     CG_CUDA(c, s.paired.ensure(capRaw));
     CG_CUDA(c, s.aln.ensure(capRaw * sizeof(uint2)));
     CG_CUDA(c, s.fid.ensure(capRaw * sizeof(uint32_t)));
@@ -887,7 +870,7 @@ int ensure_set(cg_ctx* c, BatchSet& s, int count, uint64_t capRaw) {
     CG_CUDA(c, s.fweight.ensure(capRaw * sizeof(float)));
     CG_CUDA(c, s.flen.ensure(capRaw * sizeof(uint16_t)));
     CG_CUDA(c, s.cursor.ensure(2 * sizeof(unsigned long long)));
-    CG_CUDA(c, s.work.ensure(2 * sizeof(unsigned int)));
+    CG_CUDA(c, s.work.ensure(3 * sizeof(unsigned int)));
     CG_CUDA(c, s.order.ensure(n * sizeof(uint32_t)));
     CG_CUDA(c, s.orderScratch.ensure(32 * sizeof(unsigned int)));
     CG_CUDA(c, s.bigScratch.ensure((n + 1) * sizeof(uint32_t)));
@@ -900,7 +883,6 @@ cudaError_t enqueue_batch(cg_ctx* c, BatchSet& s, int count, unsigned long long 
                           int tableRaw, int maxRows, int* kernels) {
     const StoreArg st = store_arg(c);
     const BatchArg b = set_arg(c, s, count);
-    uint32_t* uoff = s.uoff.as<uint32_t>();
     int k = 0;
     const bool learned = c->params.correctionType == CG_CORR_LEARNED;
     cudaError_t e = learned ? cudaMemsetAsync(b.colCount, 0, sizeof(unsigned int), s.stream) : cudaSuccess;
@@ -911,16 +893,9 @@ cudaError_t enqueue_batch(cg_ctx* c, BatchSet& s, int count, unsigned long long 
         e = launch_pair_flags(b, s.stream);
         k++;
     }
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(uoff, b.ncand, (size_t)count * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s.stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(uoff + count, 0, sizeof(uint32_t), s.stream);
     if (e == cudaSuccess) {
-        e = scan_exclusive_u32(uoff, (size_t)count + 1, s.scanTmp.p, s.stream);
-        k += (int)scan_launches((uint64_t)count + 1);
-    }
-    if (e == cudaSuccess) {
-        e = launch_align_filter(st, c->params, b, uoff, 0, nullptr, s.stream, &sh);
-        k += st.wp - 1 <= 8 ? 2 : 1;
+        e = launch_align(st, c->params, b, c->lenVaries, (unsigned)sh.alignBlocks, s.stream);
+        k++;
     }
     if (e == cudaSuccess) {
         e = launch_msa_order(b, s.orderScratch.as<unsigned int>(), s.order.as<uint32_t>(), s.stream);
@@ -956,9 +931,8 @@ int capture_set(cg_ctx* c, BatchSet& s, int count, unsigned long long stride, co
     g.tableRaw = tableRaw;
     g.maxRows = maxRows;
     for (const DevBuf* d : {&s.rawCount, &s.cand, &s.ncand, &s.paired, &s.aln, &s.fid, &s.fshift, &s.forient,
-                            &s.fweight, &s.flen, &s.nfinal, &s.uoff, &s.scanTmp, &s.cursor, &s.work, &s.colFeat,
-                            &s.colMeta, &s.colCount, &s.order, &s.orderScratch, &s.bigScratch, &s.perm, &c->mlp,
-                            &c->outRange,
+                            &s.fweight, &s.flen, &s.nfinal, &s.units, &s.cursor, &s.work, &s.colFeat,
+                            &s.colMeta, &s.colCount, &s.order, &s.orderScratch, &s.bigScratch, &c->mlp, &c->outRange,
                             &c->flagsRange, &c->rangeOff, &c->counters, &c->sig})
         g.ptrs.push_back(d->p);
     g.ptrs.push_back(reinterpret_cast<const void*>(static_cast<uintptr_t>(c->paramsVersion)));
@@ -1036,7 +1010,7 @@ int run_batched(cg_ctx* c, uint64_t first, uint64_t nb, const Plan& pl, const st
         c->hBatched[3 + 2 * k] = first;
         CG_CUDA(c, cudaMemcpyAsync(s.cursor.p, c->hBatched + 2 + 2 * k, 2 * sizeof(unsigned long long),
                                    cudaMemcpyHostToDevice, c->stream));
-        CG_CUDA(c, cudaMemsetAsync(s.work.p, 0, 2 * sizeof(unsigned int), c->stream));
+        CG_CUDA(c, cudaMemsetAsync(s.work.p, 0, 3 * sizeof(unsigned int), c->stream));
     }
     CG_CUDA(c, cudaEventRecord(c->evPro, c->stream));
     CG_CUDA(c, cudaEventRecord(c->evStart, c->stream));  // replays start (after any capture)
@@ -1062,22 +1036,30 @@ int join_sets(cg_ctx* c, int S, cudaStream_t to) {
     return CG_OK;
 }
 
-// A learned-decision call whose classifier blocks gave up waiting for their
-// MMAs (counters[kCounterTimeouts] grew) left those blocks' columns to the
-// fallback decision: the call reports CG_ERR_TIMEOUT instead of CG_OK.
-int check_classifier_timeouts(cg_ctx* c) {
+// The counters, read with a call's last results (before the event that ends
+// it).
+cudaError_t read_counters(cg_ctx* c) {
+    return cudaMemcpyAsync(c->hCounters, c->counters.p, kNumCounters * sizeof(unsigned long long),
+                           cudaMemcpyDeviceToHost, c->stream);
+}
+
+// A call whose kernels gave up waiting for their tensor-core products reports
+// CG_ERR_TIMEOUT instead of CG_OK: alignment blocks left their anchors
+// uncorrected, classifier blocks (kCounterTimeouts) left their columns to the
+// fallback decision.  After read_counters has arrived.
+int check_timeouts(cg_ctx* c) {
+    const unsigned long long align = c->hCounters[kCounterAlignTimeouts], mlp = c->hCounters[kCounterTimeouts];
+    const unsigned long long moreAlign = align - c->alignTimeoutsSeen, moreMlp = mlp - c->timeoutsSeen;
+    c->alignTimeoutsSeen = align;
+    if (moreAlign)
+        return fail(c, CG_ERR_TIMEOUT, "%llu alignment block(s) timed out waiting for the tensor cores", moreAlign);
     if (c->params.correctionType != CG_CORR_LEARNED || c->collecting) return CG_OK;
-    unsigned long long n = 0;
-    CG_CUDA(c, cudaMemcpy(&n, c->counters.as<unsigned long long>() + kCounterTimeouts, sizeof(n),
-                          cudaMemcpyDeviceToHost));
-    if (n > c->timeoutsSeen) {
-        const unsigned long long grew = n - c->timeoutsSeen;
-        c->timeoutsSeen = n;
+    c->timeoutsSeen = mlp;
+    if (moreMlp)
         return fail(c, CG_ERR_TIMEOUT,
                     "%llu classifier block(s) timed out waiting for the tensor cores; their columns kept the "
                     "fallback decision",
-                    grew);
-    }
+                    moreMlp);
     return CG_OK;
 }
 
@@ -1102,12 +1084,6 @@ TuneKey tune_key(const cg_ctx* c) {
                    c->maxValuesPerKey, lg);
 }
 
-int sm_count(cg_ctx* c) {
-    int sms = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess) sms = 1;
-    return std::max(sms, 1);
-}
-
 // complete a shape: unset grids become the resident maximum
 Plan fill_plan(cg_ctx* c, Plan p) {
     const StoreArg st = store_arg(c);
@@ -1118,7 +1094,7 @@ Plan fill_plan(cg_ctx* c, Plan p) {
     p.streams = std::min(p.streams, kMaxSets);
     if (p.shape.msaWarps <= 0) p.shape.msaWarps = 4;
     p.shape.msaWarps = std::min(std::max(p.shape.msaWarps, 1), 8);
-    if (p.shape.alignBlocks <= 0) p.shape.alignBlocks = sms * std::max(align_lane_occupancy(st), 1);
+    if (p.shape.alignBlocks <= 0) p.shape.alignBlocks = sms * align_occupancy(st);
     if (p.shape.msaBlocks <= 0) p.shape.msaBlocks = sms * std::max(msa_warp_occupancy(st, c->params, p.shape.msaWarps), 1);
     return p;
 }
@@ -1183,7 +1159,7 @@ int plan_for(cg_ctx* c, uint64_t first, uint64_t num, Plan* out) {
     }
     const StoreArg st = store_arg(c);
     const int sms = sm_count(c);
-    const int occA = std::max(align_lane_occupancy(st), 1);
+    const int occA = align_occupancy(st);
     Plan best = fill_plan(c, want);
     double bestSec = 0;
     int rc = time_plan(c, first, sample, best, &bestSec);
@@ -1287,13 +1263,14 @@ int correct_batched(cg_ctx* c, uint64_t first, uint64_t num, uint8_t* out_flags,
     }
     CG_CUDA(c, cudaEventRecord(c->evPro, c->copyStream));
     CG_CUDA(c, cudaStreamWaitEvent(c->stream, c->evPro, 0));
+    CG_CUDA(c, read_counters(c));
     CG_CUDA(c, cudaEventRecord(c->ev1, c->stream));
     CG_CUDA(c, cudaEventSynchronize(c->ev1));
     float ms = 0;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
     c->stats.seconds_correct = ms / 1000.0;
     c->stats.num_anchors_processed += num;
-    return check_classifier_timeouts(c);
+    return check_timeouts(c);
 }
 
 }  // namespace
@@ -1357,9 +1334,10 @@ int cg_create(const cg_options* o, cg_ctx** out) {
     if (e != cudaSuccess) return bail(e);
     e = cudaEventCreate(&c->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
-    for (cudaEvent_t* ev : {&c->st0, &c->st1, &c->st1b, &c->st2, &c->st3})
+    for (cudaEvent_t* ev : {&c->st0, &c->st1, &c->st2, &c->st3})
         if (e == cudaSuccess) e = cudaEventCreate(ev);
     if (e == cudaSuccess) e = cudaMallocHost(&c->hPinned, 4 * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMallocHost(&c->hCounters, kNumCounters * sizeof(unsigned long long));
     if (e == cudaSuccess) e = c->counters.ensure(kNumCounters * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemset(c->counters.p, 0, kNumCounters * sizeof(unsigned long long));
     if (e != cudaSuccess) return bail(e);
@@ -1396,11 +1374,11 @@ void cg_destroy(cg_ctx* c) {
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     release_tables(c);
-    for (DevBuf* b : {&c->enc, &c->len, &c->hilo, &c->qual, &c->ambig, &c->sig, &c->strand, &c->qrange, &c->rawCount,
+    for (DevBuf* b : {&c->enc, &c->len, &c->hilo, &c->qual, &c->ambig, &c->sig, &c->qrange, &c->rawCount,
                       &c->cand,
                       &c->ncand, &c->paired, &c->aln, &c->fid, &c->fshift, &c->forient, &c->fweight, &c->flen, &c->nfinal,
-                      &c->flags, &c->out, &c->counters, &c->scanTmp, &c->uoff, &c->forestNodes, &c->treeOffsets,
-                      &c->msaOrder, &c->orderScratch, &c->bigScratch, &c->perm, &c->lenRange, &c->laneWork})
+                      &c->flags, &c->out, &c->counters, &c->scanTmp, &c->forestNodes, &c->treeOffsets,
+                      &c->msaOrder, &c->orderScratch, &c->bigScratch, &c->units, &c->lenRange})
         b->release();
     for (cg_ctx::Chunk& ch : c->chunks) {
         ch.chars.release();
@@ -1417,7 +1395,8 @@ void cg_destroy(cg_ctx* c) {
     if (c->copyStream) cudaStreamDestroy(c->copyStream);
     if (c->hBatched) cudaFreeHost(c->hBatched);
     if (c->hPinned) cudaFreeHost(c->hPinned);
-    for (cudaEvent_t ev : {c->ev0, c->ev1, c->st0, c->st1, c->st1b, c->st2, c->st3})
+    if (c->hCounters) cudaFreeHost(c->hCounters);
+    for (cudaEvent_t ev : {c->ev0, c->ev1, c->st0, c->st1, c->st2, c->st3})
         if (ev) cudaEventDestroy(ev);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
@@ -1573,13 +1552,14 @@ int cg_correct(cg_ctx* c, uint64_t first, uint64_t num, uint8_t* out_flags, char
         const int rc = run_batch(c, first + a, cnt, out_flags + a, out_seq + a * out_pitch, out_pitch);
         if (rc != CG_OK) return rc;
     }
+    CG_CUDA(c, read_counters(c));
     CG_CUDA(c, cudaEventRecord(c->ev1, c->stream));
     CG_CUDA(c, cudaEventSynchronize(c->ev1));
     float ms = 0;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
     c->stats.seconds_correct = ms / 1000.0;
     c->stats.num_anchors_processed += num;
-    return check_classifier_timeouts(c);
+    return check_timeouts(c);
 }
 
 int cg_combine_results(cg_ctx* c, uint64_t first, uint64_t num, uint8_t* flags, uint64_t* num_candidate_records) {

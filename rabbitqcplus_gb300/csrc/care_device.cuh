@@ -51,6 +51,11 @@ __device__ __forceinline__ void cp_async4(uint32_t* dst, const uint32_t* src) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
 }
+// 16 bytes, both addresses 16-byte aligned (cp.async, L2 only)
+__device__ __forceinline__ void cp_async16(uint32_t* dst, const uint32_t* src) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // first anchor of the batch and anchor id of output row 0: kernel parameters,

@@ -3,9 +3,8 @@
 // Device layout (one context, one GPU):
 //   read store      enc   u32 [N][pitch]      2-bit bases, 16 per word, first base in the MSBs
 //                   len   u16 [N]
-//                   hilo  u32 [N][2][2][wp]   hi/lo bit planes (32 bases per word) of the forward
-//                                             and reverse-complement read, wp = ceil(Lmax/32)+1
-//                                             (one zero word of padding for shifted reads)
+//                   hilo  u32 [N][2][wp]      hi and lo bit planes (32 bases per word), zero past the
+//                                             read; wp = align_plane_words
 //                   qual  u8  [N][Lmax]       Phred+33 (only with quality scores)
 //                   ambig u8  [N]             read had a non-ACGT base
 //   signatures      sig   u64 [maps][N]       minhash key of every read for every map
@@ -30,6 +29,19 @@ constexpr int kMaxMaps = CG_MAX_HASHMAPS;
 constexpr int kMaxBucket = 65535;     // BucketSize is uint16 in the reference
 constexpr int kLearnedFeatures = 32;  // features of one MSA column for the learned decision
 
+// The alignment kernel's instances take reads of up to 32 W bases: W of a
+// store whose longest read has lmax bases (the read lengths in use: 75, 100 to
+// 125, 150, 250 and 300 bp sequencing, and longer merged reads), the words of a
+// bit plane it loads (W and at least one zero word, an even number so that a
+// read's planes are 16-byte pieces), and the candidates per unit of its work
+// (the columns of its products).
+constexpr int align_words(int lmax) {
+    const int need = (lmax + 31) / 32;
+    return need <= 3 ? 3 : need <= 4 ? 4 : need <= 5 ? 5 : need <= 8 ? 8 : need <= 10 ? 10 : need <= 16 ? 16 : 32;
+}
+constexpr int align_plane_words(int w) { return (w + 2) / 2 * 2; }
+constexpr int kAlignUnit = 64;
+
 struct Slot {
     unsigned long long key;
     uint32_t offset;
@@ -44,11 +56,6 @@ struct TablesArg {
     uint32_t mask[kMaxMaps];
     int nmaps;
     int maxValuesPerKey;
-    // With strand set (fewer than 2^31 reads): the read id is the low 31 bits
-    // of every bucket value; in maps 0-15 bit 31 is the value read's strand bit
-    // for that map (launch_signatures) and strand[anchor] holds the anchor's
-    // bits (zero elsewhere: no prediction).
-    const uint16_t* strand;
 };
 
 // Read store view.
@@ -143,11 +150,7 @@ cudaError_t launch_encode(const char* chars, const uint64_t* offs, const char* q
                           uint32_t* enc, uint16_t* len, uint8_t* qual, uint8_t* ambig, int pitch, int lmax,
                           cudaStream_t s);
 cudaError_t launch_hilo(StoreArg st, uint32_t* hilo, cudaStream_t s);
-// sig[maps][N]; with strand set also strand[N], bit q of strand[r] = map
-// q's minimum of read r came from a reverse complement canonical k-mer (maps
-// 0-15)
-cudaError_t launch_signatures(StoreArg st, int k, int nmaps, unsigned long long* sig, uint16_t* strand,
-                              cudaStream_t s);
+cudaError_t launch_signatures(StoreArg st, int k, int nmaps, unsigned long long* sig, cudaStream_t s);
 // out[0] = shortest, out[1] = longest read of the store (out preset to {~0, 0})
 cudaError_t launch_len_range(const uint16_t* len, uint64_t n, unsigned int* out, cudaStream_t s);
 // qualityScoreBits 1 or 2: bins the stored scores of reads [0, n) in place
@@ -158,13 +161,12 @@ cudaError_t launch_quality_bins(uint8_t* qual, const uint16_t* len, uint64_t n, 
 cudaError_t launch_table_init(Slot* t, uint64_t cap, cudaStream_t s);
 // one map's (key, read id) pairs sorted by key (read ids ascending within a
 // key) into keys/vals, from the first `bits` bits of keysIn's keys (values
-// 0 .. n - 1; with tags, n < 2^31 and bit tagBit of tags[i] rides in bit 31
-// of value i); keysAlt/valsAlt hold n pairs of scratch, temp
+// 0 .. n - 1); keysAlt/valsAlt hold n pairs of scratch, temp
 // radix_sort_temp_bytes(n) bytes
 size_t radix_sort_temp_bytes(uint64_t n);
 cudaError_t radix_sort_pairs(const unsigned long long* keysIn, uint64_t n, int bits, unsigned long long* keys,
                              uint32_t* vals, unsigned long long* keysAlt, uint32_t* valsAlt, void* temp,
-                             cudaStream_t s, const uint16_t* tags = nullptr, int tagBit = 0);
+                             cudaStream_t s);
 // runs of equal keys in sorted pairs: runOf[0..n] (scanned in place by the
 // caller into run indices, runOf[n] = number of runs R), start[0..R],
 // packed[0..R] (scanned by the caller into value offsets and totals), then
@@ -178,7 +180,7 @@ cudaError_t launch_run_pack(const unsigned long long* keys, const uint32_t* star
 cudaError_t launch_run_fill(const unsigned long long* keys, const uint32_t* ids, uint64_t n, const uint32_t* runOf,
                             const uint32_t* start, uint32_t runs, const unsigned long long* packedScan, int maxValues,
                             uint32_t* values, Slot* fin, uint32_t finMask, cudaStream_t s,
-                            uint32_t* rawAll = nullptr, uint32_t idMask = 0xffffffffu);
+                            uint32_t* rawAll = nullptr);
 
 // correction batch
 struct BatchArg {
@@ -191,20 +193,20 @@ struct BatchArg {
     uint32_t* cand;         // [totalRaw] unique candidate ids
     uint32_t* ncand;        // [count]
     uint8_t* paired;        // [totalRaw] pair flags (PE)
-    uint2* aln;             // [totalRaw] packed alignment results
+    uint2* aln;             // [totalRaw] packed alignment results (anchors of several units)
     uint32_t* fid;          // [totalRaw] filtered candidates: id
     int16_t* fshift;        // [totalRaw]
     uint8_t* forient;       // [totalRaw] 1 fwd, 2 rc
     float* fweight;         // [totalRaw]
     uint16_t* flen;         // [totalRaw] candidate length
     uint32_t* nfinal;       // [count]
-    // [totalRaw] or null: per anchor, its candidates' positions in the order
-    // the alignment takes them (lane j of an anchor gets candidate perm[j]),
-    // with each one's predicted orientation in bit 31; with lenOrder the
-    // positions are grouped by length, so that a warp's lanes see similar
-    // lengths
-    uint32_t* perm;
-    int lenOrder;
+    // The alignment's work: units {anchor, part} of up to kAlignUnit candidates
+    // (part k holds the anchor's candidates k kAlignUnit ..), appended by the
+    // candidate kernel at *unitCount and taken at *unitCursor (both zero at the
+    // start of a batch); null where only the candidates are wanted.
+    uint2* units;
+    unsigned int* unitCount;
+    unsigned int* unitCursor;
     uint8_t* flags;         // [count] CG_RESULT_*
     char* out;              // [count][outPitch]
     int outPitch;
@@ -218,14 +220,11 @@ struct BatchArg {
     //   rangeOff = exclusive scan of the raw id counts of the anchors
     //     outFirst, outFirst+1, ...; the candidate kernel takes the batch's raw
     //     offsets from it instead of a count pass and a scan per batch
-    //   work[0], work[1] = the persistent alignment and MSA kernels'
-    //     work-stealing counters (zero at the start of a batch)
-    // laneWork (plain form, optional): the alignment's own work-stealing
-    // counter, zero before its launch
+    //   work[0] = the persistent MSA kernel's work-stealing counter (zero at the
+    //     start of a batch)
     const unsigned long long* cursor;
     const unsigned long long* rangeOff;
     unsigned int* work;
-    unsigned int* laneWork;
     // Learned decision (correctionType CG_CORR_LEARNED): the MSA kernel records
     // every column of a non-HQ anchor whose consensus differs from the anchor's
     // base: 32 BF16 features (colFeat) and {output row, position | consensus
@@ -252,6 +251,7 @@ enum {
     kCounterColumnOverflow,  // columns beyond the buffer (decided by the fallback rule)
     kCounterLearnedTaken,    // columns the classifier corrected
     kCounterCandidateVotes,  // candidate corrections made by HQ anchors
+    kCounterAlignTimeouts,   // alignment blocks that gave up waiting for their tensor-core products
     kNumCounters
 };
 
@@ -280,17 +280,14 @@ struct Shape {
     int msaBlocks;    // persistent MSA blocks
 };
 
-// uoff: exclusive scan of the per-anchor candidate counts (count+1 entries),
-// totalUnique = uoff[count] (unused with a shape: the persistent kernel reads
-// uoff[count]); with uoff null the warp-per-anchor kernel runs
-cudaError_t launch_align_filter(StoreArg st, Params p, BatchArg b, const uint32_t* uoff, uint32_t totalUnique,
-                                cudaEvent_t between, cudaStream_t s,  // `between` (optional) after the alignment
-                                const Shape* shape = nullptr);
+// Aligns every unit's candidates (b.units, *b.unitCount of them) and filters
+// the anchors (b.nfinal zero before it); varies: reads of several lengths.
+// Persistent blocks: any number of them does.
+cudaError_t launch_align(StoreArg st, Params p, BatchArg b, bool varies, unsigned blocks, cudaStream_t s);
+// resident 128-thread blocks of it per SM
+int align_occupancy(StoreArg st);
 cudaError_t launch_msa_correct(StoreArg st, Params p, BatchArg b, int maxRows, cudaStream_t s,
                                const Shape* shape = nullptr);
-// resident 128-thread blocks per SM of the thread-per-candidate alignment
-// (0: it does not apply to this store's read length)
-int align_lane_occupancy(StoreArg st);
 // warp-per-anchor MSA blocks of `warps` warps that fit one SM (0: the warp
 // MSA does not apply to this store)
 int msa_warp_occupancy(StoreArg st, Params p, int warps);
@@ -305,7 +302,7 @@ cudaError_t launch_anchor_vote(StoreArg st, Params p, BatchArg b, cudaStream_t s
 // (zeroed by the caller) gains the number of saved candidate records
 cudaError_t launch_combine(StoreArg st, Params p, uint64_t first, uint64_t n, uint8_t* flags,
                            unsigned long long* records, cudaStream_t s);
-// cursor[0] += stride, work[0] = work[1] = 0 (the last node of a batch)
+// cursor[0] += stride, work[0..2] = 0 (the last node of a batch)
 cudaError_t launch_batch_advance(unsigned long long* cursor, unsigned int* work, unsigned long long stride,
                                  cudaStream_t s);
 

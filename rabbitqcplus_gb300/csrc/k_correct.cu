@@ -1,12 +1,9 @@
-// Per-anchor correction: shifted-Hamming alignment of every candidate in both
-// orientations, orientation choice, candidate filters, MSA build, region
-// refinement and the anchor correction decision.
+// Per-anchor correction: MSA build, region refinement and the anchor
+// correction decision.
 //
-// reference: src/cpu_alignment.cpp:32-497 (alignment),
-// include/alignmentorientation.hpp:10-92 (orientation),
-// include/corrector.hpp:982-1211 (flag and mismatch-ratio filters),
-// :1260-1421 (weights, MSA build, refinement), src/msa.cpp:9-173,304-453,532-734
-// (MSA, properties, corrected anchor, different-region search).
+// reference: include/corrector.hpp:1260-1421 (weights, MSA build, refinement),
+// src/msa.cpp:9-173,304-453,532-734 (MSA, properties, corrected anchor,
+// different-region search).
 //
 // Float work keeps the reference's operand order and uses explicitly rounded
 // intrinsics (the library is also built with --fmad=false): every compare the
@@ -22,789 +19,7 @@ namespace cg {
 
 namespace {
 
-// ---------------------------------------------------------------- alignment
-
-constexpr int kAlignWarps = 4;  // warps per block, one anchor per warp
 constexpr unsigned kFull = 0xffffffffu;
-
-struct AlnRes {
-    int score, overlap, shift, nOps;
-    bool valid;
-};
-
-// Warp-cooperative shifted Hamming alignment of one candidate orientation.
-//
-// Each lane evaluates shifts t = lane, lane+32, ... in the reference's scan
-// order (0, 1, .., La-minov, then -1, -2, .., -(Lc-minov)).  The winner is the
-// first shift with the smallest score among those whose mismatch count stays
-// below int(overlap * maxErrorRate); the reference's early exits only skip
-// shifts that cannot win, so evaluating all of them returns its (score, shift).
-//
-// The non-shifted side of every comparison lives in registers (aR: anchor,
-// cR: candidate, hi and lo planes); the shifted side streams from shared
-// memory one word per step.  A lane stops once its mismatch count reaches its
-// limit (the count only grows), and the warp leaves the word loop when no lane
-// is still running.
-template <int MAXW>
-__device__ __forceinline__ AlnRes align_warp(const uint32_t* __restrict__ aS, const uint32_t* __restrict__ cS, int wp,
-                                             const uint32_t (&aR)[2][MAXW], const uint32_t (&cR)[2][MAXW], int La,
-                                             int Lc, int minov, float rate) {
-    const int tb = La + Lc;
-    const int n1 = max(0, La - minov + 1);
-    const int n2 = max(0, Lc - minov);
-    const int lane = (int)lane_id();
-    uint32_t best = 0xffffffffu;
-    for (int t0 = 0; t0 < n1 + n2; t0 += 32) {
-        const int t = t0 + lane;
-        int s = 0, ov = 0;
-        if (t < n1) {
-            s = t;
-            ov = min(La - s, Lc);
-        } else if (t < n1 + n2) {
-            s = -(t - n1 + 1);
-            ov = min(La, Lc + s);
-        }
-        const int maxErr = (int)__fmul_rn((float)ov, rate);
-        bool run = t < n1 + n2 && maxErr > 0 && ov > 0;
-        const bool fwdShift = s >= 0;
-        const int sl = fwdShift ? s : -s;
-        const int parts = (ov + 31) >> 5;
-        const int rem = (parts << 5) - ov;
-        const int ws = sl >> 5, bs = sl & 31;
-        const uint32_t* sh = fwdShift ? aS : cS;
-        uint32_t curH = 0, curL = 0;
-        if (run) {
-            curH = sh[ws];
-            curL = sh[wp + ws];
-        }
-        int m = 0;
-#pragma unroll
-        for (int i = 0; i < MAXW; i++) {
-            const bool act = run && i < parts;
-            if (!__any_sync(kFull, act)) break;
-            if (act) {
-                const uint32_t nxH = sh[ws + i + 1];
-                const uint32_t nxL = sh[wp + ws + i + 1];
-                const uint32_t hi = __funnelshift_l(nxH, curH, bs);
-                const uint32_t lo = __funnelshift_l(nxL, curL, bs);
-                const uint32_t oh = fwdShift ? cR[0][i] : aR[0][i];
-                const uint32_t ol = fwdShift ? cR[1][i] : aR[1][i];
-                uint32_t x = (hi ^ oh) | (lo ^ ol);
-                if (i == parts - 1 && rem != 0) x &= 0xffffffffu << rem;
-                m += __popc(x);
-                curH = nxH;
-                curL = nxL;
-                if (m >= maxErr) run = false;
-            }
-        }
-        if (run) {
-            const int score = m + tb - 2 * ov;
-            if (score < tb) {
-                const uint32_t key = ((uint32_t)score << 16) | (uint32_t)t;
-                best = key < best ? key : best;
-            }
-        }
-    }
-    best = __reduce_min_sync(kFull, best);
-    AlnRes r;
-    int bestShift, bestScore;
-    if (best == 0xffffffffu) {
-        bestShift = -Lc;
-        bestScore = tb;
-    } else {
-        const int t = (int)(best & 0xffffu);
-        bestScore = (int)(best >> 16);
-        bestShift = t < n1 ? t : -(t - n1 + 1);
-    }
-    r.valid = bestShift != -Lc;
-    const int cb = max(-bestShift, 0);
-    const int ce = min(Lc, La - bestShift);
-    r.overlap = ce - cb;
-    r.score = bestScore;
-    r.shift = bestShift;
-    r.nOps = bestScore - tb + 2 * r.overlap;
-    return r;
-}
-
-// Register-resident variant for reads of at most 32*MAXW bases.
-//
-// Shifts are split by direction and lane l takes shifts 32k+l (right, anchor
-// shifted) and 32k+l+1 (left, candidate shifted), so a lane's bit offset is
-// the same in every iteration k and only its word offset advances.  Each lane
-// therefore funnel-shifts the shifted sequence once (SA: per anchor, SC: per
-// candidate orientation) and iteration k, word i reads SA[k+i] / SC[k+i]
-// from registers; the inner loop is XOR/OR/POPC only.  The words compared are
-// exactly those of align_warp (padding words are zero), so the result is the
-// same.  maxErrTab[ov] holds int(float(ov) * maxErrorRate).
-template <int MAXW>
-struct ShiftedRegs {
-    uint32_t h[2 * MAXW - 1], l[2 * MAXW - 1];
-};
-
-template <int MAXW>
-__device__ __forceinline__ void load_shifted(ShiftedRegs<MAXW>& r, const uint32_t* __restrict__ hi,
-                                             const uint32_t* __restrict__ lo, int wp, int wordOff, int bs) {
-#pragma unroll
-    for (int j = 0; j < 2 * MAXW - 1; j++) {
-        const int x = j + wordOff;
-        const uint32_t h0 = x < wp ? hi[x] : 0u, h1 = x + 1 < wp ? hi[x + 1] : 0u;
-        const uint32_t l0 = x < wp ? lo[x] : 0u, l1 = x + 1 < wp ? lo[x + 1] : 0u;
-        r.h[j] = __funnelshift_l(h1, h0, bs);
-        r.l[j] = __funnelshift_l(l1, l0, bs);
-    }
-}
-
-template <int MAXW, bool LEFT>
-__device__ __forceinline__ void scan_direction(const ShiftedRegs<MAXW>& S, const uint32_t (&O)[2][MAXW], int n,
-                                               int La, int Lc, int tb, int tBase, const int16_t* maxErrTab,
-                                               uint32_t& best) {
-    const int lane = (int)lane_id();
-#pragma unroll
-    for (int k = 0; k < MAXW; k++) {
-        if (32 * k >= n) break;
-        const int tl = 32 * k + lane;
-        const bool active = tl < n;
-        const int sl = LEFT ? tl + 1 : tl;
-        const int ov = active ? (LEFT ? min(La, Lc - sl) : min(La - sl, Lc)) : 0;
-        const int maxErr = maxErrTab[ov];
-        const int parts = (ov + 31) >> 5;
-        const int rem = (parts << 5) - ov;
-        const uint32_t last = 0xffffffffu << rem;  // rem < 32
-        // words 0 and 1 without branches: a word past the overlap has mask 0
-        const uint32_t mask0 = parts > 1 ? 0xffffffffu : (parts == 1 ? last : 0u);
-        const uint32_t mask1 = parts > 2 ? 0xffffffffu : (parts == 2 ? last : 0u);
-        int m = __popc(((S.h[k] ^ O[0][0]) | (S.l[k] ^ O[1][0])) & mask0) +
-                __popc(((S.h[k + 1] ^ O[0][1]) | (S.l[k + 1] ^ O[1][1])) & mask1);
-        bool run = active && maxErr > 0 && m < maxErr;
-        // the rest only while some lane of the warp can still be valid
-        if (__any_sync(kFull, run && parts > 2)) {
-#pragma unroll
-            for (int i = 2; i < MAXW; i++) {
-                const bool act = run && i < parts;
-                if (!__any_sync(kFull, act)) break;
-                if (act) {
-                    const uint32_t mask = i == parts - 1 ? last : 0xffffffffu;
-                    m += __popc(((S.h[k + i] ^ O[0][i]) | (S.l[k + i] ^ O[1][i])) & mask);
-                    run = m < maxErr;
-                }
-            }
-        }
-        if (run) {
-            const int score = m + tb - 2 * ov;
-            if (score < tb) {
-                const uint32_t key = ((uint32_t)score << 16) | (uint32_t)(tBase + tl);
-                best = key < best ? key : best;
-            }
-        }
-    }
-}
-
-template <int MAXW>
-__device__ __forceinline__ AlnRes align_regs(const ShiftedRegs<MAXW>& SA, const uint32_t (&A)[2][MAXW],
-                                             const uint32_t* __restrict__ cHi, const uint32_t* __restrict__ cLo,
-                                             int wp, int La, int Lc, int minov, const int16_t* maxErrTab) {
-    const int tb = La + Lc;
-    const int n1 = max(0, La - minov + 1);
-    const int n2 = max(0, Lc - minov);
-    const int lane = (int)lane_id();
-    uint32_t C[2][MAXW];
-#pragma unroll
-    for (int i = 0; i < MAXW; i++) {
-        C[0][i] = i < wp ? cHi[i] : 0u;
-        C[1][i] = i < wp ? cLo[i] : 0u;
-    }
-    uint32_t best = 0xffffffffu;
-    scan_direction<MAXW, false>(SA, C, n1, La, Lc, tb, 0, maxErrTab, best);
-    if (n2 > 0) {
-        ShiftedRegs<MAXW> SC;
-        load_shifted<MAXW>(SC, cHi, cLo, wp, lane == 31 ? 1 : 0, (lane + 1) & 31);
-        scan_direction<MAXW, true>(SC, A, n2, La, Lc, tb, n1, maxErrTab, best);
-    }
-    best = __reduce_min_sync(kFull, best);
-    AlnRes r;
-    int bestShift, bestScore;
-    if (best == 0xffffffffu) {
-        bestShift = -Lc;
-        bestScore = tb;
-    } else {
-        const int t = (int)(best & 0xffffu);
-        bestScore = (int)(best >> 16);
-        bestShift = t < n1 ? t : -(t - n1 + 1);
-    }
-    r.valid = bestShift != -Lc;
-    const int cb = max(-bestShift, 0);
-    const int ce = min(Lc, La - bestShift);
-    r.overlap = ce - cb;
-    r.score = bestScore;
-    r.shift = bestShift;
-    r.nOps = bestScore - tb + 2 * r.overlap;
-    return r;
-}
-
-// reference: include/alignmentorientation.hpp:12-66; 1 fwd, 2 rc, 3 none
-__device__ int choose_orientation(const AlnRes& f, const AlnRes& r, int La, float ratioParam, int minOverlap,
-                                  float maxErr) {
-    const int byRatio = (int)__fmul_rn((float)La, ratioParam);
-    const int minimumOverlap = byRatio > minOverlap ? byRatio : minOverlap;
-    int ret = 3;
-    if (f.valid && f.overlap >= minimumOverlap) {
-        if (r.valid && r.overlap >= minimumOverlap) {
-            const float ratio = __fdiv_rn((float)f.nOps, (float)f.overlap);
-            const float rratio = __fdiv_rn((float)r.nOps, (float)r.overlap);
-            if (ratio < rratio) {
-                if (ratio < maxErr) ret = 1;
-            } else if (rratio < ratio) {
-                if (rratio < maxErr) ret = 2;
-            } else {
-                if (ratio < maxErr) ret = f.overlap > r.overlap ? 1 : 2;
-            }
-        } else {
-            if (__fdiv_rn((float)f.nOps, (float)f.overlap) < maxErr) ret = 1;
-        }
-    } else if (r.valid && r.overlap >= minimumOverlap) {
-        if (__fdiv_rn((float)r.nOps, (float)r.overlap) < maxErr) ret = 2;
-    }
-    return ret;
-}
-
-__device__ __forceinline__ uint2 pack_aln(const AlnRes& r, int ori) {
-    return make_uint2((uint32_t)(uint16_t)(int16_t)r.shift | ((uint32_t)r.overlap << 16),
-                      (uint32_t)(uint16_t)r.nOps | ((uint32_t)ori << 16));
-}
-
-// Mismatch-ratio filter of one anchor (include/corrector.hpp:1053-1149 single
-// end, 1151-1211 paired end) over its aligned candidates b.aln[base, base+nc),
-// writing the kept candidates in order; one warp.
-__device__ void filter_anchor(const StoreArg& st, const Params& p, const BatchArg& b, int a, uint32_t base,
-                              uint32_t nc) {
-    const int lane = (int)lane_id();
-    float thr;
-    if (!p.paired) {
-        uint32_t c0 = 0, c1 = 0, c2 = 0;
-        for (uint32_t j = lane; j < nc; j += 32) {
-            const uint2 v = b.aln[base + j];
-            if ((v.y >> 16) != 3u) {
-                const float ratio = __fdiv_rn((float)(int)(int16_t)(v.y & 0xffffu), (float)(v.x >> 16));
-                c0 += ratio < p.mm2;
-                c1 += ratio < p.mm3;
-                c2 += ratio < p.mm4;
-            }
-        }
-        c0 = __reduce_add_sync(kFull, c0);
-        c1 = __reduce_add_sync(kFull, c1);
-        c2 = __reduce_add_sync(kFull, c2);
-        thr = -3.402823466e+38f;  // std::numeric_limits<float>::lowest()
-        if (c0 > 0 || c1 > 0 || c2 > 0) {
-            if ((float)c0 >= p.goodAlignmentsCountThreshold) thr = p.mm2;
-            else if ((float)c1 >= p.goodAlignmentsCountThreshold) thr = p.mm3;
-            else if ((float)c2 >= p.goodAlignmentsCountThreshold) thr = p.mm4;
-        }
-    } else {
-        thr = p.pairedThreshold;
-    }
-    uint32_t kept = 0, aligned = 0;
-    for (uint32_t j0 = 0; j0 < nc; j0 += 32) {
-        const uint32_t j = j0 + lane;
-        bool keep = false, isAligned = false;
-        uint2 v = make_uint2(0, 0);
-        if (j < nc) {
-            v = b.aln[base + j];
-            const int ori = (int)(v.y >> 16);
-            if (ori != 3) {
-                isAligned = true;
-                const int ov = (int)(v.x >> 16);
-                const int nOps = (int)(int16_t)(v.y & 0xffffu);
-                const float ratio = __fdiv_rn((float)nOps, (float)ov);
-                keep = ratio < thr;
-                if (p.paired && b.paired[base + j]) keep = true;
-            }
-        }
-        const uint32_t m = __ballot_sync(kFull, keep);
-        aligned += __popc(__ballot_sync(kFull, isAligned));
-        if (keep) {
-            const uint32_t pos = kept + __popc(m & ((1u << lane) - 1u));
-            const int ov = (int)(v.x >> 16);
-            const int nOps = (int)(int16_t)(v.y & 0xffffu);
-            const uint32_t cid = b.cand[base + j];
-            b.fid[base + pos] = cid;
-            b.fshift[base + pos] = (int16_t)(v.x & 0xffffu);
-            b.forient[base + pos] = (uint8_t)(v.y >> 16);
-            b.flen[base + pos] = st.len[cid];
-            // reference: include/hostdevicefunctions.cuh:93-95 (calculateOverlapWeight)
-            b.fweight[base + pos] =
-                __fsub_rn(1.0f, __fsqrt_rn(__fdiv_rn((float)nOps, __fmul_rn((float)ov, p.maxErrorRate))));
-        }
-        kept += __popc(m);
-    }
-    if (lane == 0) {
-        b.nfinal[a] = kept;
-        atomicAdd(&b.counters[kCounterAligned], (unsigned long long)aligned);
-        atomicAdd(&b.counters[kCounterMsaCands], (unsigned long long)kept);
-    }
-}
-
-// One warp per anchor: align all candidates, choose orientations, apply the
-// mismatch-ratio filter and write the filtered candidate list in order.
-// Shared memory per warp: anchor hi/lo, candidate fwd hi/lo, rc hi/lo planes.
-template <int MAXW, bool REGS>
-__global__ void __launch_bounds__(kAlignWarps * 32, REGS ? (MAXW <= 5 ? 6 : 4) : 1) align_filter_kernel(StoreArg st, Params p, BatchArg b,
-                                                                        const uint32_t* __restrict__ rawOff) {
-    extern __shared__ uint32_t smem[];
-    const int warp = threadIdx.x >> 5;
-    const int lane = (int)lane_id();
-    const int wp = st.wp;
-    int16_t* maxErrTab = reinterpret_cast<int16_t*>(smem + kAlignWarps * 6 * wp);
-    if (REGS) {
-        for (int i = threadIdx.x; i <= st.lmax; i += blockDim.x)
-            maxErrTab[i] = (int16_t)(int)__fmul_rn((float)i, p.maxErrorRate);
-        __syncthreads();
-    }
-    const int a = blockIdx.x * kAlignWarps + warp;
-    if (a >= b.count) return;
-    uint32_t* aS = smem + warp * 6 * wp;
-    uint32_t* cS = aS + 2 * wp;
-    const uint64_t aid = batch_first(b) + (uint64_t)a;
-    const int La = st.len[aid];
-    const uint32_t nc = b.ncand[a];
-    const uint32_t base = rawOff[a];
-    if (nc == 0) {
-        if (lane == 0) b.nfinal[a] = 0;
-        return;
-    }
-    const uint32_t* ahl = st.hilo + aid * 4 * (uint64_t)wp;  // forward planes
-    for (int i = lane; i < 2 * wp; i += 32) aS[i] = ahl[i];
-    __syncwarp();
-    uint32_t aR[2][MAXW];
-#pragma unroll
-    for (int i = 0; i < MAXW; i++) {
-        aR[0][i] = i < wp ? aS[i] : 0u;
-        aR[1][i] = i < wp ? aS[wp + i] : 0u;
-    }
-    const int minov = max(p.minOverlap, (int)__fmul_rn((float)La, p.minOverlapRatio));
-    ShiftedRegs<MAXW> SA;
-    if (REGS) load_shifted<MAXW>(SA, aS, aS + wp, wp, 0, lane);
-    for (uint32_t j = 0; j < nc; j++) {
-        const uint32_t id = b.cand[base + j];
-        const int Lc = st.len[id];
-        const uint32_t* chl = st.hilo + (uint64_t)id * 4 * wp;
-        __syncwarp();
-        for (int i = lane; i < 4 * wp; i += 32) cS[i] = chl[i];
-        __syncwarp();
-        if (REGS) {
-            const AlnRes f = align_regs<MAXW>(SA, aR, cS, cS + wp, wp, La, Lc, minov, maxErrTab);
-            const AlnRes r = align_regs<MAXW>(SA, aR, cS + 2 * wp, cS + 3 * wp, wp, La, Lc, minov, maxErrTab);
-            const int ori = choose_orientation(f, r, La, p.minOverlapRatio, p.minOverlap, p.orientMaxErrorRate);
-            if (lane == 0) b.aln[base + j] = pack_aln(ori == 2 ? r : f, ori);
-            continue;
-        }
-        uint32_t cR[2][MAXW];
-#pragma unroll
-        for (int i = 0; i < MAXW; i++) {
-            cR[0][i] = i < wp ? cS[i] : 0u;
-            cR[1][i] = i < wp ? cS[wp + i] : 0u;
-        }
-        const AlnRes f = align_warp<MAXW>(aS, cS, wp, aR, cR, La, Lc, minov, p.maxErrorRate);
-#pragma unroll
-        for (int i = 0; i < MAXW; i++) {
-            cR[0][i] = i < wp ? cS[2 * wp + i] : 0u;
-            cR[1][i] = i < wp ? cS[3 * wp + i] : 0u;
-        }
-        const AlnRes r = align_warp<MAXW>(aS, cS + 2 * wp, wp, aR, cR, La, Lc, minov, p.maxErrorRate);
-        const int ori = choose_orientation(f, r, La, p.minOverlapRatio, p.minOverlap, p.orientMaxErrorRate);
-        if (lane == 0) b.aln[base + j] = pack_aln(ori == 2 ? r : f, ori);
-    }
-    __syncwarp();
-    filter_anchor(st, p, b, a, base, nc);
-}
-
-// ---------------------------------------------------------------- lane per candidate
-
-// Both reads' planes for the lane kernel: words 0..MAXW (a read of at most
-// 32 * MAXW bases and the zero word after it).  Every word a shift reads lies
-// at index <= MAXW.
-template <int MAXW>
-__device__ __forceinline__ void load_planes(uint32_t (&R)[2][MAXW + 1], const uint32_t* __restrict__ hilo, int wp) {
-#pragma unroll
-    for (int i = 0; i <= MAXW; i++) {
-        R[0][i] = i < wp ? hilo[i] : 0u;
-        R[1][i] = i < wp ? hilo[wp + i] : 0u;
-    }
-}
-
-// One direction of the reference's sequential shift scan for one lane
-// (src/cpu_alignment.cpp:324-397 right, 408-481 left; the same max_errors,
-// score and break).  S: words of the shifted sequence, O: words of the other
-// one (hi, lo planes, zero past the read).  Right scan (LEFT false): shift
-// sl = 0..n-1 moves the anchor; left scan: sl = 1..n moves the candidate.
-//
-// A fast rejection for shifts whose overlap has at least 32 bases: with at
-// least 64 bases, the mismatches of the overlap's first two words (complete,
-// so no masks) against the error limit of the scan's longest overlap, tabMax;
-// with 32 to 63 bases, those of the first word against the limit at overlap
-// min(63, La, Lc), tab63.  The reference's limit at any shift is
-// min(maxErrTab[ov], ...) and the table is non-decreasing, so it is at most
-// the bound used, and the words' mismatches are part of the shift's: a shift
-// rejected here is rejected there too.  Every other shift takes the
-// reference's step.  The direction ends where the reference's does: at the
-// first shift whose limit is <= 0, i.e. whose overlap is at most
-// max((tb - best) / 2, ovPos - 1), ovPos being the smallest overlap with a
-// positive table entry; that point moves only when the best score improves.
-// Overlap at shift sl: min(X - sl, Y), X = La and Y = Lc for the right scan
-// (anchor shifted), the other way round for the left.
-//
-// Shifts go by word groups W (sl = 32 W + bb); after each group the shifted
-// read's words move down by one, so that word W + i is always S[.][i] and one
-// copy of the loop body serves every group (S is consumed).  The lanes of
-// `lanes` (one candidate each) walk the shifts in step: every loop bound is
-// the same for all of them (warp minimum or maximum of the lanes' own
-// bounds), so the common loops carry one test per shift and no per-lane
-// exits.  A lane past its own end only sees shifts that its step rejects
-// (beyond the end the limit is <= 0, and the step checks the end).
-template <int MAXW, bool LEFT>
-__device__ __forceinline__ void seq_scan_fast(uint32_t (&S)[2][MAXW + 1], const uint32_t (&O)[2][MAXW + 1], int La,
-                                              int Lc, int n, int tb, const int16_t* __restrict__ maxErrTab,
-                                              int tabMax, int tab63, int ovPos, unsigned lanes, int& bestScore,
-                                              int& bestShift) {
-    const int X = LEFT ? Lc : La, Y = LEFT ? La : Lc;
-    const int slFast = Y >= 64 ? X - 64 : -1;   // overlap >= 64 up to here
-    const int slFast1 = Y >= 32 ? X - 32 : -1;  // overlap >= 32 up to here
-    auto stopAt = [&](int best) {
-        const int dv = max((tb - best) >> 1, ovPos - 1);  // done once the overlap is <= dv
-        return Y <= dv ? 0 : X - dv;
-    };
-    int stop = min(LEFT ? n + 1 : n, stopAt(bestScore));
-    const int fastAll = __reduce_min_sync(lanes, slFast);    // every lane in the two-word tier up to here
-    const int fastAny = __reduce_max_sync(lanes, slFast);    // no lane in it past here
-    const int fast1All = __reduce_min_sync(lanes, slFast1);  // every lane in a word tier up to here
-    auto diff = [&](int bb, int i) {
-        return (__funnelshift_l(S[0][i + 1], S[0][i], bb) ^ O[0][i]) |
-               (__funnelshift_l(S[1][i + 1], S[1][i], bb) ^ O[1][i]);
-    };
-    int bb = LEFT ? 1 : 0;
-#pragma unroll 1
-    for (int base = 0; base < 32 * MAXW; base += 32, bb = 0) {
-        const int wStop = __reduce_max_sync(lanes, stop);
-        if (base >= wStop) break;
-        const int ge = min(32, wStop - base);
-        // the reference's step at shift base + bb
-        auto step = [&](int bb) {
-            const int sl = base + bb;
-            if (sl >= stop) return;
-            const int ov = min(X - sl, Y);
-            const int maxErr = min((int)maxErrTab[ov], bestScore - tb + 2 * ov);  // > 0 before `stop`
-            const int parts = (ov + 31) >> 5;
-            const uint32_t last = 0xffffffffu << ((parts << 5) - ov);
-            const uint32_t mask0 = parts > 1 ? 0xffffffffu : last;
-            const uint32_t mask1 = parts > 2 ? 0xffffffffu : (parts == 2 ? last : 0u);
-            int m = __popc(diff(bb, 0) & mask0) + __popc(diff(bb, 1) & mask1);
-            if (m < maxErr && parts > 2) {
-#pragma unroll
-                for (int i = 2; i < MAXW; i++) {
-                    if (i >= parts || m >= maxErr) break;
-                    m += __popc(diff(bb, i) & (i == parts - 1 ? last : 0xffffffffu));
-                }
-            }
-            if (m < maxErr) {
-                const int score = m + tb - 2 * ov;
-                if (score < bestScore) {
-                    bestScore = score;
-                    bestShift = LEFT ? -sl : sl;
-                    stop = min(stop, stopAt(bestScore));
-                }
-            }
-        };
-        // The fast tests only record whether each shift passes (shifted into
-        // `pass` from the bottom, so the group's last shift is bit 0); the
-        // steps run after the group's tests, each lane's in shift order.
-        // The tests do not depend on the best score, so this is the
-        // reference's sequence of steps, and lanes that pass at different
-        // shifts take their steps together instead of one shift at a time.
-        uint32_t pass = 0u;
-        // x < 0: the shift passes (its sign bit moves into pass)
-        auto record = [&](int x) { pass = __funnelshift_l((uint32_t)x, pass, 1); };
-        // shifts where the lanes' tiers differ: each lane tests its own
-        // (selected, not branched on, so the lanes stay together)
-        auto mixed = [&](int e) {
-            for (; bb < e; bb++) {
-                const int sl = base + bb;
-                const bool two = sl <= slFast, one = sl <= slFast1;
-                const int m = __popc(diff(bb, 0)) + (two ? __popc(diff(bb, 1)) : 0);
-                record(m - (two ? tabMax : one ? tab63 : 0x7fffffff));
-            }
-        };
-        {  // all lanes: two words
-            const int e = min(ge, fastAll + 1 - base);
-            if (MAXW <= 5) {  // two shifts per iteration: independent tests, steps in order
-                for (; bb + 1 < e; bb += 2) {
-                    const int ma = __popc(diff(bb, 0)) + __popc(diff(bb, 1)) - tabMax;
-                    const int mb = __popc(diff(bb + 1, 0)) + __popc(diff(bb + 1, 1)) - tabMax;
-                    record(ma);
-                    record(mb);
-                }
-            }
-            for (; bb < e; bb++) record(__popc(diff(bb, 0)) + __popc(diff(bb, 1)) - tabMax);
-        }
-        mixed(min(ge, max(bb, fastAny + 1 - base)));
-        {  // all lanes: one word
-            const int e = min(ge, fast1All + 1 - base);
-            if (MAXW <= 5) {  // two shifts per iteration
-                for (; bb + 1 < e; bb += 2) {
-                    const int ma = __popc(diff(bb, 0)) - tab63, mb = __popc(diff(bb + 1, 0)) - tab63;
-                    record(ma);
-                    record(mb);
-                }
-            }
-            for (; bb < e; bb++) record(__popc(diff(bb, 0)) - tab63);
-        }
-        mixed(ge);
-        while (__any_sync(lanes, pass != 0u)) {
-            if (pass != 0u) {
-                const int q = 31 - __clz(pass);  // the earliest shift left
-                pass ^= 1u << q;
-                step(ge - 1 - q);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < MAXW; k++) {
-            S[0][k] = S[0][k + 1];
-            S[1][k] = S[1][k + 1];
-        }
-        S[0][MAXW] = S[1][MAXW] = 0u;
-    }
-}
-
-// Both directions for one orientation of the candidate (planes at cPlanes);
-// A and C are working copies that the scans consume.
-template <int MAXW>
-__device__ __forceinline__ AlnRes align_seq_fast(const uint32_t* __restrict__ aPlanes,
-                                                 const uint32_t* __restrict__ cPlanes, int wp, uint32_t (&A)[2][MAXW + 1],
-                                                 uint32_t (&C)[2][MAXW + 1], int La, int Lc, int minov,
-                                                 const int16_t* maxErrTab, int ovPos, unsigned lanes) {
-    const int tb = La + Lc;
-    const int tabMax = maxErrTab[min(La, Lc)];
-    const int tab63 = maxErrTab[min(63, min(La, Lc))];
-    int bestScore = tb, bestShift = -Lc;
-    load_planes<MAXW>(A, aPlanes, wp);
-    load_planes<MAXW>(C, cPlanes, wp);
-    seq_scan_fast<MAXW, false>(A, C, La, Lc, La - minov + 1, tb, maxErrTab, tabMax, tab63, ovPos, lanes, bestScore,
-                               bestShift);
-    load_planes<MAXW>(A, aPlanes, wp);
-    seq_scan_fast<MAXW, true>(C, A, La, Lc, Lc - minov, tb, maxErrTab, tabMax, tab63, ovPos, lanes, bestScore,
-                              bestShift);
-    AlnRes r;
-    r.valid = bestShift != -Lc;
-    const int cb = max(-bestShift, 0);
-    const int ce = min(Lc, La - bestShift);
-    r.overlap = ce - cb;
-    r.score = bestScore;
-    r.shift = bestShift;
-    r.nOps = bestScore - tb + 2 * r.overlap;
-    return r;
-}
-
-constexpr int kLaneThreads = 128;
-
-// Whether some shift of one candidate orientation could still tie or beat
-// the other orientation's result in the orientation rule.  Every shift whose
-// overlap has at least minov (>= 32) bases is tested, both directions (right
-// shifts 0 .. La - minov move the anchor against the candidate's first word,
-// left shifts 1 .. Lc - minov the candidate against the anchor's): the hi
-// plane mismatches of the overlap's first 32 bases, a lower bound of the
-// shift's mismatches, against L.  Shifts are tested 32 at a time, fully
-// unrolled: each outcome's sign bit moves into a pass word, which is then
-// masked to the lane's own shifts.  aHi, cHi: the hi planes (wp words).
-template <int MAXW>
-__device__ __forceinline__ bool exists_close_shift(const uint32_t* __restrict__ aHi, const uint32_t* __restrict__ cHi,
-                                                   int wp, int La, int Lc, int minov, int L, unsigned lanes) {
-    bool found = false;
-#pragma unroll 1
-    for (int dir = 0; dir < 2; dir++) {
-        const uint32_t* sh = dir == 0 ? aHi : cHi;
-        const uint32_t o0 = dir == 0 ? cHi[0] : aHi[0];
-        const int n = dir == 0 ? (Lc >= minov ? La - minov + 1 : 0) : (La >= minov ? Lc - minov + 1 : 0);
-        uint32_t R[MAXW + 1];
-#pragma unroll
-        for (int i = 0; i <= MAXW; i++) R[i] = i < wp ? sh[i] : 0u;
-        const int wn = __reduce_max_sync(lanes, n);
-#pragma unroll 1
-        for (int base = 0; base < wn; base += 32) {
-            uint32_t pass = 0u;  // bit 31 - bb: shift base + bb has at most L
-#pragma unroll
-            for (int bb = 0; bb < 32; bb++) {
-                const uint32_t x = __funnelshift_l(R[1], R[0], bb) ^ o0;
-                pass = __funnelshift_l((uint32_t)((int)__popc(x) - L - 1), pass, 1);
-            }
-            const int lo = max(dir - base, 0), hi = min(n - base, 32);  // this lane's shifts [lo, hi)
-            const uint32_t mine = lo < hi ? (0xffffffffu >> lo) & ~(hi >= 32 ? 0u : 0xffffffffu >> hi) : 0u;
-            found |= (pass & mine) != 0u;
-            if (__all_sync(lanes, found)) return true;
-#pragma unroll
-            for (int k = 0; k < MAXW; k++) R[k] = R[k + 1];
-            R[MAXW] = 0u;
-        }
-    }
-    return found;
-}
-
-// A deferred candidate: its slot, anchor, and the result of the orientation
-// scanned first (shift | overlap << 16, nOps | valid << 16 | orientation << 17).
-__device__ __forceinline__ uint4 defer_entry(uint32_t slot, int a, const AlnRes& x, int o) {
-    return make_uint4(slot, (uint32_t)a, (uint32_t)(uint16_t)(int16_t)x.shift | ((uint32_t)x.overlap << 16),
-                      (uint32_t)(uint16_t)(int16_t)x.nOps | ((uint32_t)x.valid << 16) | ((uint32_t)o << 17));
-}
-
-// One thread per (anchor, candidate), warps taking 32-candidate chunks; the
-// packed result of the reference's orientation choice at the candidate's
-// slot.  uoff = exclusive scan of the per-anchor candidate counts.
-//
-// The reference aligns both orientations (its sequential shift scan) and
-// chooses by the mismatch ratios (choose_orientation).  Here each candidate's
-// orientation predicted by its shared minimum (bit 31 of its b.perm entry) is
-// scanned first, x1.  If x1 alone would be chosen and no shift of the other
-// orientation has at most L = floor(nOps1 * min(La, Lc) / overlap1) + 1
-// mismatches (exists_close_shift), the other orientation's best shift, at
-// overlap ov <= min(La, Lc), has a ratio of at least nOps1 / overlap1 + 1 /
-// ov: more than the float rounding of either ratio, so the rule chooses x1
-// as it would with both scans.  Otherwise the candidate is deferred: its
-// warp queues it and later scans the other orientation fully in a round of
-// 32 deferred candidates, and chooses from both results exactly as the
-// reference.  Either way the packed result is the reference's.
-template <int MAXW>
-__global__ void __launch_bounds__(kLaneThreads, 8) align_lane_kernel(StoreArg st, Params p, BatchArg b,
-                                                                  const uint32_t* __restrict__ rawOff,
-                                                                  const uint32_t* __restrict__ uoff, uint32_t total) {
-    __shared__ int16_t maxErrTab[CG_MAX_READ_LENGTH + 2];
-    __shared__ int ovPos;  // smallest overlap whose error limit is positive
-    __shared__ uint4 deferred[kLaneThreads / 32][64];
-    if (threadIdx.x == 0) ovPos = st.lmax + 1;
-    for (int i = threadIdx.x; i <= st.lmax; i += blockDim.x)
-        maxErrTab[i] = (int16_t)(int)__fmul_rn((float)i, p.maxErrorRate);
-    __syncthreads();
-    for (int i = threadIdx.x; i <= st.lmax; i += blockDim.x)  // the table is non-decreasing
-        if (maxErrTab[i] > 0 && (i == 0 || maxErrTab[i - 1] <= 0)) ovPos = i;
-    __syncthreads();
-    const uint64_t first = batch_first(b);
-    const int lane = (int)lane_id(), warp = (int)(threadIdx.x >> 5);
-    uint4* dq = deferred[warp];
-    int queued = 0;  // the warp's deferred candidates (the same in every lane)
-    // persistent form: warps take 32-candidate chunks from a shared counter
-    // until the batch's candidates (uoff[count], on the device) are done;
-    // otherwise one chunk per warp
-    unsigned int* const work = b.work ? b.work : b.laneWork;
-    if (work) total = uoff[b.count];
-    bool chunks = true;
-    uint32_t t0 = blockIdx.x * kLaneThreads + warp * 32;
-    const int wp = st.wp;
-    while (true) {
-        // a round: 32 deferred candidates when as many wait, else the next
-        // chunk, else what is left deferred
-        bool second = queued >= 32;
-        if (!second && chunks) {
-            if (work) {
-                uint32_t c = 0;
-                if (lane == 0) c = atomicAdd(&work[0], 32u);
-                t0 = __shfl_sync(kFull, c, 0);
-            }
-            if (t0 >= total) chunks = false;
-        }
-        if (!second && !chunks) {
-            if (queued == 0) return;
-            second = true;
-        }
-        bool has = false, defer = false;
-        uint32_t slot = 0;
-        int a = 0, o = 0;
-        AlnRes x1{};
-        if (second) {
-            const int cnt = min(queued, 32);
-            uint4 e = make_uint4(0u, 0u, 0u, 0u);
-            if (lane < cnt) e = dq[lane];
-            __syncwarp();
-            if (lane + 32 < queued) dq[lane] = dq[lane + 32];
-            __syncwarp();
-            queued -= cnt;
-            has = lane < cnt;
-            slot = e.x;
-            a = (int)e.y;
-            x1.shift = (int)(int16_t)(e.z & 0xffffu);
-            x1.overlap = (int)(e.z >> 16);
-            x1.nOps = (int)(int16_t)(e.w & 0xffffu);
-            x1.valid = ((e.w >> 16) & 1u) != 0u;
-            o = 1 - (int)((e.w >> 17) & 1u);  // the orientation not yet scanned
-        } else {
-            const uint32_t t = t0 + (uint32_t)lane;
-            has = t < total;
-            if (has) {
-                int lo = 0, hi = b.count;  // last anchor with uoff[a] <= t
-                while (hi - lo > 1) {
-                    const int mid = (lo + hi) >> 1;
-                    if (uoff[mid] <= t) lo = mid;
-                    else hi = mid;
-                }
-                a = lo;
-                const uint32_t j = t - uoff[a];
-                const uint32_t pe = b.perm ? b.perm[rawOff[a] + j] : j;  // position, predicted orientation
-                slot = rawOff[a] + (pe & 0x7fffffffu);
-                o = (int)(pe >> 31);
-            }
-        }
-        const unsigned lanes = __ballot_sync(kFull, has);  // the warp's lanes with a candidate
-        if (has) {
-            const uint64_t aid = first + (uint64_t)a;
-            const uint32_t id = b.cand[slot];
-            const int La = st.len[aid], Lc = st.len[id];
-            const int minov = max(p.minOverlap, (int)__fmul_rn((float)La, p.minOverlapRatio));
-            const uint32_t* aPl = st.hilo + aid * 4 * (uint64_t)wp;
-            const uint32_t* cPl = st.hilo + (uint64_t)id * 4 * wp;
-            uint32_t A[2][MAXW + 1], C[2][MAXW + 1];
-            const AlnRes x = align_seq_fast<MAXW>(aPl, cPl + 2 * wp * o, wp, A, C, La, Lc, minov, maxErrTab, ovPos,
-                                                  lanes);
-            if (second) {
-                const AlnRes& f = o == 0 ? x : x1;
-                const AlnRes& r = o == 0 ? x1 : x;
-                const int ori = choose_orientation(f, r, La, p.minOverlapRatio, p.minOverlap, p.orientMaxErrorRate);
-                b.aln[slot] = pack_aln(ori == 2 ? r : f, ori);
-            } else {
-                AlnRes none{};
-                none.valid = false;
-                const int solo = o == 0 ? choose_orientation(x, none, La, p.minOverlapRatio, p.minOverlap,
-                                                             p.orientMaxErrorRate)
-                                        : choose_orientation(none, x, La, p.minOverlapRatio, p.minOverlap,
-                                                             p.orientMaxErrorRate);
-                const bool test = solo != 3 && minov >= 32;
-                const unsigned tlanes = __ballot_sync(lanes, test);
-                bool close = true;
-                if (test) {
-                    const int L = (int)(((uint32_t)x.nOps * (uint32_t)min(La, Lc)) / (uint32_t)x.overlap) + 1;
-                    close = exists_close_shift<MAXW>(aPl, cPl + 2 * wp * (1 - o), wp, La, Lc, minov, L, tlanes);
-                }
-                if (!close) b.aln[slot] = pack_aln(x, solo);
-                defer = close;
-                x1 = x;
-            }
-        }
-        if (!second) {  // queue the deferred candidates of the chunk
-            const unsigned dm = __ballot_sync(kFull, defer);
-            if (defer) dq[queued + __popc(dm & ((1u << lane) - 1u))] = defer_entry(slot, a, x1, o);
-            queued += __popc(dm);
-            __syncwarp();
-            if (!work) chunks = false;  // one chunk per warp
-        }
-    }
-}
-
-// one warp per anchor: the mismatch-ratio filter after align_lane_kernel
-__global__ void __launch_bounds__(128) filter_kernel(StoreArg st, Params p, BatchArg b,
-                                                     const uint32_t* __restrict__ rawOff) {
-    const int a = (int)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (a >= b.count) return;
-    const uint32_t nc = b.ncand[a];
-    if (nc == 0) {
-        if (lane_id() == 0) b.nfinal[a] = 0;
-        return;
-    }
-    filter_anchor(st, p, b, a, rawOff[a], nc);
-}
 
 // ---------------------------------------------------------------- MSA
 
@@ -1825,7 +1040,7 @@ __host__ __device__ inline size_t msa_warp_slice_bytes(int lp, int pitch, const 
 
 // `warps` warps per block, each on its own anchors.  Plain form: anchor
 // blockIdx.x * warps + warp.  Persistent form (b.work set): warps take the
-// next anchor from the counter b.work[1] until the batch is done.
+// next anchor from the counter b.work[0] until the batch is done.
 __global__ void __launch_bounds__(256, 4) msa_warp_kernel(StoreArg st, Params p, BatchArg b,
                                                        const uint32_t* __restrict__ rawOff, int lp) {
     extern __shared__ __align__(16) unsigned char sm[];
@@ -1852,7 +1067,7 @@ __global__ void __launch_bounds__(256, 4) msa_warp_kernel(StoreArg st, Params p,
     }
     while (true) {
         int i = 0;
-        if (lane == 0) i = (int)atomicAdd(&b.work[1], 1u);
+        if (lane == 0) i = (int)atomicAdd(&b.work[0], 1u);
         i = __shfl_sync(kFull, i, 0);
         if (i >= b.count) return;
         anchor(i);
@@ -1908,57 +1123,7 @@ __global__ void msa_order_scatter_kernel(const uint32_t* __restrict__ nfinal, in
     }
 }
 
-template <int MAXW, bool REGS>
-cudaError_t launch_align_t(StoreArg st, Params p, BatchArg b, cudaStream_t s) {
-    const size_t smem = (size_t)kAlignWarps * 6 * st.wp * sizeof(uint32_t) +
-                        (REGS ? ((size_t)st.lmax + 2) * sizeof(int16_t) : 0);
-    const unsigned blocks = (unsigned)((b.count + kAlignWarps - 1) / kAlignWarps);
-    align_filter_kernel<MAXW, REGS><<<blocks, kAlignWarps * 32, smem, s>>>(st, p, b, b.rawCount);
-    return cudaGetLastError();
-}
-
 }  // namespace
-
-cudaError_t launch_align_filter(StoreArg st, Params p, BatchArg b, const uint32_t* uoff, uint32_t totalUnique,
-                                cudaEvent_t between, cudaStream_t s, const Shape* shape) {
-    const int need = st.wp - 1;  // words per plane that hold bases
-    if (need <= 8 && uoff) {
-        const bool persistent = shape && b.work;
-        if (persistent || totalUnique > 0) {
-            // persistent: the warps take 32-candidate chunks until uoff[count];
-            // with b.laneWork (plain form) as many blocks as fit the GPU do the same
-            unsigned blocks =
-                persistent ? (unsigned)shape->alignBlocks : (totalUnique + kLaneThreads - 1) / kLaneThreads;
-            if (!persistent && b.laneWork) {
-                int dev = 0, sms = 1, occ = 1;
-                if (cudaGetDevice(&dev) == cudaSuccess)
-                    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-                occ = std::max(align_lane_occupancy(st), 1);
-                blocks = std::min(blocks, (unsigned)(std::max(sms, 1) * occ));
-            }
-            if (need <= 5)
-                align_lane_kernel<5><<<blocks, kLaneThreads, 0, s>>>(st, p, b, b.rawCount, uoff, totalUnique);
-            else
-                align_lane_kernel<8><<<blocks, kLaneThreads, 0, s>>>(st, p, b, b.rawCount, uoff, totalUnique);
-            cudaError_t e = cudaGetLastError();
-            if (e != cudaSuccess) return e;
-        }
-        if (between) {
-            cudaError_t e = cudaEventRecord(between, s);
-            if (e != cudaSuccess) return e;
-        }
-        filter_kernel<<<(unsigned)(((uint64_t)b.count * 32 + 127) / 128), 128, 0, s>>>(st, p, b, b.rawCount);
-        return cudaGetLastError();
-    }
-    if (between) {
-        cudaError_t e = cudaEventRecord(between, s);  // the fused kernel below aligns and filters
-        if (e != cudaSuccess) return e;
-    }
-    if (need <= 5) return launch_align_t<5, true>(st, p, b, s);
-    if (need <= 8) return launch_align_t<8, true>(st, p, b, s);
-    if (need <= 16) return launch_align_t<16, false>(st, p, b, s);
-    return launch_align_t<32, false>(st, p, b, s);
-}
 
 int msa_threads(int maxCols) {
     int t = kMsaThreadsMin;
@@ -1984,16 +1149,6 @@ cudaError_t msa_warp_prepare(size_t smem) {
 }
 
 }  // namespace
-
-int align_lane_occupancy(StoreArg st) {
-    const int need = st.wp - 1;
-    if (need > 8) return 0;
-    int blocks = 0;
-    const cudaError_t e = need <= 5
-        ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, align_lane_kernel<5>, kLaneThreads, 0)
-        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, align_lane_kernel<8>, kLaneThreads, 0);
-    return e == cudaSuccess ? blocks : 0;
-}
 
 int msa_warp_occupancy(StoreArg st, Params p, int warps) {
     if (st.lmax > 256 || warps < 1 || warps > 8) return 0;
@@ -2099,8 +1254,7 @@ __global__ void combine_kernel(StoreArg st, Params p, uint64_t first, uint64_t n
 
 __global__ void batch_advance_kernel(unsigned long long* cursor, unsigned int* work, unsigned long long stride) {
     cursor[0] += stride;
-    work[0] = 0;
-    work[1] = 0;
+    work[0] = work[1] = work[2] = 0;
 }
 }  // namespace
 

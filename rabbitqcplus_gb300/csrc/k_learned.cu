@@ -21,6 +21,7 @@
 #include "care_device.cuh"
 #include "care_internal.h"
 #include "care_learned.h"
+#include "care_tc.cuh"
 
 namespace cg {
 
@@ -53,57 +54,6 @@ constexpr uint32_t kWaitSpins = 1u << 20;  // mbarrier polls before a wait is de
 // failed block's MMAs before its tensor memory is released always uses
 // kWaitSpins.
 __device__ uint32_t g_tileWaitSpins = kWaitSpins;
-
-// byte offset of element (row, k) of a K-major tile with kdim columns
-__device__ __forceinline__ uint32_t core_offset(int row, int k, int kdim) {
-    return (uint32_t)((((row >> 3) * (kdim >> 3) + (k >> 3)) << 7) + ((row & 7) << 4) + ((k & 7) << 1));
-}
-
-__device__ __forceinline__ uint32_t smem_u32(const void* ptr) { return (uint32_t)__cvta_generic_to_shared(ptr); }
-
-// shared-memory matrix descriptor: start address, leading byte offset (next
-// core matrix along K), stride byte offset (next 8-row group), version 1, no
-// swizzle
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((addr >> 4) & 0x3fffu) | ((uint64_t)((lbo >> 4) & 0x3fffu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3fffu) << 32) | (1ull << 46);
-}
-
-// instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both
-// K-major, M x N
-__host__ __device__ constexpr uint32_t instr_desc(int M, int N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-
-__device__ __forceinline__ void tc_mma(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(dtmem),
-        "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
-}
-
-__device__ __forceinline__ void tc_commit(uint32_t mbar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// bounded wait (at most `polls` polls) for the completion of mbarrier phase `parity`
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, uint32_t polls) {
-    for (uint32_t i = 0; i < polls; i++) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(done)
-            : "r"(mbar), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
-}
 
 // 32 consecutive FP32 accumulator columns of this thread's TMEM lane
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {

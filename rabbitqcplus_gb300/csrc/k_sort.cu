@@ -50,12 +50,11 @@ __global__ void __launch_bounds__(kSortThreads) radix_count_kernel(const unsigne
 }
 
 // One tile per block.  offsets = the exclusive scan of radix_count_kernel's
-// counts; vals == nullptr stands for the values 0, 1, ..., n - 1, each with
-// bit tagBit of tags[i] in bit 31 when tags is set.
+// counts; vals == nullptr stands for the values 0, 1, ..., n - 1.
 __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(
     const unsigned long long* __restrict__ keys, const uint32_t* __restrict__ vals, uint64_t n, int shift,
     const uint32_t* __restrict__ offsets, uint32_t tiles, unsigned long long* __restrict__ keysOut,
-    uint32_t* __restrict__ valsOut, const uint16_t* __restrict__ tags, int tagBit) {
+    uint32_t* __restrict__ valsOut) {
     __shared__ uint32_t wcount[kSortWarps][kDigits];  // per warp: digit counts, then the warp's start in the digit
     __shared__ uint32_t tileStart[kDigits];           // digit d's first position in the staged tile
     __shared__ uint32_t globalStart[kDigits];         // and in the output
@@ -77,8 +76,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(
         const uint64_t i = base + (uint64_t)(32 * j + lane);
         const bool valid = i < n;
         k[j] = valid ? keys[i] : 0ull;
-        v[j] = valid ? (vals ? vals[i] : ((uint32_t)i | (tags ? ((uint32_t)(tags[i] >> tagBit) & 1u) << 31 : 0u)))
-                     : 0u;
+        v[j] = valid ? (vals ? vals[i] : (uint32_t)i) : 0u;
         rank[j] = 0;
         const unsigned act = __ballot_sync(kFull, valid);
         if (valid) {
@@ -147,9 +145,9 @@ size_t radix_sort_temp_bytes(uint64_t n) {
 
 cudaError_t radix_sort_pairs(const unsigned long long* keysIn, uint64_t n, int bits, unsigned long long* keys,
                              uint32_t* vals, unsigned long long* keysAlt, uint32_t* valsAlt, void* temp,
-                             cudaStream_t s, const uint16_t* tags, int tagBit) {
+                             cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    if (n > 0xffffffffull || (tags && n > 0x7fffffffull)) return cudaErrorInvalidValue;
+    if (n > 0xffffffffull) return cudaErrorInvalidValue;
     const uint32_t tiles = (uint32_t)((n + kSortTile - 1) / kSortTile);
     const size_t ncounts = (size_t)kDigits * tiles;
     uint32_t* counts = static_cast<uint32_t*>(temp);
@@ -167,7 +165,7 @@ cudaError_t radix_sort_pairs(const unsigned long long* keysIn, uint64_t n, int b
         if (e != cudaSuccess) return e;
         e = scan_exclusive_u32(counts, ncounts, scanTmp, s);
         if (e != cudaSuccess) return e;
-        radix_scatter_kernel<<<tiles, kSortThreads, 0, s>>>(ki, vi, n, 8 * p, counts, tiles, ko, vo, tags, tagBit);
+        radix_scatter_kernel<<<tiles, kSortThreads, 0, s>>>(ki, vi, n, 8 * p, counts, tiles, ko, vo);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         ki = ko;

@@ -198,45 +198,36 @@ __global__ void encode_kernel(const char* __restrict__ chars, const uint64_t* __
     }
 }
 
-// one thread per read and orientation: hi/lo bit planes, 32 bases per word
+// the 16 odd (hi) or even (lo) bits of a 2-bit word, in order
+__device__ __forceinline__ uint32_t odd_bits(uint32_t x) {
+    x = (x >> 1) & 0x55555555u;
+    x = (x | (x >> 1)) & 0x33333333u;
+    x = (x | (x >> 2)) & 0x0f0f0f0fu;
+    x = (x | (x >> 4)) & 0x00ff00ffu;
+    return (x | (x >> 8)) & 0xffffu;
+}
+
+// hi/lo bit planes, 32 bases per word: one thread per word of a plane pair
+// (the 2-bit rows are zero past the read, so the planes are too)
 __global__ void hilo_kernel(StoreArg st, uint32_t* __restrict__ hilo) {
     const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t r = t >> 1;
-    const int rc = (int)(t & 1);
+    const uint64_t r = t / (uint32_t)st.wp;
     if (r >= st.n) return;
-    const int L = st.len[r];
+    const int w = (int)(t - r * (uint32_t)st.wp);
     const uint32_t* e = st.enc + r * (uint64_t)st.pitch;
-    uint32_t* hi = hilo + (r * 2 + rc) * 2 * (uint64_t)st.wp;
-    uint32_t* lo = hi + st.wp;
-    for (int w = 0; w < st.wp; w++) {
-        uint32_t h = 0, l = 0;
-        for (int j = 0; j < 32; j++) {
-            const int p = w * 32 + j;
-            if (p < L) {
-                const uint32_t bb = rc ? 3u - get2bit(e, L - 1 - p) : get2bit(e, p);
-                h |= (bb >> 1) << (31 - j);
-                l |= (bb & 1u) << (31 - j);
-            }
-        }
-        hi[w] = h;
-        lo[w] = l;
-    }
+    const uint32_t e0 = 2 * w < st.pitch ? e[2 * w] : 0u, e1 = 2 * w + 1 < st.pitch ? e[2 * w + 1] : 0u;
+    uint32_t* row = hilo + r * 2 * (uint64_t)st.wp;
+    row[w] = (odd_bits(e0) << 16) | odd_bits(e1);
+    row[st.wp + w] = (odd_bits(e0 << 1) << 16) | odd_bits(e1 << 1);
 }
 
 // Signatures: one thread per (read, group of 16 maps); threads of a warp take
 // consecutive reads of the same group so the map-major stores coalesce.
-// With `strand`, bit q of strand[read] tells whether map q's minimum (maps
-// 0-15 only) came from a k-mer whose canonical form is its reverse
-// complement: two reads that share that minimum overlap in the same
-// orientation when their bits agree, which the alignment uses to choose which
-// orientation to scan first (a prediction only: the result does not depend on
-// it).  The threads of the other maps skip the bookkeeping.
 constexpr int kSigReads = 128;
 constexpr int kSigGroup = 16;
 
 __global__ void __launch_bounds__(kSigReads * 3) signature_kernel(StoreArg st, int k, int nmaps,
-                                                                  unsigned long long* __restrict__ sig,
-                                                                  uint16_t* __restrict__ strand) {
+                                                                  unsigned long long* __restrict__ sig) {
     const uint64_t r = (uint64_t)blockIdx.x * kSigReads + (threadIdx.x % kSigReads);
     const int g = threadIdx.x / kSigReads;
     const int m0 = g * kSigGroup;
@@ -245,8 +236,6 @@ __global__ void __launch_bounds__(kSigReads * 3) signature_kernel(StoreArg st, i
     uint64_t mins[kSigGroup];
 #pragma unroll
     for (int j = 0; j < kSigGroup; j++) mins[j] = ~0ull;
-    uint32_t sb = 0;  // strand bit of each map's minimum
-    const bool track = strand && g == 0;
     const int L = st.len[r];
     if (L >= k) {
         const uint32_t* e = st.enc + r * (uint64_t)st.pitch;
@@ -261,22 +250,10 @@ __global__ void __launch_bounds__(kSigReads * 3) signature_kernel(StoreArg st, i
                 rc = (rc >> 2) | ((3ull - bb) << rcShift);
                 if (w * 16 + j >= k - 1) {
                     const uint64_t canon = fwd < rc ? fwd : rc;
-                    if (track) {  // the same for every thread of a warp
-                        const uint32_t rcBits = rc < fwd ? 0xffffu : 0u;
 #pragma unroll
-                        for (int q = 0; q < kSigGroup; q++) {
-                            const uint64_t hv = murmur64(canon + (uint64_t)(m0 + q));
-                            const bool lower = hv < mins[q];
-                            mins[q] = lower ? hv : mins[q];
-                            const uint32_t m = lower ? 1u << q : 0u;  // bit q takes this k-mer's strand
-                            sb = (sb & ~m) | (rcBits & m);
-                        }
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < kSigGroup; q++) {
-                            const uint64_t hv = murmur64(canon + (uint64_t)(m0 + q));
-                            mins[q] = hv < mins[q] ? hv : mins[q];
-                        }
+                    for (int q = 0; q < kSigGroup; q++) {
+                        const uint64_t hv = murmur64(canon + (uint64_t)(m0 + q));
+                        mins[q] = hv < mins[q] ? hv : mins[q];
                     }
                 }
             }
@@ -286,7 +263,6 @@ __global__ void __launch_bounds__(kSigReads * 3) signature_kernel(StoreArg st, i
     for (int q = 0; q < kSigGroup; q++) {
         if (m0 + q < nmaps) sig[(uint64_t)(m0 + q) * st.n + r] = mins[q] & kmask;
     }
-    if (track) strand[r] = (uint16_t)sb;
 }
 
 }  // namespace
@@ -316,7 +292,7 @@ cudaError_t launch_encode(const char* chars, const uint64_t* offs, const char* q
 }
 
 cudaError_t launch_hilo(StoreArg st, uint32_t* hilo, cudaStream_t s) {
-    const uint64_t threads = st.n * 2;
+    const uint64_t threads = st.n * (uint64_t)st.wp;
     hilo_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(st, hilo);
     return cudaGetLastError();
 }
@@ -375,10 +351,9 @@ cudaError_t launch_len_range(const uint16_t* len, uint64_t n, unsigned int* out,
     return cudaGetLastError();
 }
 
-cudaError_t launch_signatures(StoreArg st, int k, int nmaps, unsigned long long* sig, uint16_t* strand,
-                              cudaStream_t s) {
+cudaError_t launch_signatures(StoreArg st, int k, int nmaps, unsigned long long* sig, cudaStream_t s) {
     const unsigned blocks = (unsigned)((st.n + kSigReads - 1) / kSigReads);
-    signature_kernel<<<blocks, kSigReads * 3, 0, s>>>(st, k, nmaps, sig, strand);
+    signature_kernel<<<blocks, kSigReads * 3, 0, s>>>(st, k, nmaps, sig);
     return cudaGetLastError();
 }
 

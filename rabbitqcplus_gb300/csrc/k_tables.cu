@@ -75,12 +75,12 @@ __global__ void run_pack_kernel(const unsigned long long* __restrict__ keys, con
 // packedScan = exclusive scan of run_pack_kernel's output: the read ids of
 // every kept run, in order, at its value offset.  With rawAll set, each kept
 // id also adds its run's length -- its bucket's size, the ids a query of that
-// read finds in this map -- to rawAll[id & idMask] (atomic: the maps of a
-// build wave run concurrently; idMask drops a strand tag in bit 31).
+// read finds in this map -- to rawAll[id] (atomic: the maps of a build wave
+// run concurrently).
 __global__ void run_values_kernel(const unsigned long long* __restrict__ keys, const uint32_t* __restrict__ ids,
                                   uint64_t n, const uint32_t* __restrict__ runOf, const uint32_t* __restrict__ start,
                                   const unsigned long long* __restrict__ packedScan, int maxValues,
-                                  uint32_t* __restrict__ values, uint32_t* __restrict__ rawAll, uint32_t idMask) {
+                                  uint32_t* __restrict__ values, uint32_t* __restrict__ rawAll) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t r = runOf[i + 1] - 1u;
@@ -88,7 +88,7 @@ __global__ void run_values_kernel(const unsigned long long* __restrict__ keys, c
     if (!run_kept(keys[i], len, maxValues)) return;
     const uint32_t id = ids[i];
     values[(uint32_t)(packedScan[r] & 0xffffffffull) + ((uint32_t)i - s0)] = id;
-    if (rawAll) atomicAdd(&rawAll[id & idMask], len);
+    if (rawAll) atomicAdd(&rawAll[id], len);
 }
 
 // every kept run's key into the final table with its value offset and length
@@ -236,34 +236,15 @@ __device__ void gather_one(const StoreArg& st, const TablesArg& tb, const Params
     }
     for (uint32_t i = tid; i < T; i += kGatherThreads) table[i] = 0xffffffffu;
     if (tid == 0) nUnique = 0;
-    // With strand-tagged values (tb.strand set) a unique candidate's list
-    // entry is its sort key id << 1 | o, o = the orientation predicted by the
-    // map whose bucket brought its first copy: its strand bit against the
-    // anchor's for that map (0 forward, 1 reverse complement).  The ids are
-    // distinct, so sorting the keys sorts the ids.
-    const bool tagged = tb.strand != nullptr;
     constexpr int kGroup = 16, kGroups = kGatherThreads / kGroup, kMapsPer = (kMaxMaps + kGroups - 1) / kGroups;
-    const int g = tid / kGroup, gl = tid % kGroup;
-    // this thread's maps g + k kGroups: bit k = the anchor's strand bit there
-    // (maps 0-15 only; the others carry no prediction)
-    uint32_t aStrand = 0;
-    if (tagged) {
-        const uint32_t bits = tb.strand[aid];
-#pragma unroll
-        for (int k = 0; k < kMapsPer; k++) {
-            const int m = g + k * kGroups;
-            if (m < 16) aStrand |= ((bits >> m) & 1u) << k;
-        }
-    }
+    const int g = tid / kGroup, gl = tid % kGroup;  // this thread's maps: g + k kGroups
     __syncthreads();
-    auto insert = [&](uint32_t tv, int k) {  // a value of map g + k kGroups
-        const uint32_t v = tagged ? tv & 0x7fffffffu : tv;
+    auto insert = [&](uint32_t v) {
         uint32_t h = (v * 0x9E3779B1u) & mask;
         for (uint32_t probe = 0; probe < T; probe++) {
             const uint32_t old = atomicCAS(&table[h], 0xffffffffu, v);
             if (old == 0xffffffffu) {  // the first copy of v
-                if ((uint64_t)v != aid && !(p.excludeAmbiguous && st.ambig[v]))
-                    list[atomicAdd(&nUnique, 1u)] = tagged ? (v << 1) | ((tv >> 31) ^ ((aStrand >> k) & 1u)) : v;
+                if ((uint64_t)v != aid && !(p.excludeAmbiguous && st.ambig[v])) list[atomicAdd(&nUnique, 1u)] = v;
                 return;
             }
             if (old == v) return;
@@ -279,20 +260,15 @@ __device__ void gather_one(const StoreArg& st, const TablesArg& tb, const Params
     }
 #pragma unroll
     for (int k = 0; k < kMapsPer; k++)
-        if (vals[k] != 0xffffffffu) insert(vals[k], k);
+        if (vals[k] != 0xffffffffu) insert(vals[k]);
     for (int k = 0; k < kMapsPer; k++) {  // ids past a bucket's first 16
         const int m = g + k * kGroups;
         if (m >= tb.nmaps) break;
-        for (uint32_t i = kGroup + gl; i < rng[m].y; i += kGroup) insert(tb.values[m][rng[m].x + i], k);
+        for (uint32_t i = kGroup + gl; i < rng[m].y; i += kGroup) insert(tb.values[m][rng[m].x + i]);
     }
     __syncthreads();
     const uint32_t U = nUnique;
     uint32_t* out = b.cand + off;
-    const int keyShift = tagged ? 1 : 0;
-    // the sorted keys stay in shared memory for the alignment order below:
-    // in `list` after the register sort, in `table` (free once the ids are
-    // in) after the others
-    const uint32_t* sk = U <= 64 ? list : table;
     if (U <= 64) {
         // one warp: a bitonic network over 64 slots in registers, ids i and
         // i + 32 in lane i (padding sorts last; the ids are distinct)
@@ -317,11 +293,8 @@ __device__ void gather_one(const StoreArg& st, const TablesArg& tb, const Params
                     }
                 }
             }
-            if (lane < U) out[lane] = x0 >> keyShift;
-            if (lane + 32 < U) out[lane + 32] = x1 >> keyShift;
-            __syncwarp();  // every lane has read its unsorted keys
-            if (lane < U) list[lane] = x0;  // the list holds at least U entries
-            if (lane + 32 < U) list[lane + 32] = x1;
+            if (lane < U) out[lane] = x0;
+            if (lane + 32 < U) out[lane + 32] = x1;
         }
     } else if (U <= 512) {
         // rank of each id among the unique ids = its position in ascending order
@@ -329,8 +302,7 @@ __device__ void gather_one(const StoreArg& st, const TablesArg& tb, const Params
             const uint32_t v = list[i];
             uint32_t rank = 0;
             for (uint32_t k = 0; k < U; k++) rank += list[k] < v;
-            out[rank] = v >> keyShift;
-            table[rank] = v;
+            out[rank] = v;
         }
     } else {
         uint32_t S = 1;
@@ -353,64 +325,15 @@ __device__ void gather_one(const StoreArg& st, const TablesArg& tb, const Params
                 __syncthreads();
             }
         }
-        for (uint32_t i = tid; i < U; i += kGatherThreads) out[i] = table[i] >> keyShift;
-    }
-    if (b.perm && !b.lenOrder) {
-        // the alignment's order is the list's; an entry is the position with
-        // the predicted orientation in bit 31
-        __syncthreads();
-        for (uint32_t i = tid; i < U; i += kGatherThreads) b.perm[off + i] = i | (tagged ? (sk[i] & 1u) << 31 : 0u);
-    } else if (b.perm) {
-        // the alignment's order: positions grouped by words per read
-        // (length / 32, up to 8) and within that by predicted orientation,
-        // in position order within a group -- a counting sort by one warp;
-        // the list's space holds the groups.  An entry is the position, with
-        // the predicted orientation in bit 31.
-        __syncthreads();
-        if (tid < 32) {
-            constexpr unsigned kFull = 0xffffffffu;
-            constexpr int kGroups = 18;
-            const int lane = tid;
-            uint32_t cnt = 0;  // lane g < kGroups: size of group g, then its start
-            for (uint32_t i0 = 0; i0 < U; i0 += 32) {
-                const uint32_t i = i0 + (uint32_t)lane;
-                uint32_t g = kGroups;
-                if (i < U) {
-                    const uint32_t key = sk[i];
-                    g = 2 * min((uint32_t)st.len[key >> keyShift] >> 5, 8u) + (tagged ? key & 1u : 0u);
-                }
-                __syncwarp();  // sk may be `list`: every lane has its key before the groups overwrite it
-                if (i < U) list[i] = g;
-#pragma unroll
-                for (int v = 0; v < kGroups; v++) {
-                    const uint32_t n = __popc(__ballot_sync(kFull, g == (uint32_t)v));
-                    if (lane == v) cnt += n;
-                }
-            }
-            uint32_t start = cnt;  // exclusive scan over the groups
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const uint32_t y = __shfl_up_sync(kFull, start, d);
-                if (lane >= d) start += y;
-            }
-            start -= cnt;
-            for (uint32_t i0 = 0; i0 < U; i0 += 32) {
-                const uint32_t i = i0 + (uint32_t)lane;
-                const uint32_t g = i < U ? list[i] : kGroups;
-                uint32_t r = 0;
-#pragma unroll
-                for (int v = 0; v < kGroups; v++) {
-                    const uint32_t m = __ballot_sync(kFull, g == (uint32_t)v);
-                    const uint32_t s0 = __shfl_sync(kFull, start, v);
-                    if (g == (uint32_t)v) r = s0 + __popc(m & ((1u << lane) - 1u));
-                    if (lane == v) start += __popc(m);
-                }
-                if (i < U) b.perm[off + r] = i | ((g & 1u) << 31);
-            }
-        }
+        for (uint32_t i = tid; i < U; i += kGatherThreads) out[i] = table[i];
     }
     if (tid == 0) {
         b.ncand[a] = U;
+        if (b.units && U) {  // the anchor's alignment units
+            const uint32_t parts = (U + kAlignUnit - 1) / kAlignUnit;
+            const unsigned int at = atomicAdd(b.unitCount, parts);
+            for (uint32_t k = 0; k < parts; k++) b.units[at + k] = make_uint2((uint32_t)a, k);
+        }
         atomicAdd(&b.counters[kCounterRaw], (unsigned long long)raw);
         atomicAdd(&b.counters[kCounterUnique], (unsigned long long)U);
     }
@@ -430,6 +353,7 @@ __global__ void __launch_bounds__(kGatherThreads, 16) gather_unique_kernel(Store
     const int a = blockIdx.x;
     const uint64_t first = batch_first(b);
     const uint2 r = gather_range(b, rawOff, a, first, true);
+    if (b.units && threadIdx.x == 0) b.nfinal[a] = 0;  // the alignment counts an anchor's finished units in it
     if (r.y == 0) {
         if (threadIdx.x == 0) b.ncand[a] = 0;
         return;
@@ -571,10 +495,8 @@ cudaError_t launch_run_pack(const unsigned long long* keys, const uint32_t* star
 
 cudaError_t launch_run_fill(const unsigned long long* keys, const uint32_t* ids, uint64_t n, const uint32_t* runOf,
                             const uint32_t* start, uint32_t runs, const unsigned long long* packedScan, int maxValues,
-                            uint32_t* values, Slot* fin, uint32_t finMask, cudaStream_t s, uint32_t* rawAll,
-                            uint32_t idMask) {
-    run_values_kernel<<<grid_of(n), 256, 0, s>>>(keys, ids, n, runOf, start, packedScan, maxValues, values, rawAll,
-                                                 idMask);
+                            uint32_t* values, Slot* fin, uint32_t finMask, cudaStream_t s, uint32_t* rawAll) {
+    run_values_kernel<<<grid_of(n), 256, 0, s>>>(keys, ids, n, runOf, start, packedScan, maxValues, values, rawAll);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     run_place_kernel<<<grid_of(runs), 256, 0, s>>>(keys, start, runs, packedScan, maxValues, fin, finMask);

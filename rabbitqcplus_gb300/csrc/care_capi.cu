@@ -514,34 +514,31 @@ int build_tables(cg_ctx* c) {
     CG_CUDA(c, launch_signatures(st, c->k, c->nmaps, c->sig.as<unsigned long long>(), c->stream));
     if (n > 0x40000000ull) return fail(c, CG_ERR_UNSUPPORTED, "too many reads for one table (%llu)",
                                        (unsigned long long)n);
-    // The maps are built in waves of up to kTableStreams maps, one stream and
-    // one set of sorting buffers per map of a wave (as many as a quarter of the
-    // free memory holds).  A wave sorts its maps' (key, read id) pairs and
-    // marks their runs of equal keys; one synchronisation reads the run
-    // counts, a second the kept keys' and values' totals, which size one slab
-    // for the wave's slots and values; then the wave fills its maps.  The
-    // next wave's sorts follow on the same streams.
-    constexpr int kTableStreams = 8;
+    // The maps are built in waves.  A wave's maps lie one after the other and
+    // every launch covers all of them: their (key, read id) pairs are sorted,
+    // the runs of equal keys marked and, after one synchronisation for the number
+    // of runs, packed; a second one reads the maps' totals, which size one slab
+    // for the wave's slots and values; then the maps are filled.  A wave has up to
+    // 64M pairs or 8 maps (enough to fill the GPU: the build of 1M reads takes
+    // 11.0, 10.5 and 9.9 ms in waves of 8, 16 and 48 maps, of 4M reads 40.7, 40.9
+    // and 39.8 in waves of 8, 8 and 16), what a quarter of the free memory holds,
+    // and fewer than 2^32 pairs.
+    constexpr uint64_t kWavePairs = 64ull << 20;
     const int bits = std::min(64, 2 * c->k);  // the signatures keep 2k bits
-    const size_t perStream = n * (2 * sizeof(unsigned long long) + 2 * sizeof(uint32_t)) +
-                             2 * (n + 1) * sizeof(uint32_t) + (n + 1) * sizeof(unsigned long long) +
-                             radix_sort_temp_bytes(n) + scan_tmp_bytes(n + 1);
+    const size_t perMap = n * (2 * sizeof(unsigned long long) + 3 * sizeof(uint32_t)) + radix_sort_temp_bytes(n, 1) +
+                          scan_tmp_bytes(n + 1);
     size_t freeB = 0, totalB = 0;
     CG_CUDA(c, cudaMemGetInfo(&freeB, &totalB));
-    const int S = (int)std::max<size_t>(1, std::min<size_t>({(size_t)kTableStreams, (size_t)c->nmaps,
-                                                            freeB / 4 / std::max<size_t>(perStream, 1)}));
-    struct Lane {
-        cudaStream_t stream = nullptr;
-        cudaEvent_t done = nullptr;
-        DevBuf keys, ids, keysAlt, idsAlt, runOf, start, packed, sortTmp, scanTmp;
-    };
-    std::vector<Lane> lanes(S);
-    unsigned long long* hTot = nullptr;  // per map: (kept keys << 32) | values, then the runs (u32)
+    const uint64_t reads = std::max<uint64_t>(n, 1);
+    const int S = (int)std::max<uint64_t>(
+        1, std::min<uint64_t>({(uint64_t)c->nmaps, std::max<uint64_t>(8, kWavePairs / reads),
+                               freeB / 4 / std::max<size_t>(perMap, 1), 0xfffffffeull / reads}));
+    DevBuf keys, ids, keysAlt, idsAlt, runOf, sortTmp, scanTmp, totals;
+    ulonglong2* hTot = nullptr;  // per map of a wave: (kept keys << 32) | values, first value; then the runs
     release_tables(c);
     c->maps.resize(c->nmaps);
     c->stats.table_keys = 0;
     c->stats.table_values = 0;
-    cudaEvent_t sigDone = nullptr;
     int rc = CG_OK;
     auto cuda = [&](cudaError_t e, const char* what) {
         if (e != cudaSuccess && rc == CG_OK)
@@ -550,118 +547,87 @@ int build_tables(cg_ctx* c) {
         return rc == CG_OK;
     };
     // the batched driver's raw id count of every read, summed as the maps are
-    // filled (finished by ensure_batched_state); cleared before the lanes start
+    // filled (finished by ensure_batched_state)
     uint32_t* rawAll = nullptr;
     c->haveRawAll = false;
-    if (c->o.driver == CG_DRIVER_BATCHED &&
-        cuda(c->rawAll.ensure(std::max<uint64_t>(n, 1) * sizeof(uint32_t)), "raw counts") &&
+    if (c->o.driver == CG_DRIVER_BATCHED && cuda(c->rawAll.ensure(reads * sizeof(uint32_t)), "raw counts") &&
         cuda(cudaMemsetAsync(c->rawAll.p, 0, n * sizeof(uint32_t), c->stream), "raw counts"))
         rawAll = c->rawAll.as<uint32_t>();
-    if (rc == CG_OK &&
-        cuda(cudaMallocHost(&hTot, 2 * (size_t)c->nmaps * sizeof(unsigned long long)), "host totals") &&
-        cuda(cudaEventCreateWithFlags(&sigDone, cudaEventDisableTiming), "event") &&
-        cuda(cudaEventRecord(sigDone, c->stream), "event")) {
-        for (Lane& l : lanes) {
-            if (!cuda(cudaStreamCreateWithFlags(&l.stream, cudaStreamNonBlocking), "stream") ||
-                !cuda(cudaEventCreateWithFlags(&l.done, cudaEventDisableTiming), "event") ||
-                !cuda(cudaStreamWaitEvent(l.stream, sigDone, 0), "wait") ||
-                !cuda(l.keys.ensure(std::max<uint64_t>(n, 1) * sizeof(unsigned long long)), "sorted keys") ||
-                !cuda(l.ids.ensure(std::max<uint64_t>(n, 1) * sizeof(uint32_t)), "sorted ids") ||
-                !cuda(l.keysAlt.ensure(std::max<uint64_t>(n, 1) * sizeof(unsigned long long)), "sort keys") ||
-                !cuda(l.idsAlt.ensure(std::max<uint64_t>(n, 1) * sizeof(uint32_t)), "sort ids") ||
-                !cuda(l.runOf.ensure((n + 1) * sizeof(uint32_t)), "runs") ||
-                !cuda(l.start.ensure((n + 1) * sizeof(uint32_t)), "run starts") ||
-                !cuda(l.packed.ensure((n + 1) * sizeof(unsigned long long)), "run lengths") ||
-                !cuda(l.sortTmp.ensure(radix_sort_temp_bytes(n)), "sort") ||
-                !cuda(l.scanTmp.ensure(scan_tmp_bytes(n + 1)), "scan"))
-                break;
-        }
-    }
-    uint32_t* hRuns = reinterpret_cast<uint32_t*>(hTot + c->nmaps);
-    for (int w0 = 0; w0 < c->nmaps && rc == CG_OK; w0 += S) {
-        const int w1 = std::min(c->nmaps, w0 + S);
-        for (int h = w0; h < w1 && rc == CG_OK; h++) {
-            Lane& l = lanes[h - w0];
-            const unsigned long long* keys = c->sig.as<unsigned long long>() + (uint64_t)h * n;
-            cudaError_t e = radix_sort_pairs(keys, n, bits, l.keys.as<unsigned long long>(), l.ids.as<uint32_t>(),
-                                             l.keysAlt.as<unsigned long long>(), l.idsAlt.as<uint32_t>(),
-                                             l.sortTmp.p, l.stream);
-            if (e == cudaSuccess) e = launch_run_heads(l.keys.as<unsigned long long>(), n, l.runOf.as<uint32_t>(),
-                                                       l.stream);
-            if (e == cudaSuccess) e = scan_exclusive_u32(l.runOf.as<uint32_t>(), n + 1, l.scanTmp.p, l.stream);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(hRuns + h, l.runOf.as<uint32_t>() + n, sizeof(uint32_t),
-                                                      cudaMemcpyDeviceToHost, l.stream);
-            cuda(e, "sort");
-        }
-        for (int h = w0; h < w1 && rc == CG_OK; h++) cuda(cudaStreamSynchronize(lanes[h - w0].stream), "sort");
-        for (int h = w0; h < w1 && rc == CG_OK; h++) {
-            Lane& l = lanes[h - w0];
-            const uint32_t runs = hRuns[h];
-            cudaError_t e = launch_run_starts(l.keys.as<unsigned long long>(), n, l.runOf.as<uint32_t>(),
-                                              l.start.as<uint32_t>(), l.stream);
-            if (e == cudaSuccess) e = launch_run_pack(l.keys.as<unsigned long long>(), l.start.as<uint32_t>(), runs,
-                                                      c->maxValuesPerKey, l.packed.as<unsigned long long>(), l.stream);
-            if (e == cudaSuccess) e = scan_exclusive_u64(l.packed.as<unsigned long long>(), (size_t)runs + 1,
-                                                         l.scanTmp.p, l.stream);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(hTot + h, l.packed.as<unsigned long long>() + runs,
-                                                      sizeof(unsigned long long), cudaMemcpyDeviceToHost, l.stream);
-            cuda(e, "runs");
-        }
-        for (int h = w0; h < w1 && rc == CG_OK; h++) cuda(cudaStreamSynchronize(lanes[h - w0].stream), "runs");
-        if (rc != CG_OK) break;
+    const uint64_t pairs = (uint64_t)S * reads;
+    // packed run lengths and run starts take the sort's scratch, free after it
+    const bool ready = rc == CG_OK && cuda(cudaMallocHost(&hTot, (kMaxMaps + 1) * sizeof(ulonglong2)), "host totals") &&
+                       cuda(keys.ensure(pairs * sizeof(unsigned long long)), "sorted keys") &&
+                       cuda(ids.ensure(pairs * sizeof(uint32_t)), "sorted ids") &&
+                       cuda(keysAlt.ensure((pairs + 1) * sizeof(unsigned long long)), "sort keys") &&
+                       cuda(idsAlt.ensure((pairs + 1) * sizeof(uint32_t)), "sort ids") &&
+                       cuda(runOf.ensure((pairs + 1) * sizeof(uint32_t)), "runs") &&
+                       cuda(sortTmp.ensure(radix_sort_temp_bytes(n, S)), "sort") &&
+                       cuda(scanTmp.ensure(scan_tmp_bytes(pairs + 1)), "scan") &&
+                       cuda(totals.ensure(kMaxMaps * sizeof(ulonglong2)), "totals");
+    unsigned long long* const dKeys = keys.as<unsigned long long>();
+    uint32_t* const dIds = ids.as<uint32_t>();
+    unsigned long long* const packed = keysAlt.as<unsigned long long>();
+    uint32_t* const start = idsAlt.as<uint32_t>();
+    uint32_t* const dRuns = runOf.as<uint32_t>();
+    for (int w0 = 0; ready && w0 < c->nmaps && rc == CG_OK; w0 += S) {
+        const int maps = std::min(S, c->nmaps - w0);
+        const uint64_t total = (uint64_t)maps * n;
+        uint32_t* const hRuns = reinterpret_cast<uint32_t*>(hTot + kMaxMaps);
+        cudaError_t e = radix_sort_pairs(c->sig.as<unsigned long long>() + (uint64_t)w0 * n, n, maps, bits, dKeys, dIds,
+                                         packed, start, sortTmp.p, c->stream);
+        if (e == cudaSuccess) e = launch_run_heads(dKeys, n, maps, dRuns, c->stream);
+        if (e == cudaSuccess) e = scan_exclusive_u32(dRuns, total + 1, scanTmp.p, c->stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(hRuns, dRuns + total, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess) e = launch_run_starts(dKeys, n, maps, dRuns, start, c->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+        if (!cuda(e, "sort")) break;
+        const uint32_t runs = *hRuns;
+        e = launch_run_pack(dKeys, start, runs, c->maxValuesPerKey, packed, c->stream);
+        if (e == cudaSuccess) e = scan_exclusive_u64(packed, (size_t)runs + 1, scanTmp.p, c->stream);
+        if (e == cudaSuccess) e = launch_run_totals(dRuns, n, maps, packed, totals.as<ulonglong2>(), c->stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(hTot, totals.p, maps * sizeof(ulonglong2), cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+        if (!cuda(e, "runs")) break;
         uint64_t slotTotal = 0, valueTotal = 0;
-        std::vector<uint64_t> valueOff(w1 - w0);
-        for (int h = w0; h < w1; h++) {
-            MapTable& mt = c->maps[h];
-            mt.keys = hTot[h] >> 32;
-            mt.nvalues = hTot[h] & 0xffffffffull;
+        for (int m = 0; m < maps; m++) {
+            MapTable& mt = c->maps[w0 + m];
+            mt.keys = hTot[m].x >> 32;
+            mt.nvalues = hTot[m].x & 0xffffffffull;
             mt.cap = pow2_at_least(std::max<uint64_t>(2 * mt.keys, 64));
             slotTotal += mt.cap;
-        }
-        for (int h = w0; h < w1; h++) {
-            valueOff[h - w0] = valueTotal;
-            valueTotal += (std::max<uint64_t>(c->maps[h].nvalues, 1) + 3) / 4 * 4;  // 16-byte aligned per map
+            valueTotal += mt.nvalues;
         }
         c->tableSlabs.emplace_back();
         DevBuf& slab = c->tableSlabs.back();
-        if (!cuda(slab.ensure(slotTotal * sizeof(Slot) + valueTotal * sizeof(uint32_t)), "slab")) break;
-        Slot* slotBase = slab.as<Slot>();
-        uint32_t* valueBase = reinterpret_cast<uint32_t*>(slotBase + slotTotal);
-        for (int h = w0; h < w1 && rc == CG_OK; h++) {
-            Lane& l = lanes[h - w0];
-            MapTable& mt = c->maps[h];
-            mt.slots = slotBase;
-            slotBase += mt.cap;
-            mt.values = valueBase + valueOff[h - w0];
-            cudaError_t e = launch_table_init(mt.slots, mt.cap, l.stream);
-            if (e == cudaSuccess) e = launch_run_fill(l.keys.as<unsigned long long>(), l.ids.as<uint32_t>(), n,
-                                                      l.runOf.as<uint32_t>(), l.start.as<uint32_t>(),
-                                                      hRuns[h], l.packed.as<unsigned long long>(),
-                                                      c->maxValuesPerKey, mt.values, mt.slots,
-                                                      (uint32_t)(mt.cap - 1), l.stream, rawAll);
-            if (!cuda(e, "build")) break;
+        if (!cuda(slab.ensure(slotTotal * sizeof(Slot) + std::max<uint64_t>(valueTotal, 1) * sizeof(uint32_t)), "slab"))
+            break;
+        Slot* slots = slab.as<Slot>();
+        uint32_t* const values = reinterpret_cast<uint32_t*>(slots + slotTotal);
+        e = cudaMemsetAsync(slots, 0xff, slotTotal * sizeof(Slot), c->stream);  // every key empty
+        WaveTables wave{};
+        for (int m = 0; m < maps; m++) {
+            MapTable& mt = c->maps[w0 + m];
+            mt.slots = slots;
+            mt.values = values + hTot[m].y;
+            slots += mt.cap;
+            wave.slots[m] = mt.slots;
+            wave.mask[m] = (uint32_t)(mt.cap - 1);
+            wave.firstValue[m] = (uint32_t)hTot[m].y;
             c->stats.table_keys += mt.keys;
             c->stats.table_values += mt.nvalues;
-            c->tables.slots[h] = mt.slots;
-            c->tables.values[h] = mt.values;
-            c->tables.mask[h] = (uint32_t)(mt.cap - 1);
+            c->tables.slots[w0 + m] = mt.slots;
+            c->tables.values[w0 + m] = mt.values;
+            c->tables.mask[w0 + m] = wave.mask[m];
         }
+        if (e == cudaSuccess)
+            e = launch_run_fill(dKeys, dIds, n, maps, dRuns, start, runs, packed, c->maxValuesPerKey, values, wave,
+                                c->stream, rawAll);
+        cuda(e, "build");
     }
-    // the context's stream continues after every wave's last work
-    for (Lane& l : lanes) {
-        if (l.stream && l.done && cudaEventRecord(l.done, l.stream) == cudaSuccess)
-            cuda(cudaStreamWaitEvent(c->stream, l.done, 0), "join");
-    }
-    cudaError_t e = cudaStreamSynchronize(c->stream);
-    for (Lane& l : lanes) {
-        if (l.stream) cudaStreamSynchronize(l.stream);
-        for (DevBuf* d : {&l.keys, &l.ids, &l.keysAlt, &l.idsAlt, &l.runOf, &l.start, &l.packed, &l.sortTmp,
-                          &l.scanTmp})
-            d->release();
-        if (l.done) cudaEventDestroy(l.done);
-        if (l.stream) cudaStreamDestroy(l.stream);
-    }
-    if (sigDone) cudaEventDestroy(sigDone);
+    const cudaError_t e = cudaStreamSynchronize(c->stream);
+    for (DevBuf* d : {&keys, &ids, &keysAlt, &idsAlt, &runOf, &sortTmp, &scanTmp, &totals}) d->release();
     if (hTot) cudaFreeHost(hTot);
     if (rc != CG_OK) return rc;
     CG_CUDA(c, e);

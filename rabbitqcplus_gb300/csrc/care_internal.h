@@ -158,29 +158,38 @@ cudaError_t launch_len_range(const uint16_t* len, uint64_t n, unsigned int* out,
 cudaError_t launch_quality_bins(uint8_t* qual, const uint16_t* len, uint64_t n, int lmax, int bits, cudaStream_t s);
 
 // hash tables
-cudaError_t launch_table_init(Slot* t, uint64_t cap, cudaStream_t s);
-// one map's (key, read id) pairs sorted by key (read ids ascending within a
-// key) into keys/vals, from the first `bits` bits of keysIn's keys (values
-// 0 .. n - 1); keysAlt/valsAlt hold n pairs of scratch, temp
-// radix_sort_temp_bytes(n) bytes
-size_t radix_sort_temp_bytes(uint64_t n);
-cudaError_t radix_sort_pairs(const unsigned long long* keysIn, uint64_t n, int bits, unsigned long long* keys,
+// The maps of a build wave, one after the other: each map's n (key, read id)
+// pairs sorted by key (read ids ascending within a key) into keys/vals
+// [maps][n], from the first `bits` bits of keysIn's keys (values 0 .. n - 1 in
+// every map); keysAlt/valsAlt hold as many pairs of scratch, temp
+// radix_sort_temp_bytes(n, maps) bytes; n * maps < 2^32
+size_t radix_sort_temp_bytes(uint64_t n, int maps);
+cudaError_t radix_sort_pairs(const unsigned long long* keysIn, uint64_t n, int maps, int bits, unsigned long long* keys,
                              uint32_t* vals, unsigned long long* keysAlt, uint32_t* valsAlt, void* temp,
                              cudaStream_t s);
-// runs of equal keys in sorted pairs: runOf[0..n] (scanned in place by the
-// caller into run indices, runOf[n] = number of runs R), start[0..R],
-// packed[0..R] (scanned by the caller into value offsets and totals), then
-// the kept runs' ids into values and their keys into the final table (and,
-// with rawAll, each kept id's bucket size added to rawAll[id])
-cudaError_t launch_run_heads(const unsigned long long* keys, uint64_t n, uint32_t* runOf, cudaStream_t s);
-cudaError_t launch_run_starts(const unsigned long long* keys, uint64_t n, const uint32_t* runOf, uint32_t* start,
-                              cudaStream_t s);
+// Runs of equal keys in sorted pairs (total = n * maps): runOf[0..total]
+// (scanned in place by the caller into run indices, runOf[total] = number of
+// runs R), start[0..R], packed[0..R] (scanned by the caller into value offsets
+// of the wave), then per map {kept keys << 32 | values, offset of its first
+// value} into totals, the kept runs' ids into the wave's values and their keys
+// into the maps' tables (and, with rawAll, each kept id's bucket size added to
+// rawAll[id]).
+struct WaveTables {
+    Slot* slots[kMaxMaps];
+    uint32_t mask[kMaxMaps];
+    uint32_t firstValue[kMaxMaps];  // a map's first value in the wave's values
+};
+cudaError_t launch_run_heads(const unsigned long long* keys, uint64_t n, int maps, uint32_t* runOf, cudaStream_t s);
+cudaError_t launch_run_starts(const unsigned long long* keys, uint64_t n, int maps, const uint32_t* runOf,
+                              uint32_t* start, cudaStream_t s);
 cudaError_t launch_run_pack(const unsigned long long* keys, const uint32_t* start, uint32_t runs, int maxValues,
                             unsigned long long* packed, cudaStream_t s);
-cudaError_t launch_run_fill(const unsigned long long* keys, const uint32_t* ids, uint64_t n, const uint32_t* runOf,
-                            const uint32_t* start, uint32_t runs, const unsigned long long* packedScan, int maxValues,
-                            uint32_t* values, Slot* fin, uint32_t finMask, cudaStream_t s,
-                            uint32_t* rawAll = nullptr);
+cudaError_t launch_run_totals(const uint32_t* runOf, uint64_t n, int maps, const unsigned long long* packedScan,
+                              ulonglong2* totals, cudaStream_t s);
+cudaError_t launch_run_fill(const unsigned long long* keys, const uint32_t* ids, uint64_t n, int maps,
+                            const uint32_t* runOf, const uint32_t* start, uint32_t runs,
+                            const unsigned long long* packedScan, int maxValues, uint32_t* values, WaveTables tables,
+                            cudaStream_t s, uint32_t* rawAll = nullptr);
 
 // correction batch
 struct BatchArg {

@@ -1,11 +1,15 @@
 // Stable LSD radix sort of (64-bit key, 32-bit value) pairs, for the minhash
-// tables' build: one map's (key, read id) pairs sorted by key with the read
-// ids ascending within a key, so that every bucket comes out in the order the
-// reference's group-by-key gives it (include/groupbykey.hpp:69-250).
+// tables' build: the (key, read id) pairs of several maps, each map's sorted by
+// key with the read ids ascending within a key, so that every bucket comes out
+// in the order the reference's group-by-key gives it
+// (include/groupbykey.hpp:69-250).
 //
-// Per 8-bit digit, three launches: (1) the digit counts of every tile of
-// 2048 elements, (2) an exclusive scan of the counts in (digit, tile) order,
-// (3) a scatter.  The scatter ranks each element among the tile's elements
+// The maps lie one after the other in the arrays and every launch covers all of
+// them (at 200k reads a map alone fills a sixth of the GPU, and its kernels end
+// before the next launch arrives).  Per 8-bit digit: (1) the digit counts of
+// every tile of 2048 elements, (2) an exclusive scan of the counts in (map,
+// digit, tile) order, whose values are positions in the concatenated output
+// since each map's counts add up to its n elements, (3) a scatter.  The scatter ranks each element among the tile's elements
 // of the same digit in element order -- warps take contiguous sub-tiles,
 // lanes with equal digits find each other with a warp match, each warp keeps
 // its digit counts in shared memory -- stages the tile in digit order in
@@ -32,7 +36,8 @@ __device__ __forceinline__ uint32_t digit_of(unsigned long long k, int shift) {
     return (uint32_t)(k >> shift) & (kDigits - 1);
 }
 
-// counts[d * tiles + t] = elements of tile t whose digit is d
+// counts[(m * kDigits + d) * tiles + t] = elements of map m's tile t whose
+// digit is d; block (t, m)
 __global__ void __launch_bounds__(kSortThreads) radix_count_kernel(const unsigned long long* __restrict__ keys,
                                                                    uint64_t n, int shift, uint32_t* __restrict__ counts,
                                                                    uint32_t tiles) {
@@ -40,17 +45,19 @@ __global__ void __launch_bounds__(kSortThreads) radix_count_kernel(const unsigne
     h[threadIdx.x] = 0;
     __syncthreads();
     const uint64_t base = (uint64_t)blockIdx.x * kSortTile;
+    keys += (uint64_t)blockIdx.y * n;
 #pragma unroll
     for (int j = 0; j < kSortItems; j++) {
         const uint64_t i = base + (uint64_t)(j * kSortThreads) + threadIdx.x;
         if (i < n) atomicAdd(&h[digit_of(keys[i], shift)], 1u);
     }
     __syncthreads();
-    counts[(uint64_t)threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
+    counts[((uint64_t)blockIdx.y * kDigits + threadIdx.x) * tiles + blockIdx.x] = h[threadIdx.x];
 }
 
-// One tile per block.  offsets = the exclusive scan of radix_count_kernel's
-// counts; vals == nullptr stands for the values 0, 1, ..., n - 1.
+// One tile per block (t, m).  offsets = the exclusive scan of
+// radix_count_kernel's counts (positions in keysOut, valsOut); vals == nullptr
+// stands for the values 0, 1, ..., n - 1 in every map.
 __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(
     const unsigned long long* __restrict__ keys, const uint32_t* __restrict__ vals, uint64_t n, int shift,
     const uint32_t* __restrict__ offsets, uint32_t tiles, unsigned long long* __restrict__ keysOut,
@@ -62,6 +69,8 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(
     __shared__ unsigned long long skey[kSortTile];
     __shared__ uint32_t sval[kSortTile];
     const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5);
+    keys += (uint64_t)blockIdx.y * n;
+    if (vals) vals += (uint64_t)blockIdx.y * n;
     for (int i = threadIdx.x; i < kSortWarps * kDigits; i += kSortThreads) (&wcount[0][0])[i] = 0;
     __syncthreads();
     // warp w: elements tile + w * 32 * kSortItems + 32 j + lane, j = 0 .. kSortItems - 1
@@ -107,7 +116,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(
         if (lane >= s) incl += y;
     }
     if (lane == 31) warpSum[warp] = incl;
-    globalStart[d] = offsets[(uint64_t)d * tiles + blockIdx.x];
+    globalStart[d] = offsets[((uint64_t)blockIdx.y * kDigits + d) * tiles + blockIdx.x];
     __syncthreads();
     uint32_t before = 0;
     for (int w = 0; w < warp; w++) before += warpSum[w];
@@ -137,19 +146,20 @@ size_t align16(size_t b) { return (b + 15) / 16 * 16; }
 
 }  // namespace
 
-size_t radix_sort_temp_bytes(uint64_t n) {
+size_t radix_sort_temp_bytes(uint64_t n, int maps) {
     const uint64_t tiles = (n + kSortTile - 1) / kSortTile;
-    const size_t counts = (size_t)kDigits * (size_t)std::max<uint64_t>(tiles, 1);
+    const size_t counts = (size_t)kDigits * (size_t)std::max<uint64_t>(tiles, 1) * (size_t)maps;
     return align16(counts * sizeof(uint32_t)) + scan_tmp_bytes(counts);
 }
 
-cudaError_t radix_sort_pairs(const unsigned long long* keysIn, uint64_t n, int bits, unsigned long long* keys,
+cudaError_t radix_sort_pairs(const unsigned long long* keysIn, uint64_t n, int maps, int bits, unsigned long long* keys,
                              uint32_t* vals, unsigned long long* keysAlt, uint32_t* valsAlt, void* temp,
                              cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    if (n > 0xffffffffull) return cudaErrorInvalidValue;
+    if (n * (uint64_t)maps > 0xffffffffull) return cudaErrorInvalidValue;
     const uint32_t tiles = (uint32_t)((n + kSortTile - 1) / kSortTile);
-    const size_t ncounts = (size_t)kDigits * tiles;
+    const size_t ncounts = (size_t)kDigits * tiles * (size_t)maps;
+    const dim3 grid(tiles, (unsigned)maps);
     uint32_t* counts = static_cast<uint32_t*>(temp);
     void* scanTmp = static_cast<unsigned char*>(temp) + align16(ncounts * sizeof(uint32_t));
     const int passes = std::max(1, (std::min(bits, 64) + 7) / 8);
@@ -160,12 +170,12 @@ cudaError_t radix_sort_pairs(const unsigned long long* keysIn, uint64_t n, int b
         const bool toMain = ((passes - 1 - p) & 1) == 0;
         unsigned long long* ko = toMain ? keys : keysAlt;
         uint32_t* vo = toMain ? vals : valsAlt;
-        radix_count_kernel<<<tiles, kSortThreads, 0, s>>>(ki, n, 8 * p, counts, tiles);
+        radix_count_kernel<<<grid, kSortThreads, 0, s>>>(ki, n, 8 * p, counts, tiles);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         e = scan_exclusive_u32(counts, ncounts, scanTmp, s);
         if (e != cudaSuccess) return e;
-        radix_scatter_kernel<<<tiles, kSortThreads, 0, s>>>(ki, vi, n, 8 * p, counts, tiles, ko, vo);
+        radix_scatter_kernel<<<grid, kSortThreads, 0, s>>>(ki, vi, n, 8 * p, counts, tiles, ko, vo);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         ki = ko;

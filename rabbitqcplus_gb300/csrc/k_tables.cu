@@ -23,21 +23,14 @@ namespace cg {
 
 namespace {
 
-__global__ void table_init_kernel(Slot* __restrict__ t, uint64_t cap) {
-    const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < cap) {
-        t[s].key = kEmptyKey;
-        t[s].offset = 0;
-        t[s].count = 0;
-    }
-}
-
 // ---------------------------------------------------------------- runs of sorted pairs
 //
-// keys/ids: one map's pairs sorted by key.  runOf[i] = 1 where element i
-// starts a run (runOf[n] = 0); after an exclusive scan over n + 1 entries,
-// runOf[i + 1] - 1 is element i's run and runOf[n] the number of runs R.
-// start[r] = first element of run r, start[R] = n.
+// keys/ids: the pairs of a wave of maps, n per map, each map's sorted by key.
+// runOf[i] = 1 where element i starts a run (a map's first element does;
+// runOf[total] = 0); after an exclusive scan over total + 1 entries, runOf[i +
+// 1] - 1 is element i's run and runOf[total] the number of runs R.  start[r] =
+// first element of run r, start[R] = total.  The kernels over elements take map
+// blockIdx.y.
 
 __device__ __forceinline__ bool run_kept(unsigned long long key, uint32_t len, int maxValues) {
     const uint32_t upper = (uint32_t)min(maxValues, kMaxBucket);
@@ -46,17 +39,19 @@ __device__ __forceinline__ bool run_kept(unsigned long long key, uint32_t len, i
 
 __global__ void run_head_kernel(const unsigned long long* __restrict__ keys, uint64_t n,
                                 uint32_t* __restrict__ runOf) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > n) return;
-    runOf[i] = (i < n && (i == 0 || keys[i] != keys[i - 1])) ? 1u : 0u;
+    const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, i = (uint64_t)blockIdx.y * n + j;
+    if (j < n) runOf[i] = j == 0 || keys[i] != keys[i - 1] ? 1u : 0u;
+    if (j == 0 && blockIdx.y == gridDim.y - 1) runOf[(uint64_t)gridDim.y * n] = 0u;
 }
 
 __global__ void run_start_kernel(const unsigned long long* __restrict__ keys, uint64_t n,
                                  const uint32_t* __restrict__ runOf, uint32_t* __restrict__ start) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > n) return;
-    if (i == n) start[runOf[n]] = (uint32_t)n;
-    else if (i == 0 || keys[i] != keys[i - 1]) start[runOf[i]] = (uint32_t)i;
+    const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, i = (uint64_t)blockIdx.y * n + j;
+    if (j < n && (j == 0 || keys[i] != keys[i - 1])) start[runOf[i]] = (uint32_t)i;
+    if (j == 0 && blockIdx.y == gridDim.y - 1) {
+        const uint64_t total = (uint64_t)gridDim.y * n;
+        start[runOf[total]] = (uint32_t)total;
+    }
 }
 
 // packed[r] = (1 << 32) | length for a kept run, else 0; packed[R] = 0
@@ -72,8 +67,17 @@ __global__ void run_pack_kernel(const unsigned long long* __restrict__ keys, con
     packed[r] = run_kept(keys[s0], len, maxValues) ? ((1ull << 32) | len) : 0ull;
 }
 
-// packedScan = exclusive scan of run_pack_kernel's output: the read ids of
-// every kept run, in order, at its value offset.  With rawAll set, each kept
+// packedScan = exclusive scan of run_pack_kernel's output.  totals[m] = map m's
+// {kept keys << 32 | values, offset of its first value}.
+__global__ void run_totals_kernel(const uint32_t* __restrict__ runOf, uint64_t n, int maps,
+                                  const unsigned long long* __restrict__ packedScan, ulonglong2* __restrict__ totals) {
+    const int m = (int)threadIdx.x;
+    if (m >= maps) return;
+    const unsigned long long p0 = packedScan[runOf[(uint64_t)m * n]], p1 = packedScan[runOf[(uint64_t)(m + 1) * n]];
+    totals[m] = make_ulonglong2(p1 - p0, p0 & 0xffffffffull);
+}
+
+// The read ids of every kept run, in order, at its value offset.  With rawAll set, each kept
 // id also adds its run's length -- its bucket's size, the ids a query of that
 // read finds in this map -- to rawAll[id] (atomic: the maps of a build wave
 // run concurrently).
@@ -81,8 +85,8 @@ __global__ void run_values_kernel(const unsigned long long* __restrict__ keys, c
                                   uint64_t n, const uint32_t* __restrict__ runOf, const uint32_t* __restrict__ start,
                                   const unsigned long long* __restrict__ packedScan, int maxValues,
                                   uint32_t* __restrict__ values, uint32_t* __restrict__ rawAll) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, i = (uint64_t)blockIdx.y * n + j;
+    if (j >= n) return;
     const uint32_t r = runOf[i + 1] - 1u;
     const uint32_t s0 = start[r], len = start[r + 1] - s0;
     if (!run_kept(keys[i], len, maxValues)) return;
@@ -91,20 +95,22 @@ __global__ void run_values_kernel(const unsigned long long* __restrict__ keys, c
     if (rawAll) atomicAdd(&rawAll[id], len);
 }
 
-// every kept run's key into the final table with its value offset and length
+// every kept run's key into its map's table with its value offset and length
 __global__ void run_place_kernel(const unsigned long long* __restrict__ keys, const uint32_t* __restrict__ start,
                                  uint32_t runs, const unsigned long long* __restrict__ packedScan, int maxValues,
-                                 Slot* __restrict__ fin, uint32_t finMask) {
+                                 uint32_t n, WaveTables tables) {
     const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= runs) return;
     const uint32_t s0 = start[r], len = start[r + 1] - s0;
     const unsigned long long key = keys[s0];
     if (!run_kept(key, len, maxValues)) return;
+    const uint32_t m = s0 / n, finMask = tables.mask[m];
+    Slot* const fin = tables.slots[m];
     uint32_t f = slot_of(key, finMask);
     for (uint32_t probe = 0; probe <= finMask; probe++) {
         const unsigned long long old = atomicCAS(&fin[f].key, kEmptyKey, key);
         if (old == kEmptyKey) {
-            fin[f].offset = (uint32_t)(packedScan[r] & 0xffffffffull);
+            fin[f].offset = (uint32_t)(packedScan[r] & 0xffffffffull) - tables.firstValue[m];
             fin[f].count = len;
             return;
         }
@@ -469,21 +475,22 @@ __global__ void pair_flags_kernel(BatchArg b, const uint32_t* __restrict__ rawOf
 
 }  // namespace
 
-cudaError_t launch_table_init(Slot* t, uint64_t cap, cudaStream_t s) {
-    table_init_kernel<<<(unsigned)std::max<uint64_t>(1, (cap + 255) / 256), 256, 0, s>>>(t, cap);
-    return cudaGetLastError();
-}
-
 unsigned grid_of(uint64_t threads) { return (unsigned)std::max<uint64_t>(1, (threads + 255) / 256); }
 
-cudaError_t launch_run_heads(const unsigned long long* keys, uint64_t n, uint32_t* runOf, cudaStream_t s) {
-    run_head_kernel<<<grid_of(n + 1), 256, 0, s>>>(keys, n, runOf);
+cudaError_t launch_run_heads(const unsigned long long* keys, uint64_t n, int maps, uint32_t* runOf, cudaStream_t s) {
+    run_head_kernel<<<dim3(grid_of(n), (unsigned)maps), 256, 0, s>>>(keys, n, runOf);
     return cudaGetLastError();
 }
 
-cudaError_t launch_run_starts(const unsigned long long* keys, uint64_t n, const uint32_t* runOf, uint32_t* start,
-                              cudaStream_t s) {
-    run_start_kernel<<<grid_of(n + 1), 256, 0, s>>>(keys, n, runOf, start);
+cudaError_t launch_run_starts(const unsigned long long* keys, uint64_t n, int maps, const uint32_t* runOf,
+                              uint32_t* start, cudaStream_t s) {
+    run_start_kernel<<<dim3(grid_of(n), (unsigned)maps), 256, 0, s>>>(keys, n, runOf, start);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_run_totals(const uint32_t* runOf, uint64_t n, int maps, const unsigned long long* packedScan,
+                              ulonglong2* totals, cudaStream_t s) {
+    run_totals_kernel<<<1, kMaxMaps, 0, s>>>(runOf, n, maps, packedScan, totals);
     return cudaGetLastError();
 }
 
@@ -493,13 +500,15 @@ cudaError_t launch_run_pack(const unsigned long long* keys, const uint32_t* star
     return cudaGetLastError();
 }
 
-cudaError_t launch_run_fill(const unsigned long long* keys, const uint32_t* ids, uint64_t n, const uint32_t* runOf,
-                            const uint32_t* start, uint32_t runs, const unsigned long long* packedScan, int maxValues,
-                            uint32_t* values, Slot* fin, uint32_t finMask, cudaStream_t s, uint32_t* rawAll) {
-    run_values_kernel<<<grid_of(n), 256, 0, s>>>(keys, ids, n, runOf, start, packedScan, maxValues, values, rawAll);
+cudaError_t launch_run_fill(const unsigned long long* keys, const uint32_t* ids, uint64_t n, int maps,
+                            const uint32_t* runOf, const uint32_t* start, uint32_t runs,
+                            const unsigned long long* packedScan, int maxValues, uint32_t* values, WaveTables tables,
+                            cudaStream_t s, uint32_t* rawAll) {
+    run_values_kernel<<<dim3(grid_of(n), (unsigned)maps), 256, 0, s>>>(keys, ids, n, runOf, start, packedScan,
+                                                                       maxValues, values, rawAll);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    run_place_kernel<<<grid_of(runs), 256, 0, s>>>(keys, start, runs, packedScan, maxValues, fin, finMask);
+    run_place_kernel<<<grid_of(runs), 256, 0, s>>>(keys, start, runs, packedScan, maxValues, (uint32_t)n, tables);
     return cudaGetLastError();
 }
 

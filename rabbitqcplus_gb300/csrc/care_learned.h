@@ -34,12 +34,14 @@ constexpr int kMlpParamB2 = kMlpParamB1 + kMlpHidden;
 constexpr int kMlpParamB3 = kMlpParamB2 + kMlpHidden;
 constexpr int kMlpParamLoss = kMlpParamB3 + 1;
 constexpr int kMlpParams = kMlpParamLoss + 1;
+constexpr int kMlpPartStride = (kMlpParams + 3) / 4 * 4;  // floats per partial-gradient slot
 static_assert(kMlpOffB1 % 4 == 0, "bias alignment");
 
 // Adam state in device memory (FP32 master weights in parameter order).
 struct MlpAdam {
     float m[kMlpParams], v[kMlpParams], master[kMlpParams];
     float beta1, beta2, beta1Pow, beta2Pow, lr, eps;
+    unsigned int done;  // blocks of the reduction that have finished the step
 };
 
 size_t mlp_grad_smem_bytes();

@@ -187,8 +187,8 @@ int cg_train_classifier(const cg_train_options* o, const float* features, const 
     TRY(model.alloc(kMlpBytes));
     TRY(cudaMemcpyAsync(model.p, blob.data(), kMlpBytes, cudaMemcpyHostToDevice, s));
     const unsigned parts = mlp_grad_parts((unsigned)B);
-    TRY(part.alloc((size_t)parts * kMlpParams * sizeof(float)));
-    TRY(cudaMemsetAsync(part.p, 0, (size_t)parts * kMlpParams * sizeof(float), s));
+    TRY(part.alloc((size_t)parts * kMlpPartStride * sizeof(float)));
+    TRY(cudaMemsetAsync(part.p, 0, (size_t)parts * kMlpPartStride * sizeof(float), s));
     TRY(failed.alloc(sizeof(unsigned long long)));
     TRY(cudaMemsetAsync(failed.p, 0, sizeof(unsigned long long), s));
     // optimiser state: master weights from the initial model
@@ -274,8 +274,8 @@ int cg_classifier_gradients(int device, const void* model_data, size_t model_siz
     TRY(model.alloc(kMlpBytes));
     TRY(cudaMemcpyAsync(model.p, blob.data(), kMlpBytes, cudaMemcpyHostToDevice, s));
     const unsigned parts = mlp_grad_parts(n);
-    TRY(part.alloc((size_t)parts * kMlpParams * sizeof(float)));
-    TRY(cudaMemsetAsync(part.p, 0, (size_t)parts * kMlpParams * sizeof(float), s));
+    TRY(part.alloc((size_t)parts * kMlpPartStride * sizeof(float)));
+    TRY(cudaMemsetAsync(part.p, 0, (size_t)parts * kMlpPartStride * sizeof(float), s));
     TRY(grad.alloc(kMlpParams * sizeof(float)));
     TRY(failed.alloc(sizeof(unsigned long long)));
     TRY(cudaMemsetAsync(failed.p, 0, sizeof(unsigned long long), s));

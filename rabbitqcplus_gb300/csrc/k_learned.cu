@@ -256,6 +256,29 @@ __global__ void __launch_bounds__(kTcRows) mlp_infer_kernel(const unsigned char*
 constexpr int kTrainRows = 128;
 constexpr uint32_t kTrainTmemCols = 256;  // D1/D2 (0-127, later [dW2 dW1] at 0-95), dH1 (128-191)
 constexpr int kTrainOutCols = kMlpHidden + kMlpFeatures;  // N of the weight-gradient product
+// The transposed operands, written two bytes at a time with a row of the
+// minibatch per thread: 144 bytes between the core matrices along K keep a warp's
+// stores (8 rows per core matrix) out of each other's banks.
+constexpr uint32_t kTrainLbo = 144, kTrainSbo = kTrainLbo * (kTrainRows / 8);
+__device__ __forceinline__ uint32_t train_offset(int row, int k) {
+    return (uint32_t)(row >> 3) * kTrainSbo + (uint32_t)(k >> 3) * kTrainLbo + ((row & 7) << 4) + ((k & 7) << 1);
+}
+
+// Sums over the warp of 32 values per lane, column j's in lane j: every step
+// halves the columns a lane carries, so 31 shuffles do for 32 sums.  Each sum is
+// the butterfly's (lanes 16 apart first), in its order of additions.
+__device__ __forceinline__ float warp_sums(float (&v)[32], int lane) {
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) {
+        const bool up = (lane & m) != 0;
+#pragma unroll
+        for (int j = 0; j < m; j++) {
+            const float keep = up ? v[j + m] : v[j], send = up ? v[j] : v[j + m];
+            v[j] = __fadd_rn(keep, __shfl_xor_sync(kFull, send, m));
+        }
+    }
+    return v[0];
+}
 
 // shared memory of one block (every operand tile 1024-byte aligned)
 struct TrainTc {
@@ -265,8 +288,8 @@ struct TrainTc {
     unsigned char w2[kMlpHidden * kMlpHidden * 2];          // B of D2: W2 [64 out][64 in]
     unsigned char d2a[kTrainRows * kMlpHidden * 2];         // A of dH1: dH2 [128][64]
     unsigned char w2t[kMlpHidden * kMlpHidden * 2];         // B of dH1: W2^T [64 in][64 out]
-    unsigned char gA[kTrainRows * kTrainRows * 2];          // A of [dW2; dW1]: [dH2^T; dH1^T] [128][128 rows]
-    unsigned char gB[kTrainOutCols * kTrainRows * 2];       // B of [dW2; dW1]: [H1^T | X^T] [96][128 rows]
+    unsigned char gA[kTrainRows / 8 * kTrainSbo];           // A of [dW2; dW1]: [dH2^T; dH1^T] [128][128 rows]
+    unsigned char gB[kTrainOutCols / 8 * kTrainSbo];        // B of [dW2; dW1]: [H1^T | X^T] [96][128 rows]
     float b1[kMlpHidden], b2[kMlpHidden], w3[kMlpHidden];
     float red[4][3 * kMlpHidden + 2];                       // per-warp column sums: dW3, db2, db1, db3, loss
     float b3;
@@ -288,13 +311,20 @@ __global__ void __launch_bounds__(kTrainRows, 1) mlp_grad_kernel(const unsigned 
     const __nv_bfloat16* w1g = reinterpret_cast<const __nv_bfloat16*>(model + kMlpOffW1);
     const __nv_bfloat16* w2g = reinterpret_cast<const __nv_bfloat16*>(model + kMlpOffW2);
     const __nv_bfloat16* w3g = reinterpret_cast<const __nv_bfloat16*>(model + kMlpOffW3);
-    for (int i = tid; i < kMlpHidden * kMlpFeatures; i += kTrainRows)
-        *reinterpret_cast<__nv_bfloat16*>(s.w1 + core_offset(i / kMlpFeatures, i % kMlpFeatures, kMlpFeatures)) =
-            w1g[i];
-    for (int i = tid; i < kMlpHidden * kMlpHidden; i += kTrainRows) {
-        const int o = i / kMlpHidden, in = i % kMlpHidden;
-        *reinterpret_cast<__nv_bfloat16*>(s.w2 + core_offset(o, in, kMlpHidden)) = w2g[i];
-        *reinterpret_cast<__nv_bfloat16*>(s.w2t + core_offset(in, o, kMlpHidden)) = w2g[i];
+    // 8 weights (a row of a core matrix) per load
+    for (int i = tid; i < kMlpHidden * kMlpFeatures / 8; i += kTrainRows)
+        *reinterpret_cast<uint4*>(s.w1 + core_offset(i / (kMlpFeatures / 8), 8 * (i % (kMlpFeatures / 8)), kMlpFeatures)) =
+            reinterpret_cast<const uint4*>(w1g)[i];
+    for (int i = tid; i < kMlpHidden * kMlpHidden / 8; i += kTrainRows) {
+        const int o = i % kMlpHidden, in = 8 * (i / kMlpHidden);
+        const uint4 v = reinterpret_cast<const uint4*>(w2g)[o * (kMlpHidden / 8) + in / 8];
+        *reinterpret_cast<uint4*>(s.w2 + core_offset(o, in, kMlpHidden)) = v;
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            *reinterpret_cast<uint16_t*>(s.w2t + core_offset(in + 2 * q, o, kMlpHidden)) = (uint16_t)(w[q] & 0xffffu);
+            *reinterpret_cast<uint16_t*>(s.w2t + core_offset(in + 2 * q + 1, o, kMlpHidden)) = (uint16_t)(w[q] >> 16);
+        }
     }
     const float* bsrc = reinterpret_cast<const float*>(model + kMlpOffB1);
     if (tid < kMlpHidden) {
@@ -333,7 +363,7 @@ __global__ void __launch_bounds__(kTrainRows, 1) mlp_grad_kernel(const unsigned 
         const __nv_bfloat16* fv = reinterpret_cast<const __nv_bfloat16*>(f);
 #pragma unroll
         for (int k = 0; k < kMlpFeatures; k++)
-            *reinterpret_cast<__nv_bfloat16*>(s.gB + core_offset(kMlpHidden + k, tid, kTrainRows)) = fv[k];
+            *reinterpret_cast<__nv_bfloat16*>(s.gB + train_offset(kMlpHidden + k, tid)) = fv[k];
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
@@ -382,8 +412,8 @@ __global__ void __launch_bounds__(kTrainRows, 1) mlp_grad_kernel(const unsigned 
 #pragma unroll
                 for (int q = 0; q < 4; q++) {  // H1^T into rows 0-63 of the weight-gradient B operand
                     const int c = 32 * half + 8 * j + 2 * q;
-                    *reinterpret_cast<uint16_t*>(s.gB + core_offset(c, tid, kTrainRows)) = (uint16_t)(w[q] & 0xffffu);
-                    *reinterpret_cast<uint16_t*>(s.gB + core_offset(c + 1, tid, kTrainRows)) = (uint16_t)(w[q] >> 16);
+                    *reinterpret_cast<uint16_t*>(s.gB + train_offset(c, tid)) = (uint16_t)(w[q] & 0xffffu);
+                    *reinterpret_cast<uint16_t*>(s.gB + train_offset(c + 1, tid)) = (uint16_t)(w[q] >> 16);
                 }
             }
         }
@@ -428,21 +458,39 @@ __global__ void __launch_bounds__(kTrainRows, 1) mlp_grad_kernel(const unsigned 
             loss = (sp - y * z) * invTotal;
         }
     }
-    // column sums over the block's rows: four warps' shuffle sums, then in warp order
+    // column sums over the block's rows: four warps' sums, then in warp order
     auto colsum = [&](float v, int slot) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v = __fadd_rn(v, __shfl_xor_sync(kFull, v, o));
         if (lane == 0) s.red[warp][slot] = v;
     };
     if (ok) {
-#pragma unroll 4
-        for (int c = 0; c < kMlpHidden; c++) {
-            const float d2 = (h2pos >> c) & 1ull ? __fmul_rn(dz, s.w3[c]) : 0.0f;
-            colsum(__fmul_rn(dz, h2[c]), c);           // dW3
-            colsum(d2, kMlpHidden + c);                 // db2
-            const __nv_bfloat16 b = __float2bfloat16_rn(d2);
-            *reinterpret_cast<__nv_bfloat16*>(s.d2a + core_offset(tid, c, kMlpHidden)) = b;
-            *reinterpret_cast<__nv_bfloat16*>(s.gA + core_offset(c, tid, kTrainRows)) = b;  // dH2^T, rows 0-63
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+            float v[32];
+#pragma unroll
+            for (int i = 0; i < 32; i++) v[i] = __fmul_rn(dz, h2[32 * half + i]);
+            s.red[warp][32 * half + lane] = warp_sums(v, lane);  // dW3
+#pragma unroll
+            for (int i = 0; i < 32; i++) {
+                const int c = 32 * half + i;
+                v[i] = (h2pos >> c) & 1ull ? __fmul_rn(dz, s.w3[c]) : 0.0f;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                uint32_t w[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int c = 32 * half + 8 * j + 2 * q;
+                    w[q] = pack_bf16(v[8 * j + 2 * q], v[8 * j + 2 * q + 1]);
+                    // dH2^T, rows 0-63
+                    *reinterpret_cast<uint16_t*>(s.gA + train_offset(c, tid)) = (uint16_t)(w[q] & 0xffffu);
+                    *reinterpret_cast<uint16_t*>(s.gA + train_offset(c + 1, tid)) = (uint16_t)(w[q] >> 16);
+                }
+                *reinterpret_cast<uint4*>(s.d2a + core_offset(tid, 32 * half + 8 * j, kMlpHidden)) =
+                    make_uint4(w[0], w[1], w[2], w[3]);
+            }
+            s.red[warp][kMlpHidden + 32 * half + lane] = warp_sums(v, lane);  // db2
         }
         colsum(dz, 3 * kMlpHidden);      // db3
         colsum(loss, 3 * kMlpHidden + 1);
@@ -465,14 +513,14 @@ __global__ void __launch_bounds__(kTrainRows, 1) mlp_grad_kernel(const unsigned 
         for (int half = 0; half < 2; half++) {
             float v[32];
             tc_ld32(laneAddr + 2u * kMlpHidden + 32u * half, v);
-#pragma unroll 4
+#pragma unroll
             for (int i = 0; i < 32; i++) {
                 const int c = 32 * half + i;
-                const float d1 = (h1pos >> c) & 1ull ? v[i] : 0.0f;
-                colsum(d1, 2 * kMlpHidden + c);  // db1
-                *reinterpret_cast<__nv_bfloat16*>(s.gA + core_offset(kMlpHidden + c, tid, kTrainRows)) =
-                    __float2bfloat16_rn(d1);  // dH1^T, rows 64-127
+                v[i] = (h1pos >> c) & 1ull ? v[i] : 0.0f;
+                *reinterpret_cast<__nv_bfloat16*>(s.gA + train_offset(kMlpHidden + c, tid)) =
+                    __float2bfloat16_rn(v[i]);  // dH1^T, rows 64-127
             }
+            s.red[warp][2 * kMlpHidden + 32 * half + lane] = warp_sums(v, lane);  // db1
         }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -483,12 +531,13 @@ __global__ void __launch_bounds__(kTrainRows, 1) mlp_grad_kernel(const unsigned 
     if (ok && tid == 0) {
 #pragma unroll
         for (int k = 0; k < kTrainRows / 16; k++)
-            tc_mma(tbase, smem_desc(smem_u32(s.gA) + 256u * k, 128, 2048), smem_desc(smem_u32(s.gB) + 256u * k, 128, 2048),
+            tc_mma(tbase, smem_desc(smem_u32(s.gA) + 2 * kTrainLbo * k, kTrainLbo, kTrainSbo),
+                   smem_desc(smem_u32(s.gB) + 2 * kTrainLbo * k, kTrainLbo, kTrainSbo),
                    instr_desc(kTrainRows, kTrainOutCols), k > 0);
         tc_commit(mb);
     }
     if (ok) wait_mma();
-    float* out = part + (uint64_t)blockIdx.x * kMlpParams;
+    float* out = part + (uint64_t)blockIdx.x * kMlpPartStride;
     if (ok) {
         if (tid < kMlpHidden) {  // row o of dW2: columns 0-63
 #pragma unroll
@@ -496,13 +545,17 @@ __global__ void __launch_bounds__(kTrainRows, 1) mlp_grad_kernel(const unsigned 
                 float v[32];
                 tc_ld32(laneAddr + 32u * half, v);
 #pragma unroll
-                for (int i = 0; i < 32; i++) out[kMlpOffW2 / 2 + tid * kMlpHidden + 32 * half + i] = v[i];
+                for (int i = 0; i < 32; i += 4)
+                    *reinterpret_cast<float4*>(out + kMlpOffW2 / 2 + tid * kMlpHidden + 32 * half + i) =
+                        make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
             }
         } else {  // row i of dW1: columns 64-95
             float v[32];
             tc_ld32(laneAddr + (uint32_t)kMlpHidden, v);
 #pragma unroll
-            for (int f = 0; f < kMlpFeatures; f++) out[kMlpOffW1 / 2 + (tid - kMlpHidden) * kMlpFeatures + f] = v[f];
+            for (int f = 0; f < kMlpFeatures; f += 4)
+                *reinterpret_cast<float4*>(out + kMlpOffW1 / 2 + (tid - kMlpHidden) * kMlpFeatures + f) =
+                    make_float4(v[f], v[f + 1], v[f + 2], v[f + 3]);
         }
     }
     __syncthreads();
@@ -529,45 +582,57 @@ __global__ void __launch_bounds__(kTrainRows, 1) mlp_grad_kernel(const unsigned 
                      : "memory");
 }
 
-// One thread per parameter: the sum of the tiles' partials in tile order, then
-// (with `state`) an Adam step on the FP32 master copy and the BF16/FP32 model
-// the kernels read.  Thread kMlpParamLoss sums the loss into `lossOut`.
-__global__ void mlp_reduce_kernel(const float* __restrict__ part, unsigned int parts, float* __restrict__ grad,
-                                  float* lossOut, MlpAdam* state, unsigned char* model,
-                                  unsigned long long* stepPtr) {
+// One thread per parameter: the sum of the tiles' partials in tile order (eight
+// loads in flight), then (with `state`) an Adam step on the FP32 master copy and
+// the BF16/FP32 model the kernels read.  Thread kMlpParamLoss sums the loss into
+// `lossOut`.  With stepPtr the last block to finish advances the step, after
+// every thread has read the old powers.
+__global__ void __launch_bounds__(128) mlp_reduce_kernel(const float* __restrict__ part, unsigned int parts,
+                                                         float* __restrict__ grad, float* lossOut, MlpAdam* state,
+                                                         unsigned char* model, unsigned long long* stepPtr) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kMlpParams) return;
-    float sum = 0.0f;
-    for (unsigned w = 0; w < parts; w++) sum = __fadd_rn(sum, part[(uint64_t)w * kMlpParams + i]);
-    if (grad) grad[i] = sum;
-    if (i == kMlpParamLoss) {
-        if (lossOut) lossOut[stepPtr ? *stepPtr : 0] = sum;
-        return;
+    if (i < kMlpParams) {
+        float sum = 0.0f;
+        unsigned w = 0;
+        for (; w + 8 <= parts; w += 8) {
+            float x[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) x[q] = part[(uint64_t)(w + q) * kMlpPartStride + i];
+#pragma unroll
+            for (int q = 0; q < 8; q++) sum = __fadd_rn(sum, x[q]);
+        }
+        for (; w < parts; w++) sum = __fadd_rn(sum, part[(uint64_t)w * kMlpPartStride + i]);
+        if (grad) grad[i] = sum;
+        if (i == kMlpParamLoss) {
+            if (lossOut) lossOut[stepPtr ? *stepPtr : 0] = sum;
+        } else if (state) {
+            MlpAdam& a = *state;
+            const float m = a.beta1 * a.m[i] + (1.0f - a.beta1) * sum;
+            const float v = a.beta2 * a.v[i] + (1.0f - a.beta2) * sum * sum;
+            a.m[i] = m;
+            a.v[i] = v;
+            const float b1p = a.beta1Pow * a.beta1, b2p = a.beta2Pow * a.beta2;  // powers of this step
+            const float mh = m / (1.0f - b1p), vh = v / (1.0f - b2p);
+            const float w1 = a.master[i] - a.lr * mh / (sqrtf(vh) + a.eps);
+            a.master[i] = w1;
+            if (i < kMlpWeightCount) {
+                reinterpret_cast<__nv_bfloat16*>(model)[i] = __float2bfloat16_rn(w1);
+            } else {
+                reinterpret_cast<float*>(model + kMlpOffB1)[i - kMlpWeightCount] = w1;
+            }
+        }
     }
-    if (!state) return;
-    MlpAdam& a = *state;
-    const float m = a.beta1 * a.m[i] + (1.0f - a.beta1) * sum;
-    const float v = a.beta2 * a.v[i] + (1.0f - a.beta2) * sum * sum;
-    a.m[i] = m;
-    a.v[i] = v;
-    const float b1p = a.beta1Pow * a.beta1, b2p = a.beta2Pow * a.beta2;  // powers of this step
-    const float mh = m / (1.0f - b1p), vh = v / (1.0f - b2p);
-    const float w = a.master[i] - a.lr * mh / (sqrtf(vh) + a.eps);
-    a.master[i] = w;
-    if (i < kMlpWeightCount) {
-        reinterpret_cast<__nv_bfloat16*>(model)[i] = __float2bfloat16_rn(w);
-    } else {
-        reinterpret_cast<float*>(model + kMlpOffB1)[i - kMlpWeightCount] = w;
+    if (!state || !stepPtr) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&state->done, 1u) == gridDim.x - 1) {
+            state->done = 0;
+            state->beta1Pow *= state->beta1;
+            state->beta2Pow *= state->beta2;
+            *stepPtr += 1;
+        }
     }
-}
-
-// advances the step (after every thread of the reduce has read the old powers)
-__global__ void mlp_step_kernel(MlpAdam* state, unsigned long long* stepPtr) {
-    if (state) {
-        state->beta1Pow *= state->beta1;
-        state->beta2Pow *= state->beta2;
-    }
-    *stepPtr += 1;
 }
 
 __global__ void to_bf16_kernel(const float* __restrict__ in, uint64_t n, __nv_bfloat16* __restrict__ out) {
@@ -610,10 +675,7 @@ unsigned int mlp_grad_parts(unsigned int rows) { return (rows + kTrainRows - 1) 
 
 cudaError_t launch_mlp_reduce(const float* part, unsigned int parts, float* grad, float* lossOut, MlpAdam* state,
                               unsigned char* model, unsigned long long* stepPtr, cudaStream_t s) {
-    mlp_reduce_kernel<<<(kMlpParams + 255) / 256, 256, 0, s>>>(part, parts, grad, lossOut, state, model, stepPtr);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || !stepPtr) return e;
-    mlp_step_kernel<<<1, 1, 0, s>>>(state, stepPtr);
+    mlp_reduce_kernel<<<(kMlpParams + 127) / 128, 128, 0, s>>>(part, parts, grad, lossOut, state, model, stepPtr);
     return cudaGetLastError();
 }
 

@@ -127,12 +127,10 @@ BlockCache& block_cache() {
     return *c;
 }
 
-// grow-only device buffer; blocks come from and go back to the block cache,
-// except adopted ones (cached = false), which are freed
+// grow-only device buffer; blocks come from and go back to the block cache
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
-    bool cached = true;
     cudaError_t ensure(size_t n) {
         if (n <= bytes) return cudaSuccess;
         size_t want = std::max(n, bytes + bytes / 2), got = 0;
@@ -150,13 +148,9 @@ struct DevBuf {
         return cudaSuccess;
     }
     void release() {
-        if (p) {
-            if (cached) block_cache().release(p, bytes);
-            else cudaFree(p);
-        }
+        if (p) block_cache().release(p, bytes);
         p = nullptr;
         bytes = 0;
-        cached = true;
     }
     template <class T>
     T* as() const {
@@ -1976,11 +1970,14 @@ extern "C" int cg_get_candidates_noalloc(cg_ctx* c, uint64_t anchor, uint32_t* o
 // ---------------------------------------------------------------- device file path hooks
 namespace cg {
 
-int append_device_chunk(cg_ctx* c, void* dChars, uint64_t* dOffs, void* dQual, uint64_t n, int lmax) {
+cudaError_t cached_alloc(void** p, size_t n, size_t* got) { return block_cache().alloc(p, n, got); }
+void cached_release(void* p, size_t bytes) { block_cache().release(p, bytes); }
+
+int append_device_chunk(cg_ctx* c, CachedMem& chars, CachedMem& offs, CachedMem& qual, uint64_t n, int lmax) {
     if (!c) return CG_ERR_INVALID_ARGUMENT;
     if (c->built) return fail(c, CG_ERR_STATE, "reads cannot be appended after cg_build_tables");
     if (n == 0) return fail(c, CG_ERR_INVALID_ARGUMENT, "empty read batch");
-    if (c->o.use_quality_scores && !dQual)
+    if (c->o.use_quality_scores && !qual.p)
         return fail(c, CG_ERR_INVALID_ARGUMENT, "quality scores requested but not given");
     if (lmax > CG_MAX_READ_LENGTH) return fail(c, CG_ERR_UNSUPPORTED, "reads longer than %d", CG_MAX_READ_LENGTH);
     if (c->appended + n > 0xffffffffull) return fail(c, CG_ERR_UNSUPPORTED, "more than 2^32-1 reads");
@@ -1988,19 +1985,15 @@ int append_device_chunk(cg_ctx* c, void* dChars, uint64_t* dOffs, void* dQual, u
     cg_ctx::Chunk& ch = c->chunks.back();
     ch.first = c->appended;
     ch.reads = n;
-    ch.chars.p = dChars;  // the chunk owns the buffers from here on (freed after the build)
-    ch.chars.bytes = 1;
-    ch.chars.cached = false;
-    ch.offs.p = dOffs;
-    ch.offs.bytes = (n + 1) * sizeof(uint64_t);
-    ch.offs.cached = false;
-    if (c->o.use_quality_scores) {
-        ch.qual.p = dQual;
-        ch.qual.bytes = 1;
-        ch.qual.cached = false;
-    } else if (dQual) {
-        cudaFree(dQual);
-    }
+    auto take = [](DevBuf& d, CachedMem& m) {  // the chunk owns the block from here on (freed after the build)
+        d.p = m.p;
+        d.bytes = m.bytes;
+        m.p = nullptr;
+    };
+    take(ch.chars, chars);
+    take(ch.offs, offs);
+    if (c->o.use_quality_scores) take(ch.qual, qual);
+    else qual.free();
     c->appended += n;
     c->appendLmax = std::max(c->appendLmax, lmax);
     return CG_OK;

@@ -4,6 +4,7 @@
 #ifndef CARE_CAPI_INTERNAL_H
 #define CARE_CAPI_INTERNAL_H
 
+#include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
 
@@ -11,10 +12,41 @@
 
 namespace cg {
 
+// Device memory from the process's block cache (cg_release_cached_memory): at
+// least n bytes, *got of them.  cached_release waits for the device, as cudaFree
+// does, and keeps the block of the current device for a later request.
+cudaError_t cached_alloc(void** p, size_t n, size_t* got);
+void cached_release(void* p, size_t bytes);
+
+// A block of it, given back on scope exit.  Allocated and given back with the
+// same device current.
+struct CachedMem {
+    void* p = nullptr;
+    size_t bytes = 0;
+    CachedMem() = default;
+    CachedMem(const CachedMem&) = delete;
+    CachedMem& operator=(const CachedMem&) = delete;
+    ~CachedMem() { free(); }
+    cudaError_t alloc(size_t n) {
+        free();
+        const cudaError_t e = cached_alloc(&p, n < 16 ? 16 : n, &bytes);
+        if (e != cudaSuccess) p = nullptr;
+        return e;
+    }
+    void free() {
+        if (p) cached_release(p, bytes);
+        p = nullptr;
+    }
+    template <class T>
+    T* as() const {
+        return static_cast<T*>(p);
+    }
+};
+
 // cg_append_reads for one group of reads already on the device: bases back to
 // back (dChars), offsets dOffs[n+1] from 0, qualities like the bases (or
-// null).  The context takes ownership of the three cudaMalloc'd buffers.
-int append_device_chunk(cg_ctx* c, void* dChars, uint64_t* dOffs, void* dQual, uint64_t n, int lmax);
+// empty).  On success the context owns the blocks.
+int append_device_chunk(cg_ctx* c, CachedMem& chars, CachedMem& offs, CachedMem& qual, uint64_t n, int lmax);
 
 // cg_correct with flags[num] and sequences[num][pitch] in device memory.
 int correct_into_device(cg_ctx* c, uint64_t first, uint64_t num, uint8_t* dFlags, char* dSeq, size_t pitch);

@@ -288,28 +288,7 @@ __global__ void write_kernel(const ReadIdx* __restrict__ reads, uint64_t n, cons
     if (lane == 0) o[len] = '\n';
 }
 
-// device buffer freed on scope exit (unless released)
-struct DMem {
-    void* p = nullptr;
-    DMem() = default;
-    DMem(const DMem&) = delete;
-    DMem& operator=(const DMem&) = delete;
-    ~DMem() { free(); }
-    void free() {
-        if (p) cudaFree(p);
-        p = nullptr;
-    }
-    cudaError_t alloc(size_t n) { return cudaMalloc(&p, n < 16 ? 16 : n); }
-    void* release() {
-        void* q = p;
-        p = nullptr;
-        return q;
-    }
-    template <class T>
-    T* as() const {
-        return static_cast<T*>(p);
-    }
-};
+using DMem = CachedMem;
 
 struct Stream {
     cudaStream_t s = nullptr;
@@ -467,11 +446,8 @@ int correct_fastq_on_device(const cg_options& options, const std::vector<ByteSpa
                                                             chars.as<char>(), quals ? qual.as<char>() : nullptr);
         DCHECK(cudaGetLastError());
         DCHECK(cudaStreamSynchronize(s));
-        const int rc = append_device_chunk(ctx.c, chars.p, off.as<uint64_t>(), quals ? qual.p : nullptr, m, lmax);
+        const int rc = append_device_chunk(ctx.c, chars, off, qual, m, lmax);
         if (rc != CG_OK) return failf(error, rc, "append_device_chunk: %s", cg_last_error(ctx.c));
-        chars.release();  // owned by the context now
-        off.release();
-        if (quals) qual.release();
     }
     LCHECK(ctx.c, cg_build_tables(ctx.c));
     if (forest) LCHECK(ctx.c, cg_load_forest(ctx.c, forest->data(), forest->size(), maxTrees));
@@ -531,15 +507,26 @@ int correct_fastq_on_device(const cg_options& options, const std::vector<ByteSpa
                                    s));
             DCHECK(cudaStreamSynchronize(s));
             if (total == 0) continue;
-            DMem outDev;
-            DCHECK(outDev.alloc(total));
+            // queue chunks outlive this call, on whatever thread and device: their bytes are not cached
+            const bool keep = run->queueChunkBytes && !run->onChunk;
+            DMem outMem;
+            char* outDev = nullptr;
+            if (keep) {
+                void* raw = nullptr;
+                DCHECK(cudaMalloc(&raw, total));
+                outDev = static_cast<char*>(raw);
+                run->deviceOutputs[(size_t)f].bytes = raw;  // freed with the run
+            } else {
+                DCHECK(outMem.alloc(total));
+                outDev = outMem.as<char>();
+            }
             write_kernel<<<grid_for(m * 32, 256), 256, 0, s>>>(reads + r0, m, readOut.as<uint8_t>() + r0, (uint8_t)f,
                                                                pos.as<unsigned long long>(), mode.as<uint8_t>() + r0,
                                                                status.as<uint8_t>() + r0, sq, pitch,
                                                                qualityLabels ? 1 : 0, lastRec.as<unsigned int>(), r0,
-                                                               outDev.as<char>());
+                                                               outDev);
             DCHECK(cudaGetLastError());
-            if (run->queueChunkBytes && !run->onChunk) {
+            if (keep) {
                 // queue chunks: cut at record ends, each chunk the longest run of
                 // whole records under queueChunkBytes (src/correctionresultoutput.cpp:
                 // 733-745); the bytes stay on the device until emit_queue_chunks
@@ -560,11 +547,10 @@ int correct_fastq_on_device(const cg_options& options, const std::vector<ByteSpa
                     }
                 }
                 dout.chunks.emplace_back(begin, (size_t)total);
-                dout.bytes = outDev.release();
                 continue;
             }
             std::unique_ptr<char[]> bytes(new char[total]);  // left uninitialised: the copy fills it
-            DCHECK(cudaMemcpyAsync(bytes.get(), outDev.p, total, cudaMemcpyDeviceToHost, s));
+            DCHECK(cudaMemcpyAsync(bytes.get(), outDev, total, cudaMemcpyDeviceToHost, s));
             DCHECK(cudaStreamSynchronize(s));
             if (run->onChunk) {
                 run->onChunk(f, std::move(bytes), total);

@@ -22,6 +22,7 @@
 #include <random>
 #include <vector>
 
+#include "care_capi_internal.h"
 #include "care_gpu.h"
 #include "care_internal.h"
 #include "care_learned.h"
@@ -40,18 +41,7 @@ struct Header {
 };
 static_assert(sizeof(Header) == kHeader, "classifier header");
 
-// A device allocation freed on scope exit.
-struct Dev {
-    void* p = nullptr;
-    cudaError_t alloc(size_t n) { return cudaMalloc(&p, std::max<size_t>(n, 16)); }
-    ~Dev() {
-        if (p) cudaFree(p);
-    }
-    template <class T>
-    T* as() const {
-        return static_cast<T*>(p);
-    }
-};
+using Dev = CachedMem;
 
 int cuda_status(cudaError_t e) {
     if (e == cudaSuccess) return CG_OK;

@@ -55,6 +55,9 @@ cudaError_t launch_mlp_infer(const unsigned char* model, const __nv_bfloat16* fe
                              const unsigned int* countPtr, unsigned int count, unsigned int cap, float minLogit,
                              char* out, int outPitch, float* logits, unsigned long long* counters, int blocks,
                              cudaStream_t s);
+// Logits of `count` FP32 feature rows (16-byte aligned).
+cudaError_t launch_mlp_logits(const unsigned char* model, const float* feat, unsigned int count, float* logits,
+                              unsigned long long* counters, int blocks, cudaStream_t s);
 // Polls of the inference kernel's per-tile MMA waits on the current device
 // (default 1 << 20); a block whose wait runs out counts in
 // counters[kCounterTimeouts] and leaves its columns to the fallback decision.

@@ -14,6 +14,8 @@
 // every block writes its partial gradients to its own slot and one kernel sums
 // the slots in a fixed order before the Adam update.
 
+#include <algorithm>
+
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -66,15 +68,17 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
     for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
 
-// Inference over a column buffer, persistent over 128-column tiles.  With
+// Inference over a column buffer, persistent over 128-column tiles.  Rows are
+// BF16 (the column records) or FP32, rounded to BF16 as they are read.  With
 // `logits` set the outputs are written there; otherwise every column whose
 // logit reaches `minLogit` (the logit of the confidence threshold) gets the
 // consensus base in its output row, and the others keep the fallback decision
 // the MSA kernel already wrote.  A wait that does not end counts in
 // counters[kCounterTimeouts] and ends the block (after a second bounded wait
 // for its MMAs and the release of its tensor memory).
+template <class Feature>
 __global__ void __launch_bounds__(kTcRows) mlp_infer_kernel(const unsigned char* __restrict__ model,
-                                                            const __nv_bfloat16* __restrict__ feat,
+                                                            const Feature* __restrict__ feat,
                                                             const uint2* __restrict__ meta,
                                                             const unsigned int* __restrict__ countPtr,
                                                             unsigned int count, unsigned int cap, float minLogit,
@@ -137,9 +141,21 @@ __global__ void __launch_bounds__(kTcRows) mlp_infer_kernel(const unsigned char*
 #pragma unroll
         for (int j = 0; j < 4; j++) f[j] = make_uint4(0, 0, 0, 0);
         if (row < n) {
-            const uint4* src = reinterpret_cast<const uint4*>(feat + (uint64_t)row * kMlpFeatures);
+            if constexpr (sizeof(Feature) == 2) {
+                const uint4* src = reinterpret_cast<const uint4*>(feat + (uint64_t)row * kMlpFeatures);
 #pragma unroll
-            for (int j = 0; j < 4; j++) f[j] = src[j];
+                for (int j = 0; j < 4; j++) f[j] = src[j];
+            } else {
+                const float4* src = reinterpret_cast<const float4*>(feat + (uint64_t)row * kMlpFeatures);
+                float4 x[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) x[j] = src[j];
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    f[j] = make_uint4(pack_bf16(x[2 * j].x, x[2 * j].y), pack_bf16(x[2 * j].z, x[2 * j].w),
+                                      pack_bf16(x[2 * j + 1].x, x[2 * j + 1].y),
+                                      pack_bf16(x[2 * j + 1].z, x[2 * j + 1].w));
+            }
         }
 #pragma unroll
         for (int j = 0; j < 4; j++) *reinterpret_cast<uint4*>(a1 + core_offset(tid, 8 * j, kMlpFeatures)) = f[j];
@@ -651,6 +667,15 @@ cudaError_t launch_mlp_infer(const unsigned char* model, const __nv_bfloat16* fe
     if (blocks <= 0) blocks = 1;
     mlp_infer_kernel<<<blocks, kTcRows, 0, s>>>(model, feat, meta, countPtr, count, cap, minLogit, out, outPitch,
                                                  logits, counters);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_mlp_logits(const unsigned char* model, const float* feat, unsigned int count, float* logits,
+                              unsigned long long* counters, int blocks, cudaStream_t s) {
+    if (count == 0) return cudaSuccess;
+    mlp_infer_kernel<<<std::max(blocks, 1), kTcRows, 0, s>>>(model, feat, static_cast<const uint2*>(nullptr),
+                                                             static_cast<const unsigned int*>(nullptr), count, count,
+                                                             0.0f, static_cast<char*>(nullptr), 0, logits, counters);
     return cudaGetLastError();
 }
 

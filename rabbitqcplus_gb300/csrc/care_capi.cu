@@ -171,12 +171,12 @@ struct GraphSig {
     int count = 0;
     unsigned long long stride = 0;
     Shape shape{};
-    int tableRaw = 0, maxRows = 0;
+    int tableRaw = 0;
     std::vector<const void*> ptrs;
     bool operator==(const GraphSig& o) const {
         return count == o.count && stride == o.stride && shape.alignBlocks == o.shape.alignBlocks &&
                shape.msaWarps == o.shape.msaWarps && shape.msaBlocks == o.shape.msaBlocks &&
-               tableRaw == o.tableRaw && maxRows == o.maxRows && ptrs == o.ptrs;
+               tableRaw == o.tableRaw && ptrs == o.ptrs;
     }
 };
 
@@ -771,7 +771,7 @@ int enqueue_batch_plain(cg_ctx* c, int slot, uint64_t first, int count) {
     CG_CUDA(c, launch_msa_order(b, c->orderScratch.as<unsigned int>(), c->msaOrder.as<uint32_t>(), c->stream));
     c->stats.kernel_launches += 2;
     b.order = c->msaOrder.as<uint32_t>();
-    CG_CUDA(c, launch_msa_correct(st, c->params, b, (int)std::max<uint32_t>(c->hPinned[2 * slot + 1], 1), c->stream));
+    CG_CUDA(c, launch_msa_correct(st, c->params, b, c->stream));
     if (learned && !c->collecting) {
         CG_CUDA(c, launch_mlp_infer(c->mlp.as<unsigned char>(), b.colFeat, b.colMeta, b.colCount, 0, b.colCap,
                                     c->minLogit, b.out, b.outPitch, nullptr, b.counters, infer_blocks(c),
@@ -958,7 +958,7 @@ int ensure_set(cg_ctx* c, BatchSet& s, int count, uint64_t capRaw) {
 
 // The kernels of one batch, enqueued on the set's stream (captured).
 cudaError_t enqueue_batch(cg_ctx* c, BatchSet& s, int count, unsigned long long stride, const Shape& sh,
-                          int tableRaw, int maxRows, int* kernels) {
+                          int tableRaw, int* kernels) {
     const StoreArg st = store_arg(c);
     const BatchArg b = set_arg(c, s, count);
     int k = 0;
@@ -980,7 +980,7 @@ cudaError_t enqueue_batch(cg_ctx* c, BatchSet& s, int count, unsigned long long 
         k += 2;
     }
     if (e == cudaSuccess) {
-        e = launch_msa_correct(st, c->params, b, maxRows, s.stream, &sh);
+        e = launch_msa_correct(st, c->params, b, s.stream, &sh);
         k++;
     }
     if (e == cudaSuccess && learned) {
@@ -1000,14 +1000,12 @@ cudaError_t enqueue_batch(cg_ctx* c, BatchSet& s, int count, unsigned long long 
     return e;
 }
 
-int capture_set(cg_ctx* c, BatchSet& s, int count, unsigned long long stride, const Shape& sh, int tableRaw,
-                int maxRows) {
+int capture_set(cg_ctx* c, BatchSet& s, int count, unsigned long long stride, const Shape& sh, int tableRaw) {
     GraphSig g;
     g.count = count;
     g.stride = stride;
     g.shape = sh;
     g.tableRaw = tableRaw;
-    g.maxRows = maxRows;
     for (const DevBuf* d : {&s.rawCount, &s.cand, &s.ncand, &s.paired, &s.aln, &s.fid, &s.fshift, &s.forient,
                             &s.fweight, &s.flen, &s.nfinal, &s.units, &s.cursor, &s.work, &s.colFeat,
                             &s.colMeta, &s.colCount, &s.order, &s.orderScratch, &s.bigScratch, &c->mlp, &c->outRange,
@@ -1019,7 +1017,7 @@ int capture_set(cg_ctx* c, BatchSet& s, int count, unsigned long long stride, co
     s.exec = nullptr;
     CG_CUDA(c, cudaStreamBeginCapture(s.stream, cudaStreamCaptureModeThreadLocal));
     int kernels = 0;
-    const cudaError_t e = enqueue_batch(c, s, count, stride, sh, tableRaw, maxRows, &kernels);
+    const cudaError_t e = enqueue_batch(c, s, count, stride, sh, tableRaw, &kernels);
     cudaGraph_t graph = nullptr;
     const cudaError_t e2 = cudaStreamEndCapture(s.stream, &graph);
     if (e != cudaSuccess || e2 != cudaSuccess) {
@@ -1082,7 +1080,7 @@ int run_batched(cg_ctx* c, uint64_t first, uint64_t nb, const Plan& pl, const st
         BatchSet& s = c->sets[k];
         int rc = ensure_set(c, s, pl.batch, capRaw);
         if (rc != CG_OK) return rc;
-        rc = capture_set(c, s, pl.batch, B * S, pl.shape, maxRaw, maxRaw);
+        rc = capture_set(c, s, pl.batch, B * S, pl.shape, maxRaw);
         if (rc != CG_OK) return rc;
         c->hBatched[2 + 2 * k] = first + (uint64_t)k * B;
         c->hBatched[3 + 2 * k] = first;

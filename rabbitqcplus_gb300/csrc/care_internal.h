@@ -295,10 +295,11 @@ struct Shape {
 cudaError_t launch_align(StoreArg st, Params p, BatchArg b, bool varies, unsigned blocks, cudaStream_t s);
 // resident 128-thread blocks of it per SM
 int align_occupancy(StoreArg st);
-cudaError_t launch_msa_correct(StoreArg st, Params p, BatchArg b, int maxRows, cudaStream_t s,
-                               const Shape* shape = nullptr);
-// warp-per-anchor MSA blocks of `warps` warps that fit one SM (0: the warp
-// MSA does not apply to this store)
+// MSA, refinement and decision of the batch's anchors, one warp each.  With
+// b.work: persistent blocks of shape->msaWarps warps, or as many as a block's
+// shared memory holds (long reads); otherwise a block of one warp per anchor.
+cudaError_t launch_msa_correct(StoreArg st, Params p, BatchArg b, cudaStream_t s, const Shape* shape = nullptr);
+// resident MSA blocks of `warps` warps per SM
 int msa_warp_occupancy(StoreArg st, Params p, int warps);
 // order[count] = the batch's anchors by decreasing b.nfinal (log2 buckets);
 // scratch = 32 words, cleared by the launcher

@@ -21,45 +21,6 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 
-// ---------------------------------------------------------------- MSA
-
-constexpr int kMsaThreadsMin = 128;
-constexpr int kMsaCols = 4;  // columns owned per thread
-constexpr int kMsaChunkRows = 512;
-
-struct RowMeta {
-    const uint32_t* enc;  // candidate's 2-bit row
-    const uint8_t* qual;  // candidate's qualities (or null)
-    float weight;
-    int16_t shift;
-    uint16_t len;
-    uint8_t rc;
-    uint8_t pad[7];
-};
-static_assert(sizeof(RowMeta) == 32, "row meta layout");
-
-template <class T>
-__device__ __forceinline__ T block_reduce(T v, T* red, int op /*0 min 1 max 2 sum*/) {
-    for (int d = 16; d > 0; d >>= 1) {
-        const T o = __shfl_xor_sync(kFull, v, d);
-        v = op == 0 ? (o < v ? o : v) : op == 1 ? (o > v ? o : v) : v + o;
-    }
-    const int warp = threadIdx.x >> 5;
-    const int nw = blockDim.x >> 5;
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[warp] = v;
-    __syncthreads();
-    T r = red[0];
-    for (int w = 1; w < nw; w++) r = op == 0 ? (red[w] < r ? red[w] : r) : op == 1 ? (red[w] > r ? red[w] : r) : r + red[w];
-    return r;
-}
-
-// One block per anchor; column c belongs to thread c % blockDim (at most
-// kMsaCols columns per thread, kept in registers while the rows stream by).
-// Every column adds its rows in list order -- anchor first, then the kept
-// candidates as the filters left them -- so each float sum is the
-// reference's sequence of additions.  Row metadata is staged in shared memory
-// in chunks of kMsaChunkRows rows; removed rows are a shared bitset.
 // reference: include/classification.hpp:748-797 (extract_anchor_v3) and
 // include/forest.hpp:70-81,217-226 (tree walk; decide: running mean of the
 // trees' probabilities, true as soon as it reaches the threshold)
@@ -104,27 +65,6 @@ __device__ __forceinline__ void vote_word(const Params& p, uint64_t read, int w,
     atomicOr(&p.candOr[i], v);
 }
 
-// One thread votes for one row: cons(col) gives the consensus base code of
-// column col (relative to the anchor's first column).  Returns 1 if it voted.
-template <class Cons>
-__device__ __forceinline__ int vote_candidate(const Params& p, int s, int len, bool rc, uint32_t id, uint64_t aid,
-                                              int La, Cons cons) {
-    const int nc = p.newColumns;
-    if (s < -nc || s > nc || s + len > La + nc) return 0;
-    for (int w = 0; w * 32 < len; w++) {
-        unsigned long long v = 0;
-        const int pe = min(len, w * 32 + 32);
-        for (int q = w * 32; q < pe; q++) {
-            uint32_t bb = cons(s + (rc ? len - 1 - q : q));
-            if (rc) bb = 3u - bb;
-            v |= (unsigned long long)bb << (62 - 2 * (q & 31));
-        }
-        vote_word(p, id, w, v);
-    }
-    atomicAdd((uint64_t)id > aid ? &p.candVotes[id].x : &p.candVotes[id].y, 1u);
-    return 1;
-}
-
 // Quality score of position `pos` (aligned orientation) of a candidate row
 // (reference: include/corrector.hpp:1214-1239).  Rows hold Lmax scores; past
 // the read's end the store holds what the reference's decoded row holds there
@@ -134,320 +74,6 @@ __device__ __forceinline__ int vote_candidate(const Params& p, int s, int len, b
 // position pos reads score Lmax - 1 - pos.
 __device__ __forceinline__ uint8_t row_quality(const uint8_t* q, int lmax, bool rc, int pos) {
     return q[rc ? lmax - 1 - pos : pos];
-}
-
-__global__ void __launch_bounds__(1024) msa_correct_kernel(StoreArg st, Params p, BatchArg b,
-                                                          const uint32_t* __restrict__ rawOff, int maxCols,
-                                                          int bitsetWords, int storeWeights) {
-    extern __shared__ __align__(16) unsigned char sm[];
-    RowMeta* rows = reinterpret_cast<RowMeta*>(sm);
-    uint32_t* removed = reinterpret_cast<uint32_t*>(rows + kMsaChunkRows);
-    float* qw = reinterpret_cast<float*>(removed + bitsetWords);
-    int* cntA = reinterpret_cast<int*>(qw + 256);
-    int* cntC = cntA + maxCols;
-    int* cntG = cntC + maxCols;
-    int* cntT = cntG + maxCols;
-    int* cov = cntT + maxCols;
-    int* origCov = cov + maxCols;
-    float* sup = reinterpret_cast<float*>(origCov + maxCols);
-    // column weights, kept only for the forest's features
-    float* colWA = storeWeights ? sup + maxCols : nullptr;
-    float* colWC = storeWeights ? colWA + maxCols : nullptr;
-    float* colWG = storeWeights ? colWC + maxCols : nullptr;
-    float* colWT = storeWeights ? colWG + maxCols : nullptr;
-    char* cons = reinterpret_cast<char*>(sup + maxCols + (storeWeights ? 4 * maxCols : 0));
-    __shared__ float redf[32];
-    __shared__ int redi[32];
-    __shared__ int sCol, sFound, sByConsensus;
-
-    const int a = blockIdx.x;
-    const int tid = threadIdx.x;
-    const int bd = blockDim.x;
-    const uint64_t first = batch_first(b);
-    const uint64_t aid = first + (uint64_t)a;
-    const uint64_t oi = (first - out_first(b)) + (uint64_t)a;  // output row
-    const uint32_t nf = b.nfinal[a];
-    char* out = b.out + oi * b.outPitch;
-    if (nf == 0) {
-        if (tid == 0) b.flags[oi] = 0;
-        return;
-    }
-    const uint32_t base = rawOff[a];
-    const int La = st.len[aid];
-    const uint32_t* aenc = st.enc + aid * (uint64_t)st.pitch;
-    const uint8_t* aq = p.useQuality ? st.qual + aid * (uint64_t)st.lmax : nullptr;
-    for (int i = tid; i < bitsetWords; i += bd) removed[i] = 0u;
-    if (p.useQuality)
-        for (int i = tid; i < 256; i += bd) qw[i] = p.qweight[i];
-    const bool oneChunk = nf <= (uint32_t)kMsaChunkRows;
-    auto loadRows = [&](uint32_t j0, uint32_t cnt) {
-        for (uint32_t r = tid; r < cnt; r += bd) {
-            const uint32_t j = base + j0 + r;
-            const uint32_t id = b.fid[j];
-            RowMeta m;
-            m.enc = st.enc + (uint64_t)id * st.pitch;
-            m.qual = p.useQuality ? st.qual + (uint64_t)id * st.lmax : nullptr;
-            m.weight = b.fweight[j];
-            m.shift = b.fshift[j];
-            m.len = b.flen[j];
-            m.rc = b.forient[j] == 2;
-            rows[r] = m;
-        }
-    };
-    if (oneChunk) loadRows(0, nf);
-    __syncthreads();
-    auto isRemoved = [&](uint32_t j) { return (removed[j >> 5] >> (j & 31)) & 1u; };
-
-    int aBegin = 0, nActive = (int)nf, builds = 0;
-    for (int iter = 0;; iter++) {
-        // columns of the current MSA (src/msa.cpp:19-33)
-        int lo = 0, hi = La, act = 0;
-        for (uint32_t j = tid; j < nf; j += bd) {
-            if (!isRemoved(j)) {
-                const int s = b.fshift[base + j];
-                lo = min(lo, s);
-                hi = max(hi, s + (int)b.flen[base + j]);
-                act++;
-            }
-        }
-        lo = block_reduce<int>(lo, redi, 0);
-        hi = block_reduce<int>(hi, redi, 1);
-        nActive = block_reduce<int>(act, redi, 2);
-        const int nCols = hi - lo;
-        aBegin = -lo;
-        const int aEnd = aBegin + La;
-        // build: counts, weights (src/msa.cpp:93-112)
-        int nA[kMsaCols], nC[kMsaCols], nG[kMsaCols], nT[kMsaCols];
-        float wA[kMsaCols], wC[kMsaCols], wG[kMsaCols], wT[kMsaCols];
-#pragma unroll
-        for (int k = 0; k < kMsaCols; k++) {
-            nA[k] = nC[k] = nG[k] = nT[k] = 0;
-            wA[k] = wC[k] = wG[k] = wT[k] = 0.0f;
-        }
-        auto add = [&](int k, uint32_t bb, float w) {
-            if (bb == 0) { nA[k]++; wA[k] = __fadd_rn(wA[k], w); }
-            else if (bb == 1) { nC[k]++; wC[k] = __fadd_rn(wC[k], w); }
-            else if (bb == 2) { nG[k]++; wG[k] = __fadd_rn(wG[k], w); }
-            else { nT[k]++; wT[k] = __fadd_rn(wT[k], w); }
-        };
-#pragma unroll
-        for (int k = 0; k < kMsaCols; k++) {
-            const int c = tid + k * bd;
-            if (c >= aBegin && c < aEnd) {
-                const int pos = c - aBegin;
-                const float w = p.useQuality ? __fmul_rn(1.0f, qw[aq[pos]]) : 1.0f;
-                add(k, get2bit(aenc, pos), w);
-            }
-        }
-        for (uint32_t j0 = 0; j0 < nf; j0 += kMsaChunkRows) {
-            const uint32_t cnt = min((uint32_t)kMsaChunkRows, nf - j0);
-            if (!oneChunk) {
-                __syncthreads();
-                loadRows(j0, cnt);
-                __syncthreads();
-            }
-            for (uint32_t r = 0; r < cnt; r++) {
-                if (isRemoved(j0 + r)) continue;
-                const RowMeta m = rows[r];
-                const int rb = aBegin + m.shift;
-                const int re = rb + (int)m.len;
-#pragma unroll
-                for (int k = 0; k < kMsaCols; k++) {
-                    const int c = tid + k * bd;
-                    if (c >= rb && c < re) {
-                        const int pos = c - rb;
-                        const int sp = m.rc ? (int)m.len - 1 - pos : pos;
-                        uint32_t bb = get2bit(m.enc, sp);
-                        if (m.rc) bb = 3u - bb;
-                        float w = m.weight;
-                        if (p.useQuality) w = __fmul_rn(w, qw[row_quality(m.qual, st.lmax, m.rc, pos)]);
-                        add(k, bb, w);
-                    }
-                }
-            }
-        }
-        // findConsensus (src/msa.cpp:135-157), findOrigWeightAndCoverage (:159-173)
-#pragma unroll
-        for (int k = 0; k < kMsaCols; k++) {
-            const int c = tid + k * bd;
-            if (c < nCols) {
-                char cs = 'A';
-                float cw = wA[k];
-                if (wC[k] > cw) { cs = 'C'; cw = wC[k]; }
-                if (wG[k] > cw) { cs = 'G'; cw = wG[k]; }
-                if (wT[k] > cw) { cs = 'T'; cw = wT[k]; }
-                const float colW = __fadd_rn(__fadd_rn(__fadd_rn(wA[k], wC[k]), wG[k]), wT[k]);
-                cntA[c] = nA[k]; cntC[c] = nC[k]; cntG[c] = nG[k]; cntT[c] = nT[k];
-                cov[c] = nA[k] + nC[k] + nG[k] + nT[k];
-                sup[c] = __fdiv_rn(cw, colW);
-                cons[c] = cs;
-                if (storeWeights) {
-                    colWA[c] = wA[k]; colWC[c] = wC[k]; colWG[c] = wG[k]; colWT[c] = wT[k];
-                }
-                if (c >= aBegin && c < aEnd) {
-                    const uint32_t ab = get2bit(aenc, c - aBegin);
-                    origCov[c] = ab == 0 ? nA[k] : ab == 1 ? nC[k] : ab == 2 ? nG[k] : nT[k];
-                }
-            }
-        }
-        builds++;
-        __syncthreads();
-        if (iter == 5 || nActive == 0) break;
-        // findCandidatesOfDifferentRegion (src/msa.cpp:532-734)
-        bool mism = false;
-        for (int c = aBegin + tid; c < aEnd; c += bd) mism |= cons[c] != "ACGT"[get2bit(aenc, c - aBegin)];
-        if (!__syncthreads_or(mism)) break;
-        if (tid == 0) sCol = 0x7fffffff;
-        __syncthreads();
-        for (int c = aBegin + tid; c < aEnd; c += bd) {
-            const int counts[4] = {cntA[c], cntC[c], cntG[c], cntT[c]};
-            const int ci = cons[c] == 'A' ? 0 : cons[c] == 'C' ? 1 : cons[c] == 'G' ? 2 : 3;
-            bool sig = false;
-            for (int i = 0; i < 4; i++) sig |= (i != ci && p.significantCount <= counts[i]);
-            if (sig) atomicMin(&sCol, c);
-        }
-        __syncthreads();
-        const int col = sCol;
-        if (col == 0x7fffffff) break;
-        if (tid == 0) {
-            const int counts[4] = {cntA[col], cntC[col], cntG[col], cntT[col]};
-            const int ci = cons[col] == 'A' ? 0 : cons[col] == 'C' ? 1 : cons[col] == 'G' ? 2 : 3;
-            int si = -1;
-            for (int i = 0; i < 4; i++)
-                if (i != ci && p.significantCount <= counts[i]) si = i;
-            sFound = si;
-        }
-        __syncthreads();
-        const uint32_t found = (uint32_t)sFound;
-        const uint32_t orig = get2bit(aenc, col - aBegin);
-        const bool keepMatching = orig == found;
-        auto differs = [&](uint32_t j) -> bool {  // row j lies on `col` and is to be removed
-            const uint32_t g = base + j;
-            const int rb = aBegin + b.fshift[g];
-            const int len = b.flen[g];
-            if (col < rb || col >= rb + len) return false;
-            const uint32_t* e = st.enc + (uint64_t)b.fid[g] * st.pitch;
-            const int pos = col - rb;
-            const bool rc = b.forient[g] == 2;
-            uint32_t bb = get2bit(e, rc ? len - 1 - pos : pos);
-            if (rc) bb = 3u - bb;
-            return keepMatching ? (bb != found) : (bb == found);
-        };
-        bool veto = false, any = false;
-        for (uint32_t j = tid; j < nf; j += bd) {
-            if (isRemoved(j) || !differs(j)) continue;
-            any = true;
-            veto |= b.fweight[base + j] >= 0.90f;
-        }
-        const bool anyVeto = __syncthreads_or(veto);
-        const bool anyRemove = __syncthreads_or(any);
-        // a veto (or nothing to remove) leaves the MSA as it is; the
-        // reference then rebuilds the same MSA and reaches the same decision
-        if (anyVeto || !anyRemove) break;
-        for (uint32_t j = tid; j < nf; j += bd) {
-            if (!isRemoved(j) && differs(j)) atomicOr(&removed[j >> 5], 1u << (j & 31));
-        }
-        __syncthreads();
-    }
-    // getMSAProperties (src/msa.cpp:304-376) and getCorrectedAnchor (:379-453)
-    const int aEnd = aBegin + La;
-    float mins = 3.402823466e+38f;
-    int minc = 0x7fffffff, maxc = -1;
-    for (int c = aBegin + tid; c < aEnd; c += bd) {
-        mins = fminf(mins, sup[c]);
-        minc = min(minc, cov[c]);
-        maxc = max(maxc, cov[c]);
-    }
-    mins = block_reduce<float>(mins, redf, 0);
-    minc = block_reduce<int>(minc, redi, 0);
-    maxc = block_reduce<int>(maxc, redi, 1);
-    __shared__ float sAvg;
-    __shared__ int sHQ;
-    if (tid == 0) {
-        float sum = 0.0f;
-        for (int c = aBegin; c < aEnd; c++) sum = __fadd_rn(sum, sup[c]);
-        const float avg = __fdiv_rn(sum, (float)La);
-        const bool good = fgeq(avg, p.avgSupportThreshold) && fgeq(mins, p.minSupportThreshold) &&
-                          fgeq((float)minc, p.minCoverageThreshold);
-        bool hq = false;
-        if (good) {
-            int smallest = 100;
-            for (int percent = p.errPercent; percent >= 0; percent--) {
-                if (fgeq(avg, p.hqAvg[percent]) && fgeq(mins, p.hqMin[percent])) smallest = percent;
-            }
-            hq = fgeq((float)minc, p.minCoverageThreshold) && fleq((float)smallest, p.hqPercentLimit);
-        }
-        sByConsensus = good;
-        sAvg = avg;
-        sHQ = hq;
-        // the forest decision corrects every anchor that reached the MSA
-        // (include/corrector.hpp:1448-1472); the classic one needs candidates
-        const bool corrected = p.correctionType == CG_CORR_FOREST || nActive > 0;
-        if (corrected) {
-            atomicAdd(&b.counters[kCounterCorrected], 1ull);
-            if (hq) atomicAdd(&b.counters[kCounterHQ], 1ull);
-        }
-        atomicAdd(&b.counters[kCounterMsaBuilds], (unsigned long long)builds);
-        b.flags[oi] = corrected ? (uint8_t)(CG_RESULT_CORRECTED | (hq ? CG_RESULT_HQ : 0)) : (uint8_t)0;
-    }
-    __syncthreads();
-    if (p.candidates && sHQ) {
-        // candidate correction: one thread per row of the final MSA, whose
-        // consensus covers every column of the rows
-        int votes = 0;
-        for (uint32_t j = tid; j < nf; j += bd) {
-            if (isRemoved(j)) continue;
-            const uint32_t g = base + j;
-            votes += vote_candidate(p, b.fshift[g], b.flen[g], b.forient[g] == 2, b.fid[g], aid, La,
-                                    [&](int col) { return (uint32_t)base_index(cons[aBegin + col]); });
-        }
-        votes = block_reduce<int>(votes, redi, 2);
-        if (tid == 0 && votes) atomicAdd(&b.counters[kCounterCandidateVotes], (unsigned long long)votes);
-    }
-    if (p.correctionType == CG_CORR_FOREST) {
-        const bool hq = sHQ;
-        const float avg = sAvg;
-        for (int i = tid; i < La; i += bd) {
-            const int c = aBegin + i;
-            const uint32_t ab = get2bit(aenc, i);
-            const char orig = "ACGT"[ab];
-            char r = cons[c];
-            if (!hq && r != orig) {
-                const float wsum = __fadd_rn(__fadd_rn(__fadd_rn(colWA[c], colWC[c]), colWG[c]), colWT[c]);
-                float wCons, nCons;
-                switch (r) {
-                    case 'A': wCons = colWA[c]; nCons = (float)cntA[c]; break;
-                    case 'C': wCons = colWC[c]; nCons = (float)cntC[c]; break;
-                    case 'G': wCons = colWG[c]; nCons = (float)cntG[c]; break;
-                    default: wCons = colWT[c]; nCons = (float)cntT[c]; break;
-                }
-                const float wOrig = ab == 0 ? colWA[c] : ab == 1 ? colWC[c] : ab == 2 ? colWG[c] : colWT[c];
-                const float cv = (float)cov[c];
-                const float oc = (float)origCov[c];
-                const float ec = p.estimatedCoverage;
-                const float f[13] = {__fdiv_rn(oc, cv),           __fdiv_rn(wOrig, wsum), __fdiv_rn(wOrig, oc),
-                                     __fdiv_rn(nCons, cv),        sup[c],                 __fdiv_rn(wCons, nCons),
-                                     __fdiv_rn(wsum, cv),         __fdiv_rn(cv, ec),      __fdiv_rn(wsum, ec),
-                                     avg,                         mins,                   __fdiv_rn((float)maxc, ec),
-                                     __fdiv_rn((float)minc, ec)};
-                if (!forest_decide(p, f)) r = orig;
-            }
-            out[i] = r;
-        }
-        return;
-    }
-    if (nActive == 0) return;
-    const bool byCons = sByConsensus;
-    for (int i = tid; i < La; i += bd) {
-        const int c = aBegin + i;
-        char r;
-        if (byCons) {
-            r = cons[c];
-        } else {
-            r = (sup[c] > 0.90f && origCov[c] <= 2) ? cons[c] : "ACGT"[get2bit(aenc, i)];
-        }
-        out[i] = r;
-    }
 }
 
 // ---------------------------------------------------------------- MSA, warp per anchor
@@ -484,71 +110,345 @@ __device__ __forceinline__ ColInfo col_info(const uint2* wc, int cp, int c) {
     return r;
 }
 
-// One warp per anchor (one warp per block) for reads up to 256 bp.
+// One warp per anchor.
 //
 // Everything the path reads from an MSA -- the different-region search, the
 // properties and both decisions -- lies in the anchor's columns, so only the
 // part of each row that overlaps the anchor is accumulated, in anchor
-// coordinates (column = anchor position).  Shared memory holds per anchor
-// position and base the weight and the count side by side (one 8-byte
-// access per addition); rows are added one at a time
-// (anchor, then the kept candidates in list order) with the lanes over the
-// row's positions, so every column receives its additions in the reference's
-// order.  Lane l owns the columns c with c % 32 == l in every pass (rows,
-// consensus, properties, decision), so consecutive rows need no warp sync.
-// The 2-bit words and the metadata of 32 rows are staged in shared memory per
-// chunk.
+// coordinates (column = anchor position).  Lane l owns the columns c with c % 32
+// == l in every pass.
 //
-// `sm` is the warp's own slice of shared memory (msa_warp_slice_bytes), `qw`
-// the block's quality weights.
-// Walk of the chunk staging loop: word i0 + lane of a chunk's rows is word
-// off of row r (r = (i0 + lane) / pitch); (r0, off0) at i0 = 0 and the step
-// (dr, doff) per 32 words, so that the loop divides nothing.
-struct StageWalk {
-    int r0, off0, dr, doff;
+// Nearly every base of a row equals its column's base, so the build separates the
+// two.  For 32 rows at a time, lane r brings row r's bit planes into the anchor's
+// columns and compares them with the columns' bases: one word of matches and one
+// of mismatches per 32 columns.  The match words are transposed across the warp,
+// so that a lane holds its columns' rows as bits, and each lane adds the rows'
+// weights to its columns' sums in registers, in list order: a test and an addition
+// per row and 32 columns, the counts by population count.  The mismatches (one or
+// two per row) go to a list in row order and are added to their (base, column)
+// entries in shared memory 32 at a time, entries that meet in one place by their
+// order in the list.  A column's base is the anchor's, unless the first 32 rows say
+// that the anchor errs there.  A column's sum of a base thus receives the
+// reference's additions in the reference's order (anchor, then the kept candidates
+// in list order); sums of different bases are independent.
+// Measured, MSA stage: 2M anchors of 150 bp with repeats 13.7 ms (row by row in
+// shared memory 17.2 ms: 116 instructions per row); 60,000 anchors of 300 bp
+// 0.71 ms, 30,000 of 640 bp 1.64 ms, 20,000 of 1000 bp 4.6 ms (a block per anchor,
+// which reads longer than 256 bp used to take, 2.9, 3.1 and 4.2 ms).  It issues in
+// 6 of 10 cycles: a warp's steps depend on one another, and registers and the sums
+// in shared memory leave room for 26 warps per SM (150 bp).
+//
+// `sm` is the warp's own slice of shared memory (MsaSlice), `qw` the block's
+// quality weights.
+
+// Offsets in bytes of one warp's shared memory.  Its first 16 lp bytes hold the
+// weights and counts [4][lp].
+struct MsaSlice {
+    size_t sup, stage, weight, ref, meta, cons, bytes;
+    __host__ __device__ MsaSlice(int lp, int pitch, int wp, const Params& p) {
+        const int words = pitch > 2 * wp ? pitch : 2 * wp;
+        sup = (size_t)lp * 4 * sizeof(uint2);
+        stage = sup + (size_t)lp * sizeof(float);           // 32 rows' planes or 2-bit words; the mismatch list
+        weight = stage + (size_t)32 * words * sizeof(uint32_t);  // [32]
+        ref = weight + 32 * sizeof(float);                   // planes of the columns' bases [2][wp]
+        meta = ref + (size_t)(2 * wp + 3) / 4 * 16;          // [32]: shift, len | orient << 16, weight, id
+        cons = meta + (p.useQuality || p.candidates ? 32 * sizeof(int4) : 0);
+        // candidate correction: the consensus codes of Lmax + 2 new_columns_to_correct columns
+        const size_t cols = (size_t)lp + 2 * (size_t)p.newColumns;
+        bytes = cons + (p.candidates ? (cols + 15) / 16 * 16 + 2 * ((cols + 31) / 32 + 1) * sizeof(uint64_t) : 0);
+    }
 };
 
-template <bool QUAL>
+// x's bits from the n-th most significant on (none from 32 up), and its n most
+// significant bits
+__device__ __forceinline__ uint32_t bits_from(int n) { return __funnelshift_rc(0xffffffffu, 0u, (uint32_t)max(n, 0)); }
+__device__ __forceinline__ uint32_t bits_to(int n) { return ~bits_from(n); }
+
+// A value that is the same in all lanes of the warp, made known as such to the
+// compiler: branches on it need no preparation for a warp that has split.
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __reduce_max_sync(kFull, v); }
+
+// x[k] and its assignment for a k known at run time only, x in registers
+template <int K, typename T>
+__device__ __forceinline__ T pick(const T (&x)[K], int k) {
+    T v = x[0];
+#pragma unroll
+    for (int q = 1; q < K; q++) v = q == k ? x[q] : v;
+    return v;
+}
+template <int K, typename T>
+__device__ __forceinline__ void put(T (&x)[K], int k, T v) {
+#pragma unroll
+    for (int q = 0; q < K; q++) x[q] = q == k ? v : x[q];
+}
+
+// Transposes K 32 x 32 bit matrices, lane r holding row r, most significant bit
+// first: afterwards lane c holds column c.
+template <int K>
+__device__ __forceinline__ void transpose_bits(uint32_t (&x)[K], int lane) {
+    uint32_t half = 0xffff0000u;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+        const bool low = (lane & s) != 0;
+        const uint32_t keep = low ? ~half : half, turn = low ? s : 32 - s;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            const uint32_t y = __shfl_xor_sync(kFull, x[k], s);
+            x[k] = (x[k] & keep) | (__funnelshift_l(y, y, turn) & ~keep);
+        }
+        half = s == 16 ? 0xff00ff00u : s == 8 ? 0xf0f0f0f0u : s == 4 ? 0xccccccccu : 0xaaaaaaaau;
+    }
+}
+
+template <bool QUAL, int K>
 __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params& p, const BatchArg& b,
                                              const uint32_t* __restrict__ rawOff, int lp, int a, uint64_t first,
-                                             unsigned char* sm, const float* qw, const StageWalk sw) {
+                                             unsigned char* sm, const MsaSlice& sl, const float* qw) {
     const int lane = (int)lane_id();
     uint2* wc = reinterpret_cast<uint2*>(sm);                    // [4][lp]: weight bits, count
-    float* sup = reinterpret_cast<float*>(wc + 4 * lp);          // [lp]
-    uint32_t* stage = reinterpret_cast<uint32_t*>(sup + lp);     // [32][pitch]
-    int4* meta = reinterpret_cast<int4*>(stage + 32 * st.pitch);  // [32]: shift, len | orient << 16, weight, id
+    float* sup = reinterpret_cast<float*>(sm + sl.sup);          // [lp]
+    uint32_t* stage = reinterpret_cast<uint32_t*>(sm + sl.stage);
+    uint32_t* list = stage;
+    float* weight = reinterpret_cast<float*>(sm + sl.weight);
+    uint32_t* ref = reinterpret_cast<uint32_t*>(sm + sl.ref);
+    int4* meta = reinterpret_cast<int4*>(sm + sl.meta);  // [32]: shift, len | orient << 16, weight, id
     const uint64_t aid = first + (uint64_t)a;
     const uint64_t oi = (first - out_first(b)) + (uint64_t)a;   // output row
-    const uint32_t nf = b.nfinal[a];
+    const uint32_t nf = warp_uniform(b.nfinal[a]);
     char* out = b.out + oi * b.outPitch;
     if (nf == 0) {
         if (lane == 0) b.flags[oi] = 0;
         return;
     }
-    const uint32_t base = rawOff[a];
-    const int La = st.len[aid];
+    const uint32_t base = warp_uniform(rawOff[a]);
+    const int La = (int)warp_uniform((uint32_t)st.len[aid]);
     const int pitch = st.pitch;
     const uint32_t* aenc = st.enc + aid * (uint64_t)pitch;
     const uint8_t* aq = QUAL ? st.qual + aid * (uint64_t)st.lmax : nullptr;
     constexpr uint8_t kRm = 0x80;
 
-    // Rows are added (sign +1: every row still in the MSA, after the anchor
-    // row) or taken out again (sign -1: the rows just removed, marked kNew).
-    // Returns the number of rows added or taken out.
     constexpr uint8_t kNew = 0x40;
-    auto rowsPass = [&](auto addTag) -> int {
-        constexpr bool add = decltype(addTag)::value;
+    const int wp = st.wp;
+    const uint32_t mine = 0x80000000u >> lane;  // the lane's column in a 32-column word
+    const int listMax = 64 * wp;  // entries the staging area holds
+    using Bits = std::conditional_t<(K <= 16), uint32_t, uint64_t>;  // two bits per 32 columns
+    Bits anchorBits = 0;  // bits 2 k: the anchor's base in column 32 k + lane
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const uint32_t* planes = st.hilo + aid * (2 * (uint64_t)wp) + k;
+        anchorBits |= (Bits)((planes[0] & mine ? 2u : 0u) + (planes[wp] & mine ? 1u : 0u)) << (2 * k);
+    }
+    Bits refBits = 0;  // bits 2 k: the base of column 32 k + lane
+    auto ref_entry = [&](int k) -> uint2* { return wc + (uint32_t)((refBits >> (2 * k)) & 3u) * (uint32_t)lp + (uint32_t)(32 * k + lane); };
+    // The rows still in the MSA (add), or the rows just removed (marked kNew, the
+    // mark is cleared) with their weights' signs turned, are added to wc.  Returns
+    // their number.
+    auto planePass = [&](const bool add) -> int {
         int selected = 0;
+#pragma unroll 1
+        for (uint32_t j0 = 0; j0 < nf; j0 += 32) {
+            const uint32_t jr = j0 + lane;
+            uint32_t mo = kRm, mid = 0;
+            int shift = 0, len = 0;
+            float mw = 0.0f;
+            if (jr < nf) {
+                mo = b.forient[base + jr];
+                shift = b.fshift[base + jr];
+                len = b.flen[base + jr];
+                mid = b.fid[base + jr];
+                mw = b.fweight[base + jr];
+            }
+            const bool sel = jr < nf && (add ? !(mo & kRm) : (mo & kNew) != 0);
+            const unsigned selRows = __ballot_sync(kFull, sel);
+            if (!selRows) continue;
+            if (sel) {  // the row's planes
+                const uint32_t* src = st.hilo + (uint64_t)mid * (2 * wp);
+                for (int q = 0; q < 2 * wp; q += 4) cp_async16(stage + lane * 2 * wp + q, src + q);
+            }
+            if (!add && sel) b.forient[base + jr] = (uint8_t)(mo & ~kNew);
+            if (!add) mw = -mw;
+            weight[lane] = sel ? mw : 0.0f;
+            const bool rc = (mo & 3u) == 2;
+            cp_async_wait_all();
+            __syncwarp();
+            // Columns 32 k .. 32 k + 31 of the row.  Forward they are the stored bases
+            // from -shift + 32 k on; for a reverse complement the last of them is base
+            // len - 32 + shift - 32 k, their order turned.  Words in front of or behind
+            // the row's are whatever lies there in the warp's slice (at most K words before
+            // and K after the staged rows, wp being at least K); the valid columns
+            // leave them out.
+            uint32_t hi[K], lo[K], miss[K];
+            uint32_t rowsOf[K];  // bit 31 - r: row r matches in the lane's column
+            const int to = sel ? min(La, shift + len) : 0;  // its columns: shift .. to - 1
+            int cnt = 0;
+            {
+                const int p0 = rc ? len - 32 + shift : -shift, step = rc ? -1 : 1;
+                const uint32_t* h = stage + lane * 2 * wp + (p0 >> 5) + (rc ? 1 : 0);
+                const uint32_t turn = rc ? 32u - (uint32_t)(p0 & 31) : (uint32_t)(p0 & 31), flip = rc ? ~0u : 0u;
+                uint32_t h0 = h[0], l0 = h[wp];
+                if (rc) {
+                    h0 = __brev(h0);
+                    l0 = __brev(l0);
+                }
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    if (K > 5 && 32 * k >= La) {  // (a store of reads of many lengths)
+                        hi[k] = lo[k] = miss[k] = rowsOf[k] = 0;
+                        continue;
+                    }
+                    h += step;
+                    uint32_t h1 = h[0], l1 = h[wp];
+                    if (rc) {
+                        h1 = __brev(h1);
+                        l1 = __brev(l1);
+                    }
+                    hi[k] = __funnelshift_lc(h1, h0, turn) ^ flip;
+                    lo[k] = __funnelshift_lc(l1, l0, turn) ^ flip;
+                    h0 = h1;
+                    l0 = l1;
+                    const uint32_t valid = bits_from(shift - 32 * k) & bits_to(to - 32 * k);
+                    const uint32_t x = (hi[k] ^ ref[k]) | (lo[k] ^ ref[wp + k]);
+                    rowsOf[k] = valid & ~x;
+                    miss[k] = valid & x;
+                }
+            }
+            transpose_bits(rowsOf, lane);
+            if (add && !selected) {
+                // a column in which far fewer rows match than in the next one: most
+                // likely the anchor's error; its base is then the first mismatching
+                // row's
+                unsigned odd[K], some = 0;
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    const int have = __popc(rowsOf[k]);
+                    odd[k] = __ballot_sync(kFull, 4 * have < __shfl_xor_sync(kFull, have, 1));
+                    some |= (odd[k] ? 1u : 0u) << k;
+                }
+#pragma unroll 1
+                while (some) {  // (one copy of the code for the K words)
+                    const int k = __ffs(some) - 1;
+                    unsigned cols = pick<K>(odd, k);
+                    const int c = __ffs(cols) - 1;
+                    cols &= cols - 1;
+                    put<K>(odd, k, cols);
+                    if (!cols) some &= some - 1;
+                    const uint32_t bit = 0x80000000u >> c, h = pick<K>(hi, k) & bit, l = pick<K>(lo, k) & bit;
+                    uint32_t m = pick<K>(miss, k);
+                    const unsigned differ = __ballot_sync(kFull, (m & bit) != 0);
+                    if (!differ) continue;
+                    const uint32_t nh = __shfl_sync(kFull, h, __ffs(differ) - 1);
+                    const uint32_t nl = __shfl_sync(kFull, l, __ffs(differ) - 1);
+                    const bool in = 32 * k + c >= shift && 32 * k + c < to;
+                    const bool same = in && h == nh && l == nl;
+                    m = (m & ~bit) | (in && !same ? bit : 0u);
+                    put<K>(miss, k, m);
+                    const unsigned now = __ballot_sync(kFull, same);
+                    if (lane == c) {
+                        put<K>(rowsOf, k, __brev(now));
+                        refBits ^= (((refBits >> (2 * k)) & 3u) ^ (Bits)((nh ? 2u : 0u) | (nl ? 1u : 0u))) << (2 * k);
+                        ref[k] = (ref[k] & ~bit) | nh;
+                        ref[wp + k] = (ref[wp + k] & ~bit) | nl;
+                    }
+                    __syncwarp();
+                }
+            }
+            selected += __popc(selRows);
+            // the mismatches, listed as row << 20 | base << 16 | column
+#pragma unroll
+            for (int k = 0; k < K; k++) cnt += __popc(miss[k]);
+            int incl = cnt;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_up_sync(kFull, incl, d);
+                if (lane >= d) incl += y;
+            }
+            const int total = __shfl_sync(kFull, incl, 31);  // all rows' planes have been read
+            for (int from = 0; from < total; from += listMax) {
+                int at = incl - cnt - from;
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    for (uint32_t x = miss[k]; x != 0u;) {
+                        const int bit = __clz(x);
+                        x ^= 0x80000000u >> bit;
+                        const uint32_t q = 2u * ((hi[k] << bit) >> 31) + ((lo[k] << bit) >> 31);
+                        if ((unsigned)at < (unsigned)listMax)
+                            list[at] = ((uint32_t)lane << 20) | (q << 16) | (uint32_t)(32 * k + bit);
+                        at++;
+                    }
+                }
+                __syncwarp();
+                const int n0 = min(listMax, total - from);
+                for (int e0 = 0; e0 < n0; e0 += 32) {
+                    const bool has = e0 + lane < n0;
+                    const uint32_t e = has ? list[e0 + lane] : 0xffffffffu;
+                    const uint32_t c = e & 0xffffu, slot = ((e >> 16) & 3u) * (uint32_t)lp + c, r = (e >> 20) & 31u;
+                    const float wt = weight[r];
+                    const uint32_t before = __popc(__match_any_sync(kFull, e & 0xfffffu) & ((1u << lane) - 1u));
+                    const uint32_t rounds = __reduce_max_sync(kFull, has ? before : 0u);
+                    for (uint32_t t = 0; t <= rounds; t++) {
+                        if (has && before == t) {
+                            uint2 v = wc[slot];
+                            v.x = __float_as_uint(__fadd_rn(__uint_as_float(v.x), wt));
+                            v.y += add ? 1u : ~0u;
+                            wc[slot] = v;
+                        }
+                        __syncwarp();
+                    }
+                }
+            }
+            // the matches
+            const int rows = 32 - __clz(selRows);
+            float w[K];
+#pragma unroll
+            for (int k = 0; k < K; k++) w[k] = rowsOf[k] ? __uint_as_float(ref_entry(k)->x) : 0.0f;
+            uint32_t left[K];
+#pragma unroll
+            for (int k = 0; k < K; k++) left[k] = rowsOf[k];
+#pragma unroll 1
+            for (int r0 = 0; r0 < rows; r0 += 8) {
+                float wr[8];
+                *reinterpret_cast<float4*>(wr) = *reinterpret_cast<const float4*>(weight + r0);
+                *reinterpret_cast<float4*>(wr + 4) = *reinterpret_cast<const float4*>(weight + r0 + 4);
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    if (K > 5 && 32 * k >= La) break;
+#pragma unroll
+                    for (int r = 0; r < 8; r++)
+                        if (left[k] & (0x80000000u >> r)) w[k] = __fadd_rn(w[k], wr[r]);
+                    left[k] <<= 8;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < K; k++) {
+                if (!rowsOf[k]) continue;
+                uint2* const entry = ref_entry(k);
+                const int n = __popc(rowsOf[k]);
+                *entry = make_uint2(__float_as_uint(w[k]), entry->y + (add ? n : -n));
+            }
+            __syncwarp();  // the next chunk overwrites the staged rows and weights
+        }
+        __syncwarp();
+        return selected;
+    };
+
+    // The same with quality scores: every base has its own weight, so the rows are
+    // added one at a time, with the lanes over the row's columns.  (The other pass
+    // needs a load per row and 32 columns for the matches' qualities as well, and
+    // then measured 6.5 ms where this one takes 5.5: 300,000 reads of 50 to 250 bp.)
+    auto qualityPass = [&](const bool add) -> int {
+        int selected = 0;
+        const uint32_t one = add ? 1u : ~0u;
+#pragma unroll 1
         for (uint32_t j0 = 0; j0 < nf; j0 += 32) {
             const uint32_t jr = j0 + lane;
             const int rows = (int)min(32u, nf - j0);
             uint32_t mo = kRm, mid = 0;
-            int mshift = 0, mlen = 0;
+            int shift = 0, len = 0;
             float mw = 0.0f;
             if (jr < nf) {
                 mo = b.forient[base + jr];
-                mshift = b.fshift[base + jr];
-                mlen = b.flen[base + jr];
+                shift = b.fshift[base + jr];
+                len = b.flen[base + jr];
                 mid = b.fid[base + jr];
                 mw = b.fweight[base + jr];
             }
@@ -557,63 +457,46 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
             if (!selRows) continue;
             selected += __popc(selRows);
             if (!add && sel) b.forient[base + jr] = (uint8_t)(mo & ~kNew);
-            // the selected rows' 2-bit words, copied without a register round
-            // trip and waited for once
-            {
-                const int total = rows * pitch;
-                int r = sw.r0, off = sw.off0;
-                for (int i0 = 0; i0 < total; i0 += 32) {  // warp-uniform trip count
-                    const int rr = min(r, rows - 1);
-                    const uint32_t rid = __shfl_sync(kFull, mid, rr);
-                    if (i0 + lane < total && ((selRows >> rr) & 1u))
-                        cp_async4(stage + i0 + lane, st.enc + (uint64_t)rid * pitch + off);
-                    r += sw.dr;
-                    off += sw.doff;
-                    if (off >= pitch) {
-                        off -= pitch;
-                        r++;
-                    }
-                }
+            if (sel) {
+                const uint32_t* src = st.hilo + (uint64_t)mid * (2 * wp);
+                for (int q = 0; q < 2 * wp; q += 4) cp_async16(stage + lane * 2 * wp + q, src + q);
             }
-            meta[lane] = make_int4(mshift, mlen | (int)((mo & 3u) << 16), __float_as_int(mw), (int)mid);
+            meta[lane] = make_int4(shift, len | (int)((mo & 3u) << 16), __float_as_int(add ? mw : -mw), (int)mid);
             cp_async_wait_all();
             __syncwarp();
+#pragma unroll 1
             for (int r = 0; r < rows; r++) {
                 if (!((selRows >> r) & 1u)) continue;
                 const int4 md = meta[r];
                 const bool rc = ((uint32_t)md.y >> 16) == 2;
-                const int shift = md.x, len = md.y & 0xffff;
-                const float weight = __int_as_float(md.z);
-                const uint32_t* e = stage + r * pitch;
-                const uint8_t* q = QUAL ? st.qual + (uint64_t)(uint32_t)md.w * st.lmax : nullptr;
-                const int c0 = max(shift, 0), c1 = min(La, shift + len);  // overlap with the anchor
-                int c = c0 + ((lane - c0) & 31);                           // this lane's first column
-                // the row position moves by 32 per column step of the lane, so
-                // its word moves by 2 and its bit offset stays
-                int sp = rc ? len - 1 - (c - shift) : c - shift;
-                const int dsp = rc ? -32 : 32, dwi = rc ? -2 : 2;
-                const uint32_t sh = 30u - 2u * (uint32_t)(sp & 15), flip = rc ? 3u : 0u;
-                // quality index: sp, or for a reverse complement row Lmax - 1 - (c - shift)
-                const int qd = rc ? st.lmax - len : 0;
-                // padding past the read's end is read as stored
-                auto wtAt = [&](int s) -> float { return QUAL ? __fmul_rn(weight, qw[q[s + qd]]) : weight; };
-                auto upd = [&](uint2& v, float wt) {
-                    if (add) {
-                        v.x = __float_as_uint(__fadd_rn(__uint_as_float(v.x), wt));
-                        v.y++;
-                    } else {
-                        v.x = __float_as_uint(__fsub_rn(__uint_as_float(v.x), wt));
-                        v.y--;
-                    }
+                const int rshift = md.x, rlen = md.y & 0xffff;
+                const float wr = __int_as_float(md.z);
+                const uint32_t* h = stage + r * 2 * wp;
+                const int c0 = max(rshift, 0), c1 = min(La, rshift + rlen);  // overlap with the anchor
+                int c = c0 + ((lane - c0) & 31);                             // this lane's first column
+                // the row position moves by 32 per column step of the lane, so its
+                // word moves by one and its bit stays
+                int sp = rc ? rlen - 1 - (c - rshift) : c - rshift;
+                const int dsp = rc ? -32 : 32, dwi = rc ? -1 : 1;
+                const int up = sp & 31;
+                const uint32_t flip = rc ? 3u : 0u;
+                // quality of position sp (row_quality; padding past the read's end is
+                // read as stored)
+                const uint8_t* q = st.qual + (uint64_t)(uint32_t)md.w * st.lmax + (rc ? st.lmax - rlen : 0);
+                auto baseAt = [&](int w) -> uint32_t {
+                    return (((h[w] << up) >> 31) * 2u + ((h[wp + w] << up) >> 31)) ^ flip;
                 };
-                int wi = sp >> 4;
-                // two of the lane's columns (c and c + 32) per iteration: both
-                // words and both entries are read before either is written
-                // (distinct columns, distinct entries)
+                auto upd = [&](uint2& v, float wt) {
+                    v.x = __float_as_uint(__fadd_rn(__uint_as_float(v.x), wt));
+                    v.y += one;
+                };
+                int wi = sp >> 5;
+                // two of the lane's columns (c and c + 32) per iteration: both words and
+                // both entries are read before either is written (distinct columns,
+                // distinct entries)
                 for (; c + 32 < c1; c += 64, wi += 2 * dwi, sp += 2 * dsp) {
-                    const uint32_t b0 = ((e[wi] >> sh) & 3u) ^ flip;
-                    const uint32_t b1 = ((e[wi + dwi] >> sh) & 3u) ^ flip;
-                    const float w0 = wtAt(sp), w1 = wtAt(sp + dsp);
+                    const uint32_t b0 = baseAt(wi), b1 = baseAt(wi + dwi);
+                    const float w0 = __fmul_rn(wr, qw[q[sp]]), w1 = __fmul_rn(wr, qw[q[sp + dsp]]);
                     uint2* p0 = wc + b0 * lp + c;
                     uint2* p1 = wc + b1 * lp + (c + 32);
                     uint2 v0 = *p0, v1 = *p1;
@@ -623,74 +506,122 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
                     *p1 = v1;
                 }
                 if (c < c1) {
-                    const uint32_t b0 = ((e[wi] >> sh) & 3u) ^ flip;
-                    uint2* p0 = wc + b0 * lp + c;
+                    uint2* p0 = wc + baseAt(wi) * lp + c;
                     uint2 v0 = *p0;
-                    upd(v0, wtAt(sp));
+                    upd(v0, __fmul_rn(wr, qw[q[sp]]));
                     *p0 = v0;
                 }
             }
             __syncwarp();  // the next chunk overwrites the staged rows
         }
+        __syncwarp();
         return selected;
     };
-    // The MSA of the rows still in it, built as the reference builds it: the
-    // anchor row (weight 1 times the quality weight), then the rows in order.
-    // Returns the number of rows it holds besides the anchor.
-    auto build = [&]() -> int {
-        for (int pos = lane; pos < La; pos += 32) {
-            const uint32_t bb = get2bit(aenc, pos);
-            const float wt = QUAL ? __fmul_rn(1.0f, qw[aq[pos]]) : 1.0f;
+    // add: builds the MSA of the rows still in it as the reference does, from the
+    // anchor row (weight 1 times the quality weight) and the rows in order.
+    // Otherwise takes the rows just removed out of wc.  Returns the number of rows.
+    auto rowsPass = [&](const bool add) -> int {
+        if (add) {
+            refBits = anchorBits;
+            if (!QUAL)
+                for (int i = lane; i < 2 * wp; i += 32) ref[i] = st.hilo[aid * (2 * (uint64_t)wp) + i];
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                wc[q * lp + pos] = (uint32_t)q == bb ? make_uint2(__float_as_uint(__fadd_rn(0.0f, wt)), 1u)
-                                                     : make_uint2(__float_as_uint(0.0f), 0u);
+            for (int k = 0; k < K; k++) {
+                const int c = 32 * k + lane;
+                if (c >= La) break;
+#pragma unroll
+                for (int q = 0; q < 4; q++) wc[q * lp + c] = make_uint2(0u, 0u);
+                *ref_entry(k) = make_uint2(__float_as_uint(QUAL ? __fmul_rn(1.0f, qw[aq[c]]) : 1.0f), 1u);
             }
         }
-        __syncwarp();
-        return rowsPass(std::true_type{});
+        if constexpr (QUAL)
+            return qualityPass(add);
+        else
+            return planePass(add);
     };
 
-    int builds = 0;
-    bool exact = true, haveS = false;
-    int nActive = build();
+    // Rounds of refinement.  A round begins with a build, or with the removal of
+    // the rows that the one before it took out; `last` ends them after the next
+    // build.  Everything that is read from a column's sums is read once a round,
+    // and stays in registers: the consensus (consBits, as anchorBits), whether at
+    // most two rows have the anchor's base (fewBits), the support, the coverage.
+    int builds = 1, iter = 0, nActive = -1;
+    bool build = true, haveS = false, last = false;
+    Bits consBits;
+    uint32_t fewBits;
+    float support[K];
+    int minc, maxc;
     const float tol = __fmul_rn(2.5f * 5.9604645e-8f, (float)(3 * nf + 4));  // 2 E_c / S_c with slack
-    for (int iter = 0;; iter++) {
-        builds++;
-        if (iter == 5 || nActive == 0) break;
-        if (!exact) {
-            bool close = false;
-            for (int c = lane; c < La; c += 32) {
-                float t1 = 0.0f, t2 = 0.0f;  // the two largest weights
-                const ColInfo ci = col_info(wc, lp, c);
+    while (true) {
+        const int rows = rowsPass(build);
+        if (nActive < 0) nActive = rows;
+        const bool exact = build;
+        bool close = false, mism = false;
+        int firstSig = 0x7fffffff;
+        consBits = 0;
+        fewBits = 0;
+        minc = 0x7fffffff;
+        maxc = -1;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            const int c = 32 * k + lane;
+            support[k] = 0.0f;
+            if (c >= La) continue;
+            float v[4];
+            int n[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const uint2 e = wc[q * lp + c];
+                v[q] = __uint_as_float(e.x);
+                n[q] = (int)e.y;
+            }
+            const float colW = __fadd_rn(__fadd_rn(__fadd_rn(v[0], v[1]), v[2]), v[3]);
+            float consW = v[0];
+            uint32_t cons = 0;
+#pragma unroll
+            for (int q = 1; q < 4; q++)
+                if (v[q] > consW) {
+                    consW = v[q];
+                    cons = q;
+                }
+            if (!exact) {  // are the two largest weights too close to tell them apart?
+                float t1 = 0.0f, t2 = 0.0f;
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    const float v = ci.w[q];
-                    t2 = fmaxf(t2, fminf(t1, v));
-                    t1 = fmaxf(t1, v);
+                    t2 = fmaxf(t2, fminf(t1, v[q]));
+                    t1 = fmaxf(t1, v[q]);
                 }
                 close |= !(__fsub_rn(t1, t2) > __fmul_rn(tol, sup[c]));
             }
-            if (__any_sync(kFull, close)) {
-                build();
-                exact = true;
-            }
-        }
-        // findCandidatesOfDifferentRegion (src/msa.cpp:532-734), in anchor coordinates
-        bool mism = false;
-        int firstSig = 0x7fffffff;
-        for (int c = lane; c < La; c += 32) {
-            const ColInfo ci = col_info(wc, lp, c);
-            mism |= ci.cons != "ACGT"[get2bit(aenc, c)];
-            const int cidx = base_index(ci.cons);
+            const uint32_t ab = (uint32_t)(anchorBits >> (2 * k)) & 3u;
+            mism |= cons != ab;
             bool sig = false;
 #pragma unroll
-            for (int i = 0; i < 4; i++) sig |= (i != cidx && p.significantCount <= (int)ci.n[i]);
-            if (sig && c < firstSig) firstSig = c;
+            for (int q = 0; q < 4; q++) sig |= (uint32_t)q != cons && p.significantCount <= n[q];
+            if (sig) firstSig = min(firstSig, c);
+            consBits |= (Bits)cons << (2 * k);
+            if ((ab & 2u ? (ab & 1u ? n[3] : n[2]) : (ab & 1u ? n[1] : n[0])) <= 2) fewBits |= 1u << k;
+            support[k] = __fdiv_rn(consW, colW);
+            const int cov = n[0] + n[1] + n[2] + n[3];
+            minc = min(minc, cov);
+            maxc = max(maxc, cov);
         }
-        if (!__any_sync(kFull, mism)) break;
+        if (last) break;
+        last = build = true;  // unless this round removes rows
+        if (iter == 5 || nActive == 0) {
+            if (exact) break;
+            continue;
+        }
+        if (__any_sync(kFull, close)) {
+            last = false;  // the round again, from an exact MSA
+            continue;
+        }
+        // findCandidatesOfDifferentRegion (src/msa.cpp:532-734), in anchor coordinates
         const int col = __reduce_min_sync(kFull, firstSig);
-        if (col == 0x7fffffff) break;
+        if (!__any_sync(kFull, mism) || col == 0x7fffffff) {
+            if (exact) break;
+            continue;
+        }
         int found;
         {
             const ColInfo ci = col_info(wc, lp, col);
@@ -715,6 +646,7 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
             return keepMatching ? (bb != (uint32_t)found) : (bb == (uint32_t)found);
         };
         bool veto = false, any = false;
+#pragma unroll 1
         for (uint32_t j = lane; j < nf; j += 32) {
             if ((b.forient[base + j] & kRm) || !differs(j)) continue;
             any = true;
@@ -722,8 +654,12 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
         }
         // a veto (or nothing to remove) leaves the MSA as it is; the
         // reference then rebuilds the same MSA and reaches the same decision
-        if (__any_sync(kFull, veto) || !__any_sync(kFull, any)) break;
+        if (__any_sync(kFull, veto) || !__any_sync(kFull, any)) {
+            if (exact) break;
+            continue;
+        }
         int act = 0;
+#pragma unroll 1
         for (uint32_t j = lane; j < nf; j += 32) {
             const uint8_t o = b.forient[base + j];
             if (!(o & kRm) && differs(j)) b.forient[base + j] = o | kRm | kNew;
@@ -731,25 +667,23 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
         }
         nActive = __reduce_add_sync(kFull, act);
         if (!haveS) {  // S_c (the first build, which wc still holds), kept in `sup` until the properties
+#pragma unroll 1
             for (int c = lane; c < La; c += 32) sup[c] = col_info(wc, lp, c).colW;
             haveS = true;
         }
         __syncwarp();
-        rowsPass(std::false_type{});
-        exact = false;
+        last = build = false;
+        iter++;
+        builds++;
     }
-    if (!exact) build();
     // getMSAProperties (src/msa.cpp:304-376) and the decision
     float mins = 3.402823466e+38f;
-    int minc = 0x7fffffff, maxc = -1;
-    for (int c = lane; c < La; c += 32) {
-        const ColInfo ci = col_info(wc, lp, c);
-        const float s = __fdiv_rn(ci.consW, ci.colW);
-        sup[c] = s;
-        mins = fminf(mins, s);
-        const int cv = ci.cov();
-        minc = min(minc, cv);
-        maxc = max(maxc, cv);
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const int c = 32 * k + lane;
+        if (c >= La) continue;
+        sup[c] = support[k];
+        mins = fminf(mins, support[k]);
     }
     for (int d = 16; d > 0; d >>= 1) mins = fminf(mins, __shfl_xor_sync(kFull, mins, d));
     minc = __reduce_min_sync(kFull, minc);
@@ -760,10 +694,12 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
         float sum = 0.0f;
         const float4* s4 = reinterpret_cast<const float4*>(sup);
         int i = 0;
+#pragma unroll 4
         for (; i + 4 <= La; i += 4) {
             const float4 v = s4[i >> 2];
             sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, v.x), v.y), v.z), v.w);
         }
+#pragma unroll 1
         for (; i < La; i++) sum = __fadd_rn(sum, sup[i]);
         avg = __fdiv_rn(sum, (float)La);
     }
@@ -773,6 +709,7 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
     bool hq = false;
     if (good) {
         int smallest = 100;
+#pragma unroll 1
         for (int percent = p.errPercent; percent >= 0; percent--) {
             if (fgeq(avg, p.hqAvg[percent]) && fgeq(mins, p.hqMin[percent])) smallest = percent;
         }
@@ -789,35 +726,38 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
         b.flags[oi] = corrected ? (uint8_t)(CG_RESULT_CORRECTED | (hq ? CG_RESULT_HQ : 0)) : (uint8_t)0;
     }
     if (!corrected) return;
-    for (int c = lane; c < La; c += 32) {
+    if (!forest) {
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            const int c = 32 * k + lane;
+            const bool take = good || (support[k] > 0.90f && ((fewBits >> k) & 1u));
+            const uint32_t code = (uint32_t)((take ? consBits : anchorBits) >> (2 * k)) & 3u;
+            if (c < La) out[c] = (char)__byte_perm(0x54474341u, 0u, code);  // "ACGT"[code]
+        }
+    }
+#pragma unroll 1
+    for (int c = lane; forest && c < La; c += 32) {
         const uint32_t ab = get2bit(aenc, c);
         const char orig = "ACGT"[ab];
         const ColInfo ci = col_info(wc, lp, c);
         const int origCov = (int)ci.nOf(ab);
-        char r;
-        if (forest) {
-            // correctAnchorClf (include/corrector.hpp:1448-1472), features of
-            // include/classification.hpp:748-797
-            r = ci.cons;
-            if (!hq && r != orig) {
-                const int ci_ = base_index(ci.cons);
-                const float wCons = ci.wOf((uint32_t)ci_);
-                const float nCons = (float)ci.nOf((uint32_t)ci_);
-                const float wOrig = ci.wOf(ab);
-                const float cv = (float)ci.cov();
-                const float oc = (float)origCov;
-                const float ec = p.estimatedCoverage;
-                const float f[13] = {__fdiv_rn(oc, cv),      __fdiv_rn(wOrig, ci.colW), __fdiv_rn(wOrig, oc),
-                                     __fdiv_rn(nCons, cv),   sup[c],                    __fdiv_rn(wCons, nCons),
-                                     __fdiv_rn(ci.colW, cv), __fdiv_rn(cv, ec),         __fdiv_rn(ci.colW, ec),
-                                     avg,                    mins,                      __fdiv_rn((float)maxc, ec),
-                                     __fdiv_rn((float)minc, ec)};
-                if (!forest_decide(p, f)) r = orig;
-            }
-        } else if (good) {
-            r = ci.cons;
-        } else {
-            r = (sup[c] > 0.90f && origCov <= 2) ? ci.cons : orig;
+        // correctAnchorClf (include/corrector.hpp:1448-1472), features of
+        // include/classification.hpp:748-797
+        char r = ci.cons;
+        if (!hq && r != orig) {
+            const int ci_ = base_index(ci.cons);
+            const float wCons = ci.wOf((uint32_t)ci_);
+            const float nCons = (float)ci.nOf((uint32_t)ci_);
+            const float wOrig = ci.wOf(ab);
+            const float cv = (float)ci.cov();
+            const float oc = (float)origCov;
+            const float ec = p.estimatedCoverage;
+            const float f[13] = {__fdiv_rn(oc, cv),      __fdiv_rn(wOrig, ci.colW), __fdiv_rn(wOrig, oc),
+                                 __fdiv_rn(nCons, cv),   sup[c],                    __fdiv_rn(wCons, nCons),
+                                 __fdiv_rn(ci.colW, cv), __fdiv_rn(cv, ec),         __fdiv_rn(ci.colW, ec),
+                                 avg,                    mins,                      __fdiv_rn((float)maxc, ec),
+                                 __fdiv_rn((float)minc, ec)};
+            if (!forest_decide(p, f)) r = orig;
         }
         out[c] = r;
     }
@@ -828,12 +768,15 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
         // e - nc left of the anchor, or La + e - nc right of it).  cons8[x] =
         // consensus base code of column x - nc, for x in [0, La + 2 nc).
         const int nc = p.newColumns;
-        uint8_t* cons8 = reinterpret_cast<uint8_t*>(meta + 32);
+        uint8_t* cons8 = reinterpret_cast<uint8_t*>(sm + sl.cons);
+#pragma unroll 1
         for (int c = lane; c < La; c += 32) cons8[nc + c] = (uint8_t)base_index(col_info(wc, lp, c).cons);
+#pragma unroll 1
         for (int e0 = 0; e0 < 2 * nc; e0 += 32) {  // warp-uniform trip count
             const int e = e0 + lane;
             const int col = e < nc ? e - nc : La + (e - nc);
             float w4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 1
             for (uint32_t j0 = 0; j0 < nf; j0 += 32) {
                 const uint32_t jr = j0 + lane;
                 const int rows = (int)min(32u, nf - j0);
@@ -851,6 +794,7 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
                 const bool sel = jr < nf && !(mo & kRm) && (mshift < 0 || mshift + mlen > La);
                 const unsigned selRows = __ballot_sync(kFull, sel);
                 if (!selRows) continue;
+#pragma unroll 1
                 for (int i0 = 0; i0 < rows * pitch; i0 += 32) {
                     const int idx = i0 + lane;
                     const int r = min(idx / pitch, rows - 1);
@@ -860,6 +804,7 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
                 }
                 meta[lane] = make_int4(mshift, mlen | (int)((mo & 3u) << 16), __float_as_int(mw), (int)mid);
                 __syncwarp();
+#pragma unroll 1
                 for (int r = 0; r < rows; r++) {
                     if (!((selRows >> r) & 1u)) continue;
                     const int4 md = meta[r];
@@ -902,8 +847,10 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
             reinterpret_cast<unsigned long long*>(cons8 + ((size_t)lp + 2 * (size_t)nc + 15) / 16 * 16);
         unsigned long long* rv = fw + nw + 1;
         __syncwarp();
+#pragma unroll 1
         for (int u = lane; u <= nw; u += 32) {
             unsigned long long f = 0, r = 0;
+#pragma unroll 1
             for (int t = 0; t < 32; t++) {
                 const int x = 32 * u + t;
                 if (x < X) {
@@ -917,6 +864,7 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
         __syncwarp();
         // one row per lane
         int votes = 0;
+#pragma unroll 1
         for (uint32_t j = lane; j < nf; j += 32) {
             const uint32_t g = base + j;
             const uint8_t o = b.forient[g];
@@ -927,6 +875,7 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
             const unsigned long long* src = rc ? rv : fw;
             const int y0 = rc ? X - (nc + s) - len : nc + s;  // the slice's first position in src
             const uint32_t id = b.fid[g];
+#pragma unroll 1
             for (int w = 0; w * 32 < len; w++) {
                 const int y = y0 + 32 * w, u = y >> 5, off = 2 * (y & 31);
                 unsigned long long v = src[u] << off;
@@ -947,10 +896,12 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
     // anchor's base, with its features; the classifier then replaces the
     // decision written above (the fallback) where it is confident.
     int nd = 0;
+#pragma unroll 1
     for (int c = lane; c < La; c += 32) nd += col_info(wc, lp, c).cons != "ACGT"[get2bit(aenc, c)];
     nd = __reduce_add_sync(kFull, nd);
     const float ec = p.estimatedCoverage;
     const float invLa = __fdiv_rn(1.0f, (float)La);
+#pragma unroll 1
     for (int c0 = 0; c0 < La; c0 += 32) {  // warp-uniform trip count
         const int c = c0 + lane;
         bool rec = false;
@@ -1029,50 +980,43 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
     }
 }
 
-// Bytes of shared memory one warp of msa_warp_kernel works in (with candidate
-// correction, the consensus codes of Lmax + 2 new_columns_to_correct columns
-// follow the row metadata).
-__host__ __device__ inline size_t msa_warp_slice_bytes(int lp, int pitch, const Params& p) {
-    const size_t cols = (size_t)lp + 2 * (size_t)p.newColumns;
-    const size_t cand = p.candidates ? (cols + 15) / 16 * 16 + 2 * ((cols + 31) / 32 + 1) * sizeof(uint64_t) : 0;
-    return (size_t)lp * (9 * sizeof(float)) + (size_t)32 * pitch * sizeof(uint32_t) + 32 * sizeof(int4) + cand;
-}
-
 // `warps` warps per block, each on its own anchors.  Plain form: anchor
 // blockIdx.x * warps + warp.  Persistent form (b.work set): warps take the
 // next anchor from the counter b.work[0] until the batch is done.
-__global__ void __launch_bounds__(256, 4) msa_warp_kernel(StoreArg st, Params p, BatchArg b,
-                                                       const uint32_t* __restrict__ rawOff, int lp) {
+// At least as many registers as the K-word arrays need; shared memory bounds the
+// resident warps from K = 8 on.
+template <bool QUAL, int K>
+__global__ void __launch_bounds__(256, K > 16 ? 1 : K > 8 ? 2 : QUAL || K > 5 ? 3 : 4)
+    msa_warp_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ rawOff, int lp) {
     extern __shared__ __align__(16) unsigned char sm[];
-    float* qw = reinterpret_cast<float*>(sm);  // [256] (quality scores only)
     const int warp = (int)(threadIdx.x >> 5), warps = (int)(blockDim.x >> 5);
-    const size_t qbytes = p.useQuality ? 256 * sizeof(float) : 0;
-    unsigned char* slice = sm + qbytes + (size_t)warp * msa_warp_slice_bytes(lp, st.pitch, p);
-    if (p.useQuality) {
+    const MsaSlice sl(lp, st.pitch, st.wp, p);
+    // The slice's address is kept in a register: left to itself the compiler builds
+    // a shared address from the block's number in its cluster for every access.
+    uint32_t at = (uint32_t)__cvta_generic_to_shared(sm + (QUAL ? 256 * sizeof(float) : 0) + (size_t)warp * sl.bytes);
+    asm volatile("" : "+r"(at));
+    unsigned char* slice = static_cast<unsigned char*>(__cvta_shared_to_generic(at));
+    uint32_t qwAt = (uint32_t)__cvta_generic_to_shared(sm);
+    asm volatile("" : "+r"(qwAt));
+    float* qw = static_cast<float*>(__cvta_shared_to_generic(qwAt));  // [256] (quality scores only)
+    if (QUAL) {
         for (int i = threadIdx.x; i < 256; i += blockDim.x) qw[i] = p.qweight[i];
         __syncthreads();
     }
     const uint64_t first = batch_first(b);
-    const int lane = (int)lane_id(), pitch = st.pitch;
-    const StageWalk sw{lane / pitch, lane % pitch, 32 / pitch, 32 % pitch};
-    auto anchor = [&](int i) {
-        const int a = b.order ? (int)b.order[i] : i;
-        if (p.useQuality) msa_warp_anchor<true>(st, p, b, rawOff, lp, a, first, slice, qw, sw);
-        else msa_warp_anchor<false>(st, p, b, rawOff, lp, a, first, slice, qw, sw);
-    };
-    if (!b.work) {
-        const int i = blockIdx.x * warps + warp;
-        if (i < b.count) anchor(i);
-        return;
-    }
-    while (true) {
-        int i = 0;
-        if (lane == 0) i = (int)atomicAdd(&b.work[0], 1u);
-        i = __shfl_sync(kFull, i, 0);
+    const int lane = (int)lane_id();
+    const bool persistent = b.work != nullptr;
+    int i = blockIdx.x * warps + warp;
+    do {
+        if (persistent) {
+            i = lane == 0 ? (int)atomicAdd(&b.work[0], 1u) : 0;
+        }
+        i = (int)warp_uniform((uint32_t)i);
         if (i >= b.count) return;
-        anchor(i);
+        const int a = (int)warp_uniform(b.order ? b.order[i] : (uint32_t)i);
+        msa_warp_anchor<QUAL, K>(st, p, b, rawOff, lp, a, first, slice, sl, qw);
         __syncwarp();
-    }
+    } while (persistent);
 }
 
 constexpr int kOrderBuckets = 16;
@@ -1125,66 +1069,67 @@ __global__ void msa_order_scatter_kernel(const uint32_t* __restrict__ nfinal, in
 
 }  // namespace
 
-int msa_threads(int maxCols) {
-    int t = kMsaThreadsMin;
-    while (t * kMsaCols < maxCols) t += 32;
-    return t;
-}
-
-size_t msa_smem_bytes(int maxCols, int bitsetWords, int storeWeights) {
-    return sizeof(RowMeta) * kMsaChunkRows + sizeof(uint32_t) * bitsetWords + 256 * sizeof(float) +
-           (size_t)maxCols * (7 * sizeof(int) + 1 + (storeWeights ? 4 * sizeof(float) : 0));
-}
-
 namespace {
 
-size_t msa_warp_smem(StoreArg st, Params p, int warps) {
-    const int lp = (st.lmax + 31) / 32 * 32;
-    return (p.useQuality ? 256 * sizeof(float) : 0) + (size_t)warps * msa_warp_slice_bytes(lp, st.pitch, p);
+// The instance for a store -- as many 32-column words as its longest read takes,
+// every word costs a share of each pass -- and its shared memory per warp.
+struct MsaInstance {
+    void (*kernel)(StoreArg, Params, BatchArg, const uint32_t*, int);
+    size_t slice;
+};
+template <int K>
+MsaInstance msa_instance_of(StoreArg st, const Params& p) {
+    return {p.useQuality ? msa_warp_kernel<true, K> : msa_warp_kernel<false, K>,
+            MsaSlice((st.lmax + 31) / 32 * 32, st.pitch, st.wp, p).bytes};
+}
+MsaInstance msa_instance(StoreArg st, const Params& p) {
+    const int words = (st.lmax + 31) / 32;
+    return words <= 4    ? msa_instance_of<4>(st, p)
+           : words <= 5  ? msa_instance_of<5>(st, p)
+           : words <= 8  ? msa_instance_of<8>(st, p)
+           : words <= 10 ? msa_instance_of<10>(st, p)
+           : words <= 16 ? msa_instance_of<16>(st, p)
+           : words <= 20 ? msa_instance_of<20>(st, p)
+                         : msa_instance_of<32>(st, p);
 }
 
-cudaError_t msa_warp_prepare(size_t smem) {
+size_t msa_warp_smem(const MsaInstance& m, const Params& p, int warps) {
+    return (p.useQuality ? 256 * sizeof(float) : 0) + (size_t)warps * m.slice;
+}
+
+// warps per block: as asked for, but no more than the shared memory of a block holds
+int msa_fit_warps(const MsaInstance& m, const Params& p, int warps) {
+    while (warps > 1 && msa_warp_smem(m, p, warps) > 227 * 1024) warps--;
+    return warps < 1 ? 1 : warps;
+}
+
+cudaError_t msa_warp_prepare(const MsaInstance& m, size_t smem) {
     if (smem <= 40 * 1024) return cudaSuccess;  // leaves room for the kernel's static shared memory
-    return cudaFuncSetAttribute(msa_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return cudaFuncSetAttribute(m.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
 }  // namespace
 
 int msa_warp_occupancy(StoreArg st, Params p, int warps) {
-    if (st.lmax > 256 || warps < 1 || warps > 8) return 0;
-    const size_t smem = msa_warp_smem(st, p, warps);
-    if (msa_warp_prepare(smem) != cudaSuccess) return 0;
+    const MsaInstance m = msa_instance(st, p);
+    warps = msa_fit_warps(m, p, warps);
+    const size_t smem = msa_warp_smem(m, p, warps);
+    if (msa_warp_prepare(m, smem) != cudaSuccess) return 0;
     int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, msa_warp_kernel, warps * 32, smem) != cudaSuccess)
-        return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, m.kernel, warps * 32, smem) != cudaSuccess) return 0;
     return blocks;
 }
 
-cudaError_t launch_msa_correct(StoreArg st, Params p, BatchArg b, int maxRows, cudaStream_t s, const Shape* shape) {
-    const int maxCols = 3 * st.lmax + 4;
-    if (st.lmax <= 256) {
-        const int lp = (st.lmax + 31) / 32 * 32;
-        const bool persistent = shape && b.work;
-        const int warps = persistent ? shape->msaWarps : 1;
-        const size_t smem = msa_warp_smem(st, p, warps);
-        cudaError_t e = msa_warp_prepare(smem);
-        if (e != cudaSuccess) return e;
-        const unsigned blocks = persistent ? (unsigned)shape->msaBlocks : (unsigned)b.count;
-        if (blocks == 0) return cudaSuccess;
-        msa_warp_kernel<<<blocks, warps * 32, smem, s>>>(st, p, b, b.rawCount, lp);
-        return cudaGetLastError();
-    }
-    const int bitsetWords = (maxRows + 31) / 32 + 1;
-    const int storeWeights = p.correctionType == CG_CORR_FOREST;
-    const size_t smem = msa_smem_bytes(maxCols, bitsetWords, storeWeights);
-    if (smem > 40 * 1024) {  // leaves room for the kernel's static shared memory
-        cudaError_t e = cudaFuncSetAttribute(msa_correct_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return e;
-    }
-    if (b.count == 0) return cudaSuccess;
-    msa_correct_kernel<<<b.count, msa_threads(maxCols), smem, s>>>(st, p, b, b.rawCount, maxCols, bitsetWords,
-                                                                    storeWeights);
+cudaError_t launch_msa_correct(StoreArg st, Params p, BatchArg b, cudaStream_t s, const Shape* shape) {
+    const bool persistent = shape && b.work;
+    const MsaInstance m = msa_instance(st, p);
+    const int warps = persistent ? msa_fit_warps(m, p, shape->msaWarps) : 1;
+    const size_t smem = msa_warp_smem(m, p, warps);
+    const cudaError_t e = msa_warp_prepare(m, smem);
+    if (e != cudaSuccess) return e;
+    const unsigned blocks = persistent ? (unsigned)shape->msaBlocks : (unsigned)b.count;
+    if (blocks == 0) return cudaSuccess;
+    m.kernel<<<blocks, warps * 32, smem, s>>>(st, p, b, b.rawCount, (st.lmax + 31) / 32 * 32);
     return cudaGetLastError();
 }
 

@@ -53,6 +53,10 @@ __device__ __forceinline__ void cp_async16(uint32_t* dst, const uint32_t* src) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
+// A value that is the same in all lanes of the warp, made known as such to the
+// compiler: branches on it need no preparation for a warp that has split.
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __reduce_max_sync(0xffffffffu, v); }
+
 // first anchor of the batch and anchor id of output row 0: kernel parameters,
 // or device memory in graph replays
 __device__ __forceinline__ uint64_t batch_first(const BatchArg& b) { return b.cursor ? b.cursor[0] : b.first; }

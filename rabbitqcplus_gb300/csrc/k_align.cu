@@ -310,8 +310,12 @@ __global__ void __launch_bounds__(kAlignThreads, align_blocks_per_sm(W))
 align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ rawOff, int varies) {
     using Sm = AlignBlock<W>;
     extern __shared__ __align__(1024) unsigned char smraw[];
-    Sm& sm = *reinterpret_cast<Sm*>(smraw);
-    const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // The block's shared memory by an address kept in a register: left to itself the
+    // compiler builds it anew at every access.
+    uint32_t smAt = smem_u32(smraw);
+    asm volatile("" : "+r"(smAt));
+    Sm& sm = *static_cast<Sm*>(__cvta_shared_to_generic(smAt));
+    const int tid = (int)threadIdx.x, lane = tid & 31, warp = (int)warp_uniform((uint32_t)tid >> 5);
     const float rate = p.maxErrorRate, slope = fmaxf(1.0f - 2.0f * rate, 0.0f);
     unsigned int next = 0;  // thread 64: the unit after the one in work
     if (tid == 64) next = atomicAdd(b.unitCursor, 1u);
@@ -429,11 +433,12 @@ align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ raw
     uint32_t phase = 0;
     bool failed = false;
     for (int u = 0;; u ^= 1) {
-        const int n = sm.unit[u].n, La = sm.unit[u].len;  // n == 0: the first unit is still to be loaded
+        // n == 0: the first unit is still to be loaded
+        const int n = (int)warp_uniform((uint32_t)sm.unit[u].n), La = (int)warp_uniform((uint32_t)sm.unit[u].len);
         if (tid == 64 && n) next = atomicAdd(b.unitCursor, 1u);  // arrives while this unit is in work
         const int minov = max(p.minOverlap, (int)__fmul_rn((float)La, p.minOverlapRatio));
         const uint16_t* lens = sm.lens[u];
-        const int lcMin = lens[0], lcMax = lens[max(n - 1, 0)];
+        const int lcMin = (int)warp_uniform(lens[0]), lcMax = (int)warp_uniform(lens[max(n - 1, 0)]);
         const int right = max(La - minov + 1, 0);  // the reference's shifts 0 .. right - 1, then the left ones
         // the forward candidates' shifts (a read shorter than minov overlaps by its whole length,
         // and then the other orientation's shifts reach further)
@@ -533,7 +538,7 @@ align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ raw
                 tc_fence_before();
             }
             __syncthreads();
-            const int entries = (int)sm.queued;
+            const int entries = (int)warp_uniform(sm.queued);
             if (job == jobs || entries > kAlignQueue - kAlignThreads) {  // done, or no room for a tile's worst case
                 count(entries);
                 __syncthreads();

@@ -164,10 +164,6 @@ struct MsaSlice {
 __device__ __forceinline__ uint32_t bits_from(int n) { return __funnelshift_rc(0xffffffffu, 0u, (uint32_t)max(n, 0)); }
 __device__ __forceinline__ uint32_t bits_to(int n) { return ~bits_from(n); }
 
-// A value that is the same in all lanes of the warp, made known as such to the
-// compiler: branches on it need no preparation for a warp that has split.
-__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __reduce_max_sync(kFull, v); }
-
 // x[k] and its assignment for a k known at run time only, x in registers
 template <int K, typename T>
 __device__ __forceinline__ T pick(const T (&x)[K], int k) {

@@ -217,17 +217,23 @@ __device__ __forceinline__ void tc_fill8(uint32_t taddr, float v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1};\n" ::"r"(taddr), "r"(r)
                  : "memory");
 }
-// and into its first ncol columns (16, 32, 48 or 64), from one register vector
-__device__ __forceinline__ void tc_fill(uint32_t taddr, float v, int ncol) {
-    const uint32_t r = __float_as_uint(v);
-    asm volatile(
-        "{\n\t.reg .pred p, q, s;\n\tsetp.gt.s32 p, %2, 16;\n\tsetp.gt.s32 q, %2, 32;\n\tsetp.gt.s32 s, %2, 48;\n\t"
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};\n\t"
-        "@p tcgen05.st.sync.aligned.32x32b.x16.b32 [%0 + 16], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};\n\t"
-        "@q tcgen05.st.sync.aligned.32x32b.x16.b32 [%0 + 32], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};\n\t"
-        "@s tcgen05.st.sync.aligned.32x32b.x16.b32 [%0 + 48], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};\n\t}\n"
-        ::"r"(taddr), "r"(r), "r"(ncol)
-        : "memory");
+// and into its first ncol columns (16, 32, 48 or 64).  zero: 0, unknown to the
+// compiler, which would otherwise fill a register vector for every store (64 moves
+// instead of 16).
+__device__ __forceinline__ void tc_fill(uint32_t taddr, float v, int ncol, uint32_t zero) {
+    uint32_t r[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) r[i] = __float_as_uint(v) + (uint32_t)i * zero;
+#pragma unroll
+    for (int c = 0; c < 64; c += 16) {
+        if (c >= ncol) break;
+        asm volatile(
+            "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(
+                taddr + (uint32_t)c),
+            "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+            "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+            : "memory");
+    }
 }
 
 struct AlignUnit {
@@ -298,12 +304,12 @@ constexpr int align_blocks_per_sm(int w) { return w <= 5 ? 8 : w <= 8 ? 5 : w <=
 // part of a unit.
 //
 // Measured, alignment and filter of 2M anchors of 150 bp (105M candidates, 10 Mbp
-// genome with repeats): 23.6 ms; the scan of every shift by XOR and popcount that
+// genome with repeats): 22.5 ms; the scan of every shift by XOR and popcount that
 // this replaces, 33.2 ms with its filter kernel (integer pipe 85% busy, popcounts at
-// a quarter of its rate).  60k anchors of 300 bp: 1.7 ms against 16.1.  Issue is 70%
+// a quarter of its rate).  60k anchors of 300 bp: 1.6 ms against 16.1.  Issue is 68%
 // busy, the tensor pipe 18%: what is left is bound by the instructions around the
-// products (about 8,500 warp instructions a unit, a third of them signs and start
-// values).  The same test with mma.sync took 61 ms: e4m3 operands are unpacked to
+// products (about 7,800 warp instructions a unit, a quarter of them signs and start
+// values) and by waiting for the products in between.  The same test with mma.sync took 61 ms: e4m3 operands are unpacked to
 // FP16 there, at a quarter of this rate.
 template <int W>
 __global__ void __launch_bounds__(kAlignThreads, align_blocks_per_sm(W))
@@ -338,6 +344,7 @@ align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ raw
     tc_fence_after();
     const uint32_t tmem = sm.tmem, acc = tmem + ((uint32_t)(warp * 32) << 16);  // acc: this thread's TMEM lane
     const uint32_t mb = smem_u32(&sm.mbar);
+    const uint32_t zero = (uint32_t)st.lmax >> 20;
     const uint64_t adesc = smem_desc(smem_u32(sm.toeplitz), 16, 16 * Sm::kCopy);
     const uint64_t bdesc = smem_desc(smem_u32(sm.cands), 128, 256 * W);
     const int rowShift = 16 * (tid & 7) + (tid >> 3);  // this thread's row of a tile
@@ -469,7 +476,7 @@ align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ raw
                 return 0.25f - slope * (float)max(ov, min(low, lc));
             };
             if (!varies) {
-                tc_fill(acc, value(lcMin), ncol);
+                tc_fill(acc, value(lcMin), ncol, zero);
             } else {
 #pragma unroll 1
                 for (int c = 0; c < ncol; c += 8) tc_fill8(acc + (uint32_t)c, c < n ? value(lens[c]) : -1e6f);

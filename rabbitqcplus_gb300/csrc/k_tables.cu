@@ -189,7 +189,14 @@ __global__ void range_batch_max_kernel(const unsigned long long* __restrict__ of
     atomicMax(&maxima[0], off[b1] - off[b0]);
 }
 
+// Threads per block.  An anchor's buckets (most hold 10 to 20 ids) keep 128 busy.
+// Those of the large-table pass have more ids, and shared memory leaves room for four
+// blocks per SM: with 512 threads it takes 40 us per 65,536 anchors of a genome with
+// repeats, with 128 it took 87.  The pass over the others takes 210 us, 216 with an
+// exchange for every id: two thirds of the issue slots, a fifth of them idle lanes of
+// short buckets.
 constexpr int kGatherThreads = 128;
+constexpr int kGatherBigThreads = 512;
 
 // One block per anchor: the union of the anchor's buckets, ascending, without
 // the anchor itself (and without ambiguous reads if requested).  The raw ids
@@ -221,6 +228,7 @@ __device__ __forceinline__ uint2 gather_range(const BatchArg& b, const uint32_t*
 // Groups of 16 threads take the maps in turn (a bucket's first 16 ids with one
 // load per thread, all maps' loads issued before the inserts); an id joins the
 // unique list when its first copy enters the hash set.
+template <int Threads>
 __device__ void gather_one(const StoreArg& st, const TablesArg& tb, const Params& p, const BatchArg& b, int a,
                            uint64_t aid, uint32_t off, uint32_t raw, uint32_t* table, int tableSize, uint2* rng,
                            uint32_t* nUniqueS) {
@@ -240,15 +248,19 @@ __device__ void gather_one(const StoreArg& st, const TablesArg& tb, const Params
             rng[tid] = b.qrange[(uint64_t)a * tb.nmaps + tid];
         }
     }
-    for (uint32_t i = tid; i < T; i += kGatherThreads) table[i] = 0xffffffffu;
+    for (uint32_t i = tid; i < T / 4; i += Threads)
+        reinterpret_cast<uint4*>(table)[i] = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
     if (tid == 0) nUnique = 0;
-    constexpr int kGroup = 16, kGroups = kGatherThreads / kGroup, kMapsPer = (kMaxMaps + kGroups - 1) / kGroups;
+    constexpr int kGroup = 16, kGroups = Threads / kGroup, kMapsPer = (kMaxMaps + kGroups - 1) / kGroups;
     const int g = tid / kGroup, gl = tid % kGroup;  // this thread's maps: g + k kGroups
     __syncthreads();
     auto insert = [&](uint32_t v) {
         uint32_t h = (v * 0x9E3779B1u) & mask;
         for (uint32_t probe = 0; probe < T; probe++) {
-            const uint32_t old = atomicCAS(&table[h], 0xffffffffu, v);
+            // most ids are copies: a load finds them, the exchange is for free slots
+            uint32_t old = *(volatile uint32_t*)&table[h];
+            if (old == v) return;
+            if (old == 0xffffffffu) old = atomicCAS(&table[h], 0xffffffffu, v);
             if (old == 0xffffffffu) {  // the first copy of v
                 if ((uint64_t)v != aid && !(p.excludeAmbiguous && st.ambig[v])) list[atomicAdd(&nUnique, 1u)] = v;
                 return;
@@ -304,7 +316,7 @@ __device__ void gather_one(const StoreArg& st, const TablesArg& tb, const Params
         }
     } else if (U <= 512) {
         // rank of each id among the unique ids = its position in ascending order
-        for (uint32_t i = tid; i < U; i += kGatherThreads) {
+        for (uint32_t i = tid; i < U; i += Threads) {
             const uint32_t v = list[i];
             uint32_t rank = 0;
             for (uint32_t k = 0; k < U; k++) rank += list[k] < v;
@@ -313,11 +325,11 @@ __device__ void gather_one(const StoreArg& st, const TablesArg& tb, const Params
     } else {
         uint32_t S = 1;
         while (S < U) S <<= 1;  // S <= T: the hash table's space becomes the sort buffer
-        for (uint32_t i = tid; i < S; i += kGatherThreads) table[i] = i < U ? list[i] : 0xffffffffu;
+        for (uint32_t i = tid; i < S; i += Threads) table[i] = i < U ? list[i] : 0xffffffffu;
         __syncthreads();
         for (uint32_t k = 2; k <= S; k <<= 1) {
             for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-                for (uint32_t i = tid; i < S; i += kGatherThreads) {
+                for (uint32_t i = tid; i < S; i += Threads) {
                     const uint32_t ixj = i ^ j;
                     if (ixj > i) {
                         const uint32_t x = table[i], y = table[ixj];
@@ -331,7 +343,7 @@ __device__ void gather_one(const StoreArg& st, const TablesArg& tb, const Params
                 __syncthreads();
             }
         }
-        for (uint32_t i = tid; i < U; i += kGatherThreads) out[i] = table[i];
+        for (uint32_t i = tid; i < U; i += Threads) out[i] = table[i];
     }
     if (tid == 0) {
         b.ncand[a] = U;
@@ -353,7 +365,7 @@ __global__ void __launch_bounds__(kGatherThreads, 16) gather_unique_kernel(Store
                                                                        BatchArg b, const uint32_t* __restrict__ rawOff,
                                                                        int tableSize, uint32_t smallCap,
                                                                        uint32_t* bigList, unsigned int* bigCount) {
-    extern __shared__ uint32_t table[];  // [tableSize], then list[tableSize / 2]
+    extern __shared__ __align__(16) uint32_t table[];  // [tableSize], then list[tableSize / 2]
     __shared__ uint2 rng[kMaxMaps];
     __shared__ uint32_t nUnique;
     const int a = blockIdx.x;
@@ -368,15 +380,15 @@ __global__ void __launch_bounds__(kGatherThreads, 16) gather_unique_kernel(Store
         if (threadIdx.x == 0) bigList[atomicAdd(bigCount, 1u)] = (uint32_t)a;
         return;
     }
-    gather_one(st, tb, p, b, a, first + (uint64_t)a, r.x, r.y, table, tableSize, rng, &nUnique);
+    gather_one<kGatherThreads>(st, tb, p, b, a, first + (uint64_t)a, r.x, r.y, table, tableSize, rng, &nUnique);
 }
 
 // Persistent blocks over the deferred anchors of gather_unique_kernel.
-__global__ void __launch_bounds__(kGatherThreads) gather_big_kernel(StoreArg st, TablesArg tb, Params p, BatchArg b,
+__global__ void __launch_bounds__(kGatherBigThreads) gather_big_kernel(StoreArg st, TablesArg tb, Params p, BatchArg b,
                                                                     const uint32_t* __restrict__ rawOff,
                                                                     int tableSize, const uint32_t* bigList,
                                                                     const unsigned int* bigCount) {
-    extern __shared__ uint32_t table[];
+    extern __shared__ __align__(16) uint32_t table[];
     __shared__ uint2 rng[kMaxMaps];
     __shared__ uint32_t nUnique;
     const uint64_t first = batch_first(b);
@@ -384,7 +396,7 @@ __global__ void __launch_bounds__(kGatherThreads) gather_big_kernel(StoreArg st,
     for (unsigned int i = blockIdx.x; i < n; i += gridDim.x) {
         const int a = (int)bigList[i];
         const uint2 r = gather_range(b, rawOff, a, first, false);
-        gather_one(st, tb, p, b, a, first + (uint64_t)a, r.x, r.y, table, tableSize, rng, &nUnique);
+        gather_one<kGatherBigThreads>(st, tb, p, b, a, first + (uint64_t)a, r.x, r.y, table, tableSize, rng, &nUnique);
         __syncthreads();  // the next anchor reuses the shared arrays
     }
 }
@@ -562,7 +574,7 @@ cudaError_t launch_gather_unique(StoreArg st, TablesArg tb, Params p, BatchArg b
     int dev = 0, sms = 1;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const unsigned blocks = (unsigned)std::min<int>(b.count, std::max(sms, 1) * kGatherBigBlocksPerSm);
-    gather_big_kernel<<<blocks, kGatherThreads, smemB, s>>>(st, tb, p, b, b.rawCount, Tb, bigList, bigCount);
+    gather_big_kernel<<<blocks, kGatherBigThreads, smemB, s>>>(st, tb, p, b, b.rawCount, Tb, bigList, bigCount);
     return cudaGetLastError();
 }
 

@@ -69,16 +69,19 @@ from rabbitqcplus_gb300 import capi, learned, shard, sim  # noqa: E402
 METRIC = "corrected reads/s on 1 GB300: plain vs batched+learned, at equal TP/FP vs truth"
 UNIT = "reads/s"
 WINDOW = 4_194_304  # anchors per step
-# DRAM bytes (read + write) of align_lane_kernel per candidate, its warp
-# instructions per candidate and its ALU pipe activity, measured by ncu on one
-# 65536-anchor launch of the 100M-read workload's shape at 20 Mbp
-# (profiles/align_lane_kernel_c4_shape_20mbp.md: 738.1 MB and 7.67810e8 warp
-# instructions for the launch's 3.3555M candidates, ALU pipe 84.9% active).
-# On the 2M-read workload with repeats the DRAM bytes per candidate are far
-# fewer (candidates shared by the anchors of a batch hit in L2 there).
-ALIGN_DRAM_BYTES_PER_CANDIDATE = 738.1e6 / 3.3555e6
-ALIGN_WARP_INST_PER_CANDIDATE = 7.67810e8 / 3.3555e6
-ALIGN_ALU_PIPE_ACTIVE = 0.849
+# DRAM bytes (read + write) of align_kernel per candidate, its warp instructions
+# per candidate and the pipes' activity, measured by ncu on one 65536-anchor
+# launch of the 100M-read workload's shape at 20 Mbp
+# (profiles/top_kernels_c4_shape_20mbp.md: 474.4 MB and 5.58698e8 warp
+# instructions for the launch's 3.3555M candidates, issue 64.4%, ALU pipe 54.6%,
+# tensor pipe 18.2% active).  On the 2M-read workload with repeats the DRAM
+# bytes per candidate are far fewer (candidates shared by the anchors of a
+# batch hit in L2 there).
+ALIGN_DRAM_BYTES_PER_CANDIDATE = 474.4e6 / 3.3555e6
+ALIGN_WARP_INST_PER_CANDIDATE = 5.58698e8 / 3.3555e6
+ALIGN_ISSUE_ACTIVE = 0.644
+ALIGN_ALU_PIPE_ACTIVE = 0.546
+ALIGN_TENSOR_PIPE_ACTIVE = 0.182
 # STEP2 speed of the oracle (the port) over the reference's own build, both on
 # 8 threads of an Intel Xeon @ 2.70 GHz, 2M-read 150 bp workload with repeats,
 # outputs byte-identical (python oracle/port_speed.py --threads 8): the port
@@ -458,14 +461,15 @@ def main():
         cands = p1["unique_candidates"] - p0["unique_candidates"]
         msa_c = p1["msa_candidates"] - p0["msa_candidates"]
         raw = p1["raw_candidate_ids"] - p0["raw_candidate_ids"]
-        wp = (lmax + 31) // 32 + 1
+        words = next(w for w in (3, 4, 5, 8, 10, 16, 32) if 32 * w >= lmax)
+        wp = (words + 2) // 2 * 2  # words per bit plane of a read
         pitch = (lmax + 15) // 16
         if dom == "align":
-            kbytes = cands * (4 + 2 + 16 * wp + 8) + n_anchors * (8 * wp + 10)
+            kbytes = cands * (4 + 2 + 8 * wp) + msa_c * 13 + n_anchors * (8 * wp + 10)
             launches = p1["align_launches"] - p0["align_launches"]
-            kname = "align_lane_kernel"
+            kname = "align_kernel"
         elif dom == "msa":
-            kbytes = msa_c * (13 + 4 * pitch) + n_anchors * (4 * pitch + 2 + lmax + 1)
+            kbytes = msa_c * (13 + 8 * wp) + n_anchors * (8 * wp + 2 + lmax + 1)
             launches = p1["msa_launches"] - p0["msa_launches"]
             kname = "msa_warp_kernel"
         else:
@@ -488,10 +492,10 @@ def main():
                 "algorithmic_bytes_per_anchor": path_bytes / max(n_anchors, 1),
                 "kernel_bytes_per_launch": kbytes / launches, "avg_launch_ms": dur * 1e3,
                 "stage_seconds_per_step": {k: v / max(steps, 1) for k, v in stages.items()},
-                "note": "integer-issue bound, see `int`; the HBM fraction is low by construction.  traffic = "
-                        "measured DRAM bytes per candidate (ncu) x candidates per launch: the kernel reads each "
-                        "candidate's precomputed forward and reverse-complement hi/lo planes (96 B, in 32 B sectors) "
-                        "where the algorithmic count takes its 40 B 2-bit row"}
+                "note": "bound by instruction issue and the waits between a unit's products, see `int`; the HBM "
+                        "fraction is low by construction.  traffic = measured DRAM bytes per candidate (ncu) x "
+                        "candidates per launch: the kernel reads each candidate's hi/lo planes (48 B at 150 bp, in "
+                        "32 B sectors) where the algorithmic count takes its 40 B 2-bit row"}
         if dom == "align":
             # warp instructions per candidate (ncu, committed profile) x the launch's candidates,
             # over the launch's CUDA-event time, against 152 SMs x 4 schedulers x 1 instruction per
@@ -502,9 +506,10 @@ def main():
             roof["int"] = {"bound": "int-issue", "achieved": inst / dur / 1e9, "peak": peak_i / 1e9,
                            "unit": "G warp-instructions/s", "frac": inst / dur / peak_i, "sm_mhz": mhz,
                            "warp_instructions_per_candidate": ALIGN_WARP_INST_PER_CANDIDATE,
-                           "alu_pipe_active_ncu": ALIGN_ALU_PIPE_ACTIVE,
+                           "issue_active_ncu": ALIGN_ISSUE_ACTIVE, "alu_pipe_active_ncu": ALIGN_ALU_PIPE_ACTIVE,
+                           "tensor_pipe_active_ncu": ALIGN_TENSOR_PIPE_ACTIVE,
                            "source": "smsp__inst_executed.sum per candidate from ncu "
-                                     "(profiles/align_lane_kernel_c4_shape_20mbp.md) x candidates of an average launch"}
+                                     "(profiles/top_kernels_c4_shape_20mbp.md) x candidates of an average launch"}
         return roof
 
     clk = ClockSampler(local, paused=True)

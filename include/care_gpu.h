@@ -158,7 +158,7 @@ typedef struct cg_stats {
     uint64_t kernel_launches;         /* kernels this context launched, accumulated */
     uint64_t align_launches;          /* launches of the alignment/filter kernel */
     uint64_t msa_launches;            /* launches of the MSA/correction kernel */
-    double seconds_filter;            /* device time in the mismatch-ratio filter kernel, accumulated */
+    double seconds_filter;            /* 0: the mismatch-ratio filter is part of the alignment kernel */
     /* batched driver: the shape in use and the time its tuning took */
     int32_t batch_anchors;
     int32_t align_blocks;
@@ -244,6 +244,8 @@ int cg_build_tables(cg_ctx* ctx);
  * CG_RESULT_CORRECTED is set, out_sequences[j * out_pitch .. + length) gets the
  * corrected bases as 'A','C','G','T' (reference: TempCorrectedSequence::sequence).
  * In paired mode first_read and num_anchors must be even.
+ * CG_ERR_TIMEOUT: alignment (or classifier) blocks gave up a bounded wait for
+ * their tensor-core products; their anchors are not corrected.
  */
 int cg_correct(cg_ctx* ctx, uint64_t first_read, uint64_t num_anchors,
                uint8_t* out_flags, char* out_sequences, size_t out_pitch);

@@ -890,8 +890,8 @@ int run_plain(cg_ctx* c, uint64_t first, uint64_t num, int B, uint8_t* flags, ch
 // ---------------------------------------------------------------- batched driver
 //
 // One CUDA graph per batch pipeline, captured once per shape and replayed for
-// every batch: the candidate kernel (bucket lookup, gather, unique), the
-// candidate numbering scan, the persistent alignment kernel, the filter, the
+// every batch: the candidate kernels (bucket lookup, gather, unique; they list
+// the alignment's units), the persistent alignment and filter kernel, the
 // persistent MSA/correction kernel and a one-thread kernel that advances the
 // pipeline's device cursor to its next batch.  Nothing in a replay depends on
 // a host value: the batch's first anchor is read from the cursor, its raw id

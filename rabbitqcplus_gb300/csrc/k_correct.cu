@@ -603,7 +603,7 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
             maxc = max(maxc, cov);
         }
         if (last) break;
-        last = build = true;  // unless this round removes rows
+        last = build = true;  // unless rows are removed below
         if (iter == 5 || nActive == 0) {
             if (exact) break;
             continue;

@@ -891,29 +891,32 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
     // Learned decision: record every column whose consensus differs from the
     // anchor's base, with its features; the classifier then replaces the
     // decision written above (the fallback) where it is confident.
+    // The columns are listed first, in order, so that a lane takes one each.
+    uint32_t differ = 0;  // bit k: column 32 k + lane
+#pragma unroll
+    for (int k = 0; k < K; k++)
+        if (32 * k + lane < La && ((consBits ^ anchorBits) >> (2 * k) & 3u) != 0) differ |= 1u << k;
     int nd = 0;
-#pragma unroll 1
-    for (int c = lane; c < La; c += 32) nd += col_info(wc, lp, c).cons != "ACGT"[get2bit(aenc, c)];
-    nd = __reduce_add_sync(kFull, nd);
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const unsigned m = __ballot_sync(kFull, (differ >> k) & 1u);
+        if ((differ >> k) & 1u) list[nd + __popc(m & ((1u << lane) - 1u))] = (uint32_t)(32 * k + lane);
+        nd += __popc(m);
+    }
+    if (nd == 0) return;
+    unsigned slot0 = 0;
+    if (lane == 0) slot0 = atomicAdd(b.colCount, (unsigned)nd);
+    slot0 = __shfl_sync(kFull, slot0, 0);
+    __syncwarp();
     const float ec = p.estimatedCoverage;
     const float invLa = __fdiv_rn(1.0f, (float)La);
 #pragma unroll 1
-    for (int c0 = 0; c0 < La; c0 += 32) {  // warp-uniform trip count
-        const int c = c0 + lane;
-        bool rec = false;
-        ColInfo ci{};
-        uint32_t ab = 0;
-        if (c < La) {
-            ab = get2bit(aenc, c);
-            ci = col_info(wc, lp, c);
-            rec = ci.cons != "ACGT"[ab];
-        }
-        const unsigned m = __ballot_sync(kFull, rec);
-        if (!m) continue;
-        unsigned slot = 0;
-        if (lane == 0) slot = atomicAdd(b.colCount, (unsigned)__popc(m));
-        slot = __shfl_sync(kFull, slot, 0) + (unsigned)__popc(m & ((1u << lane) - 1u));
-        if (!rec || slot >= b.colCap) continue;
+    for (int i = lane; i < nd; i += 32) {
+        const unsigned slot = slot0 + (unsigned)i;
+        if (slot >= b.colCap) break;
+        const int c = (int)list[i];
+        const uint32_t ab = get2bit(aenc, c);
+        const ColInfo ci = col_info(wc, lp, c);
         const int cb = base_index(ci.cons);
         float n4[4], w4[4];
 #pragma unroll

@@ -131,9 +131,9 @@ __device__ __forceinline__ ColInfo col_info(const uint2* wc, int cp, int c) {
 // that the anchor errs there.  A column's sum of a base thus receives the
 // reference's additions in the reference's order (anchor, then the kept candidates
 // in list order); sums of different bases are independent.
-// Measured, MSA stage: 2M anchors of 150 bp with repeats 13.7 ms (row by row in
+// Measured, MSA stage: 2M anchors of 150 bp with repeats 12.9 ms (row by row in
 // shared memory 17.2 ms: 116 instructions per row); 60,000 anchors of 300 bp
-// 0.71 ms, 30,000 of 640 bp 1.64 ms, 20,000 of 1000 bp 4.6 ms (a block per anchor,
+// 0.70 ms, 30,000 of 640 bp 1.60 ms, 20,000 of 1000 bp 4.6 ms (a block per anchor,
 // which reads longer than 256 bp used to take, 2.9, 3.1 and 4.2 ms).  It issues in
 // 6 of 10 cycles: a warp's steps depend on one another, and registers and the sums
 // in shared memory leave room for 26 warps per SM (150 bp).
@@ -982,10 +982,14 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
 // `warps` warps per block, each on its own anchors.  Plain form: anchor
 // blockIdx.x * warps + warp.  Persistent form (b.work set): warps take the
 // next anchor from the counter b.work[0] until the batch is done.
-// At least as many registers as the K-word arrays need; shared memory bounds the
-// resident warps from K = 8 on.
+// Registers: as many as the K-word arrays need without lowering the number of
+// resident warps, which shared memory bounds: 27 per SM at K = 5, which 72 registers
+// allow (MSA stage 12.9 ms for 2M anchors; 13.7 with 64, which spill, 13.8 with 88),
+// 16 at K = 8 (200,000 anchors of 250 bp 1.67 ms with 112, 1.94 with 80), 9 at K = 16
+// (40,000 of 500 bp 1.24 ms with 224, 1.76 with 128).  256 threads, the most a block
+// has, fit the register file in each case.
 template <bool QUAL, int K>
-__global__ void __launch_bounds__(256, K > 16 ? 1 : K > 8 ? 2 : QUAL || K > 5 ? 3 : 4)
+__global__ void __maxnreg__(K > 16 ? 255 : K > 10 ? 224 : K > 8 ? 144 : K > 5 ? 112 : 72)
     msa_warp_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ rawOff, int lp) {
     extern __shared__ __align__(16) unsigned char sm[];
     const int warp = (int)(threadIdx.x >> 5), warps = (int)(blockDim.x >> 5);

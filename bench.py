@@ -461,7 +461,7 @@ def main():
         cands = p1["unique_candidates"] - p0["unique_candidates"]
         msa_c = p1["msa_candidates"] - p0["msa_candidates"]
         raw = p1["raw_candidate_ids"] - p0["raw_candidate_ids"]
-        words = next(w for w in (3, 4, 5, 8, 10, 16, 32) if 32 * w >= lmax)
+        words = next(w for w in (3, 4, 5, 8, 10, 16, 20, 32) if 32 * w >= lmax)
         wp = (words + 2) // 2 * 2  # words per bit plane of a read
         pitch = (lmax + 15) // 16
         if dom == "align":

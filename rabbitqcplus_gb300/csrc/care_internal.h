@@ -37,7 +37,8 @@ constexpr int kLearnedFeatures = 32;  // features of one MSA column for the lear
 // (the columns of its products).
 constexpr int align_words(int lmax) {
     const int need = (lmax + 31) / 32;
-    return need <= 3 ? 3 : need <= 4 ? 4 : need <= 5 ? 5 : need <= 8 ? 8 : need <= 10 ? 10 : need <= 16 ? 16 : 32;
+    return need <= 3 ? 3 : need <= 4 ? 4 : need <= 5 ? 5 : need <= 8 ? 8 : need <= 10 ? 10 : need <= 16 ? 16
+           : need <= 20 ? 20 : 32;
 }
 constexpr int align_plane_words(int w) { return (w + 2) / 2 * 2; }
 constexpr int kAlignUnit = 64;

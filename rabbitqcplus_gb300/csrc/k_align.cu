@@ -290,9 +290,11 @@ constexpr int align_blocks_per_sm(int w) { return w <= 5 ? 8 : w <= 8 ? 6 : w <=
 // values moved by r positions, and the 16 copies are the 8-row groups.  A tile is
 // 16 (2 W + 15) windows of 16 values for two tiles, each expanded once from the
 // bit plane.  The accumulators start at minus the smallest sum that a shift under its
-// mismatch limit can have -- at most (1 - 2 maxErrorRate) * overlap -- so a shift
-// passes where the sign bit is clear, and each lane shifts its row's signs into a
-// word per 32 columns, one instruction per element.
+// mismatch limit can have -- (1 - 2 maxErrorRate) * overlap -- so a shift passes
+// where the sign bit is clear, and each lane shifts its row's signs into a word per
+// 32 columns, one instruction per element.  With a limit above half the overlap that
+// sum is negative and the test could rule out next to nothing: every shift passes to
+// the exact count.
 //
 // With several read lengths the columns are in order of length, and the start
 // value of a group of 8 columns is that of its shortest candidate (lower for
@@ -326,6 +328,7 @@ align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ raw
     Sm& sm = *static_cast<Sm*>(__cvta_shared_to_generic(smAt));
     const int tid = (int)threadIdx.x, lane = tid & 31, warp = (int)warp_uniform((uint32_t)tid >> 5);
     const float rate = p.maxErrorRate, slope = fmaxf(1.0f - 2.0f * rate, 0.0f);
+    const bool allPass = rate > 0.5f;
     unsigned int next = 0;  // thread 64: the unit after the one in work
     if (tid == 64) next = atomicAdd(b.unitCursor, 1u);
     if (tid == 0) {
@@ -472,11 +475,12 @@ align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ raw
             }
         };
         // the accumulators' start values for this thread's row, shift sp
+        const float lift = allPass ? 0.25f + (float)La : 0.25f;  // no sum is below -La
         auto start = [&](int sp) {
             const int low = min(minov, La);
             auto value = [&](int lc) {
                 const int ov = sp >= 0 ? min(La - sp, lc) : min(La, lc + sp);
-                return 0.25f - slope * (float)max(ov, min(low, lc));
+                return lift - slope * (float)max(ov, min(low, lc));
             };
             if (!varies) {
                 tc_fill(acc, value(lcMin), ncol, zero);

@@ -61,3 +61,14 @@ def test_few_anchors(count):
 @pytest.mark.parametrize("lo", [60, 150])
 def test_limits(lo, kw):
     check(lo, 150, **kw)
+
+
+# above one half a shift under its limit can have more hi plane mismatches than matches
+@pytest.mark.parametrize("rate", [0.5, 0.55, 0.7, 0.9, 1.5])
+@pytest.mark.parametrize("lo,hi", [(150, 150), (60, 150), (300, 300)])
+def test_max_error_rate_above_half(lo, hi, rate):
+    check(lo, hi, max_error_rate=rate)
+
+
+def test_max_error_rate_above_half_in_units_of_several_parts():
+    check(60, 150, coverage=180, driver=capi.CG_DRIVER_BATCHED, max_error_rate=0.8)

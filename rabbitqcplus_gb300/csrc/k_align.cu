@@ -449,7 +449,8 @@ align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ raw
         // n == 0: the first unit is still to be loaded
         const int n = (int)warp_uniform((uint32_t)sm.unit[u].n), La = (int)warp_uniform((uint32_t)sm.unit[u].len);
         if (tid == 64 && n) next = atomicAdd(b.unitCursor, 1u);  // arrives while this unit is in work
-        const int minov = max(p.minOverlap, (int)__fmul_rn((float)La, p.minOverlapRatio));
+        // (shifts without overlap have no mismatch limit to stay under: a negative minimum is none)
+        const int minov = max(max(p.minOverlap, (int)__fmul_rn((float)La, p.minOverlapRatio)), 0);
         const uint16_t* lens = sm.lens[u];
         const int lcMin = (int)warp_uniform(lens[0]), lcMax = (int)warp_uniform(lens[max(n - 1, 0)]);
         const int right = max(La - minov + 1, 0);  // the reference's shifts 0 .. right - 1, then the left ones

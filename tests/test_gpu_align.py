@@ -72,3 +72,9 @@ def test_max_error_rate_above_half(lo, hi, rate):
 
 def test_max_error_rate_above_half_in_units_of_several_parts():
     check(60, 150, coverage=180, driver=capi.CG_DRIVER_BATCHED, max_error_rate=0.8)
+
+
+# a shift without overlap is no shift, however far the options let it go
+@pytest.mark.parametrize("min_overlap", [0, -1, -70_000])
+def test_no_smallest_overlap(min_overlap):
+    check(60, 150, min_overlap=min_overlap, min_overlap_ratio=-1000.0)

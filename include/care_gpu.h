@@ -213,6 +213,12 @@ int cg_set_allocation_fault(int64_t after);
  * reference. */
 int cg_set_classifier_wait_limit(int device, int64_t polls);
 
+/* The same for the alignment's waits of this context's calls.  A block that
+ * gives up leaves the anchors of its units uncorrected (flags 0), drains its
+ * products and releases its tensor memory; the other anchors are corrected as
+ * ever, and the call returns CG_ERR_TIMEOUT. */
+int cg_set_alignment_wait_limit(cg_ctx* ctx, int64_t polls);
+
 /* Message of the last failing call on this context (never NULL). */
 const char* cg_last_error(const cg_ctx* ctx);
 

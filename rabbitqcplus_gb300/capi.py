@@ -109,7 +109,8 @@ EXPORTED = ["cg_default_options", "cg_create", "cg_destroy", "cg_last_error", "c
             "cg_get_candidates", "cg_correct_files", "cg_load_forest", "cg_get_candidates_noalloc",
             "cg_classifier_size", "cg_load_classifier", "cg_get_columns", "cg_default_train_options",
             "cg_train_classifier", "cg_classifier_gradients", "cg_classifier_logits", "cg_release_cached_memory",
-            "cg_combine_results", "cg_set_classifier_wait_limit", "cg_set_allocation_fault"]
+            "cg_combine_results", "cg_set_classifier_wait_limit", "cg_set_allocation_fault",
+            "cg_set_alignment_wait_limit"]
 CLASSIFIER_FEATURES = 32
 CLASSIFIER_PARAMS = 6337  # w1 64x32, w2 64x64, w3 64, b1 64, b2 64, b3
 
@@ -173,6 +174,7 @@ def gpu_lib() -> ctypes.CDLL:
         L.cg_release_cached_memory.argtypes = [ctypes.c_int]
         L.cg_set_classifier_wait_limit.argtypes = [ctypes.c_int, ctypes.c_int64]
         L.cg_set_allocation_fault.argtypes = [ctypes.c_int64]
+        L.cg_set_alignment_wait_limit.argtypes = [P, ctypes.c_int64]
         for f in EXPORTED:
             if f not in ("cg_destroy", "cg_default_options", "cg_last_error", "cg_classifier_size",
                          "cg_default_train_options"):
@@ -293,6 +295,10 @@ class CareGpu:
         self._check(self._L.cg_get_candidates_noalloc(self._h, anchor, out.ctypes.data, out.size, ctypes.byref(cnt)),
                     "cg_get_candidates_noalloc")
         return cnt.value
+
+    def set_alignment_wait_limit(self, polls: int):
+        """Polls of the alignment blocks' waits for their products (< 0: the default)."""
+        self._check(self._L.cg_set_alignment_wait_limit(self._h, polls), "cg_set_alignment_wait_limit")
 
     def load_classifier(self, data: bytes):
         buf = np.frombuffer(data, np.uint8)

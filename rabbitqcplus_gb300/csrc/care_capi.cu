@@ -183,7 +183,7 @@ struct GraphSig {
 // One batch pipeline of the batched driver: its buffers, stream and graph.
 struct BatchSet {
     DevBuf rawCount, cand, ncand, paired, aln, fid, fshift, forient, fweight, flen, nfinal, cursor, work, colFeat,
-        colMeta, colCount, order, orderScratch, bigScratch, units;
+        colMeta, colCount, order, orderScratch, bigScratch, units, unitsDone;
     cudaStream_t stream = nullptr;
     cudaEvent_t joined = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -195,7 +195,8 @@ struct BatchSet {
         if (joined) cudaEventDestroy(joined);
         joined = nullptr;
         for (DevBuf* b : {&rawCount, &cand, &ncand, &paired, &aln, &fid, &fshift, &forient, &fweight, &flen, &nfinal,
-                          &cursor, &work, &colFeat, &colMeta, &colCount, &order, &orderScratch, &bigScratch, &units})
+                          &cursor, &work, &colFeat, &colMeta, &colCount, &order, &orderScratch, &bigScratch, &units,
+                          &unitsDone})
             b->release();
         if (stream) cudaStreamDestroy(stream);
         stream = nullptr;
@@ -210,6 +211,7 @@ struct Plan {
 };
 
 constexpr int kMaxSets = 2;
+constexpr uint32_t kDefaultPolls = 1u << 20;  // of a wait for tensor-core products
 
 // One of the plain driver's two batches in flight: the buffers that outlive
 // the batch's kernels (its bucket ranges are looked up while the batch before
@@ -274,7 +276,7 @@ struct cg_ctx {
 
     // batch buffers
     DevBuf cand, ncand, paired, aln, fid, fshift, forient, fweight, flen, nfinal, counters;
-    DevBuf scanTmp, msaOrder, orderScratch, bigScratch, units, lenRange;
+    DevBuf scanTmp, msaOrder, orderScratch, bigScratch, units, unitsDone, lenRange;
     uint32_t* hPinned = nullptr;  // per slot: total raw, max raw
     unsigned long long* hCounters = nullptr;  // pinned copy of the counters (read_counters)
     bool lenVaries = false;       // reads of different lengths
@@ -293,6 +295,7 @@ struct cg_ctx {
     bool haveMlp = false;
     bool collecting = false;  // cg_get_columns: record the columns, do not score them
     float minLogit = 0.0f;    // logit of threshold_anchor
+    uint32_t alignPolls = kDefaultPolls;  // cg_set_alignment_wait_limit
     // alignment and classifier blocks whose tensor-core wait ran out, already reported
     unsigned long long alignTimeoutsSeen = 0, timeoutsSeen = 0;
 
@@ -335,6 +338,11 @@ uint64_t pow2_at_least(uint64_t x) {
     return p;
 }
 
+// polls of a wait as the cg_set_*_wait_limit calls take them
+uint32_t poll_limit(int64_t polls) {
+    return polls < 0 ? kDefaultPolls : (uint32_t)std::min<int64_t>(polls, 0xffffffffll);
+}
+
 // Float constants in the reference's operand order (host, no contraction).
 void make_params(cg_ctx* c) {
     c->paramsVersion++;  // captured batch graphs hold the parameters by value
@@ -363,6 +371,7 @@ void make_params(cg_ctx* c) {
         p.hqMin[pc] = 1.0f - 3.0f * factor;
     }
     p.significantCount = int(int(o.estimated_coverage) * 0.3f);     // msa.cpp:536-540
+    p.alignPolls = c->alignPolls;
     p.useQuality = o.use_quality_scores != 0;
     p.excludeAmbiguous = o.exclude_ambiguous_reads != 0;
     p.paired = o.pair_mode == CG_PAIR_PE;
@@ -658,6 +667,7 @@ BatchArg batch_arg(cg_ctx* c, const PlainSlot& sl, uint64_t first, int count) {
     b.flen = c->flen.as<uint16_t>();
     b.nfinal = c->nfinal.as<uint32_t>();
     b.units = c->units.as<uint2>();
+    b.unitsDone = c->unitsDone.as<uint32_t>();
     b.unitCursor = b.rawCount + count + 2;  // cleared with the raw counts
     b.unitCount = b.rawCount + count + 3;
     b.flags = sl.flags.as<uint8_t>();
@@ -723,6 +733,7 @@ int enqueue_gather(cg_ctx* c, int slot, uint64_t first, int count) {
     CG_CUDA(c, c->nfinal.ensure((size_t)count * sizeof(uint32_t)));
     CG_CUDA(c, c->cand.ensure(cap * sizeof(uint32_t)));
     CG_CUDA(c, c->units.ensure(unit_slots(count, total) * sizeof(uint2)));
+    CG_CUDA(c, c->unitsDone.ensure((size_t)count * sizeof(uint32_t)));
     CG_CUDA(c, c->paired.ensure(cap));
     CG_CUDA(c, c->aln.ensure(cap * sizeof(uint2)));
     CG_CUDA(c, c->fid.ensure(cap * sizeof(uint32_t)));
@@ -917,6 +928,7 @@ BatchArg set_arg(cg_ctx* c, BatchSet& s, int count) {
     b.flen = s.flen.as<uint16_t>();
     b.nfinal = s.nfinal.as<uint32_t>();
     b.units = s.units.as<uint2>();
+    b.unitsDone = s.unitsDone.as<uint32_t>();
     b.flags = c->flagsRange.as<uint8_t>();
     b.out = c->outRange.as<char>();
     b.outPitch = c->lmax;
@@ -939,6 +951,7 @@ int ensure_set(cg_ctx* c, BatchSet& s, int count, uint64_t capRaw) {
     CG_CUDA(c, s.ncand.ensure(n * sizeof(uint32_t)));
     CG_CUDA(c, s.nfinal.ensure(n * sizeof(uint32_t)));
     CG_CUDA(c, s.units.ensure(unit_slots(count, capRaw) * sizeof(uint2)));
+    CG_CUDA(c, s.unitsDone.ensure(n * sizeof(uint32_t)));
     CG_CUDA(c, s.cand.ensure(capRaw * sizeof(uint32_t)));
     CG_CUDA(c, s.paired.ensure(capRaw));
     CG_CUDA(c, s.aln.ensure(capRaw * sizeof(uint2)));
@@ -1007,7 +1020,7 @@ int capture_set(cg_ctx* c, BatchSet& s, int count, unsigned long long stride, co
     g.shape = sh;
     g.tableRaw = tableRaw;
     for (const DevBuf* d : {&s.rawCount, &s.cand, &s.ncand, &s.paired, &s.aln, &s.fid, &s.fshift, &s.forient,
-                            &s.fweight, &s.flen, &s.nfinal, &s.units, &s.cursor, &s.work, &s.colFeat,
+                            &s.fweight, &s.flen, &s.nfinal, &s.units, &s.unitsDone, &s.cursor, &s.work, &s.colFeat,
                             &s.colMeta, &s.colCount, &s.order, &s.orderScratch, &s.bigScratch, &c->mlp, &c->outRange,
                             &c->flagsRange, &c->rangeOff, &c->counters, &c->sig})
         g.ptrs.push_back(d->p);
@@ -1428,10 +1441,16 @@ int cg_set_classifier_wait_limit(int device, int64_t polls) {
         cudaGetLastError();
         return CG_ERR_INVALID_ARGUMENT;
     }
-    const uint32_t p = polls < 0 ? (1u << 20) : (uint32_t)std::min<int64_t>(polls, 0xffffffffll);
-    const cudaError_t e = set_classifier_wait_limit(p);
+    const cudaError_t e = set_classifier_wait_limit(poll_limit(polls));
     cudaSetDevice(cur);
     return e == cudaSuccess ? CG_OK : CG_ERR_CUDA;
+}
+
+int cg_set_alignment_wait_limit(cg_ctx* c, int64_t polls) {
+    if (!c) return CG_ERR_INVALID_ARGUMENT;
+    c->alignPolls = poll_limit(polls);
+    if (c->built) make_params(c);
+    return CG_OK;
 }
 
 void cg_destroy(cg_ctx* c) {
@@ -1442,7 +1461,7 @@ void cg_destroy(cg_ctx* c) {
     for (DevBuf* b : {&c->enc, &c->len, &c->hilo, &c->qual, &c->ambig, &c->sig, &c->cand,
                       &c->ncand, &c->paired, &c->aln, &c->fid, &c->fshift, &c->forient, &c->fweight, &c->flen, &c->nfinal,
                       &c->counters, &c->scanTmp, &c->forestNodes, &c->treeOffsets,
-                      &c->msaOrder, &c->orderScratch, &c->bigScratch, &c->units, &c->lenRange})
+                      &c->msaOrder, &c->orderScratch, &c->bigScratch, &c->units, &c->unitsDone, &c->lenRange})
         b->release();
     for (cg_ctx::Chunk& ch : c->chunks) {
         ch.chars.release();

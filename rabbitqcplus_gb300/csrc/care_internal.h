@@ -93,6 +93,7 @@ struct Params {
     float hqAvg[101];           // 1 - 1*percent/100 for percent 0..100
     float hqMin[101];           // 1 - 3*percent/100
     int significantCount;       // int(int(cov) * 0.3f)
+    uint32_t alignPolls;        // polls of an alignment block's wait for its products
     int useQuality;
     int excludeAmbiguous;
     int paired;
@@ -209,7 +210,7 @@ struct BatchArg {
     uint8_t* forient;       // [totalRaw] 1 fwd, 2 rc
     float* fweight;         // [totalRaw]
     uint16_t* flen;         // [totalRaw] candidate length
-    uint32_t* nfinal;       // [count]
+    uint32_t* nfinal;       // [count] kept candidates; 0 until the anchor's filter has run
     // The alignment's work: units {anchor, part} of up to kAlignUnit candidates
     // (part k holds the anchor's candidates k kAlignUnit ..), appended by the
     // candidate kernel at *unitCount and taken at *unitCursor (both zero at the
@@ -217,6 +218,7 @@ struct BatchArg {
     uint2* units;
     unsigned int* unitCount;
     unsigned int* unitCursor;
+    uint32_t* unitsDone;    // [count] finished units of an anchor of several (zero at the start of a batch)
     uint8_t* flags;         // [count] CG_RESULT_*
     char* out;              // [count][outPitch]
     int outPitch;
@@ -291,7 +293,8 @@ struct Shape {
 };
 
 // Aligns every unit's candidates (b.units, *b.unitCount of them) and filters
-// the anchors (b.nfinal zero before it); varies: reads of several lengths.
+// the anchors (b.nfinal and b.unitsDone zero before it; b.nfinal stays zero
+// where a block gave up waiting for its products); varies: reads of several lengths.
 // Persistent blocks: any number of them does.
 cudaError_t launch_align(StoreArg st, Params p, BatchArg b, bool varies, unsigned blocks, cudaStream_t s);
 // resident 128-thread blocks of it per SM

@@ -146,7 +146,7 @@ __device__ void filter_anchor(const StoreArg& st, const Params& p, const BatchAr
 constexpr int kAlignThreads = 128;         // a thread per TMEM lane
 constexpr uint32_t kAlignTmemCols = kAlignUnit;  // a column per candidate of a unit
 constexpr int kAlignQueue = 256;
-constexpr uint32_t kAlignSpins = 1u << 20;  // mbarrier polls before a wait is declared failed
+constexpr uint32_t kAlignSpins = 1u << 20;  // polls of the wait that drains a failed block's products
 constexpr uint32_t kOnes = 0x38383838u;    // four e4m3 +1 (the sign bit makes -1)
 
 // `keep` most significant bits (any keep: all from 32 up, none from 0 down)
@@ -568,7 +568,7 @@ align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ raw
             }
             if (warp >= 2 && steps < 4) step();
             bool ok = true;
-            if (warp == 0) ok = mbar_wait(mb, phase, kAlignSpins);  // the other warps wait at the barrier
+            if (warp == 0) ok = mbar_wait(mb, phase, p.alignPolls);  // the other warps wait at the barrier
             phase ^= 1u;
             if (__syncthreads_or(!ok)) {
                 failed = true;
@@ -677,9 +677,9 @@ align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ raw
                     atomicAdd(&b.counters[kCounterAligned], (unsigned long long)(mine.w + other.w));
                     atomicAdd(&b.counters[kCounterMsaCands], (unsigned long long)total);
                 }
-            } else if (warp == 0) {  // nfinal counts the anchor's finished units (zero before the launch)
+            } else if (warp == 0) {  // the last of the anchor's units to finish filters it
                 uint32_t done = 0;
-                if (lane == 0) done = atomicAdd(&b.nfinal[un.a], 1u);
+                if (lane == 0) done = atomicAdd(&b.unitsDone[un.a], 1u);
                 done = __shfl_sync(kFull, done, 0);
                 if (done == (un.nc - 1) / (uint32_t)kAlignUnit) {
                     __threadfence();

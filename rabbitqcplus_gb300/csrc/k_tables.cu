@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(kGatherThreads, 16) gather_unique_kernel(Store
     const int a = blockIdx.x;
     const uint64_t first = batch_first(b);
     const uint2 r = gather_range(b, rawOff, a, first, true);
-    if (b.units && threadIdx.x == 0) b.nfinal[a] = 0;  // the alignment counts an anchor's finished units in it
+    if (b.units && threadIdx.x == 0) b.nfinal[a] = b.unitsDone[a] = 0;
     if (r.y == 0) {
         if (threadIdx.x == 0) b.ncand[a] = 0;
         return;

@@ -193,3 +193,40 @@ def test_bad_offsets_are_refused_at_the_first_bad_read():
     flags, _ = g.correct()
     assert int((flags & capi.CG_RESULT_CORRECTED).astype(bool).sum()) > r.n // 4
     g.close()
+
+
+@pytest.mark.parametrize("polls", [0, 1, 3])
+@pytest.mark.parametrize("driver", [capi.CG_DRIVER_PLAIN, capi.CG_DRIVER_BATCHED])
+def test_alignment_timeout_leaves_anchors_uncorrected(driver, polls):
+    """The alignment's waits given a few polls, anchors of one unit and of several: an anchor that lost a unit is
+    uncorrected, the others are corrected as ever, and the context recovers.  With 0 polls every block gives up on
+    its first unit, so no anchor is corrected."""
+    r = sim.SimReads(sim.SimConfig(seed=75, genome_length=6_000, repeat_families=2, repeat_copies=3,
+                                   repeat_min_len=300, repeat_max_len=600, num_reads=6_000, sub_rate_5p=0.004,
+                                   sub_rate_3p=0.03))
+    g = capi.CareGpu(capi.CareOptions.defaults(120.0, driver=driver, batch_anchors=1024, align_blocks=304,
+                                               msa_warps=4, streams=2))
+    g.append_reads(r.sequences, r.offsets)
+    g.build_tables()
+    n, lmax = g.read_info()
+    rc, flags, out = correct_into(g, n, lmax)
+    assert rc == capi.CG_OK
+    st = g.stats()
+    assert st["unique_candidates"] > 64 * n  # most anchors have several units
+    g.set_alignment_wait_limit(polls)
+    rc, tf, to = correct_into(g, n, lmax)
+    g.set_alignment_wait_limit(-1)
+    if polls == 0:
+        assert rc == capi.CG_ERR_TIMEOUT
+        assert "alignment block" in g._L.cg_last_error(g._h).decode()
+        assert not tf.any()
+        assert g.stats()["msa_builds"] == st["msa_builds"]
+    else:
+        assert rc in (capi.CG_OK, capi.CG_ERR_TIMEOUT)
+        assert rc == capi.CG_ERR_TIMEOUT or np.array_equal(tf, flags)
+    for i in np.flatnonzero(tf):
+        assert tf[i] == flags[i] and np.array_equal(to[i, :r.lengths[i]], out[i, :r.lengths[i]]), i
+    rc, f2, o2 = correct_into(g, n, lmax)
+    assert rc == capi.CG_OK
+    same_results(r, (f2, o2), (flags, out))
+    g.close()

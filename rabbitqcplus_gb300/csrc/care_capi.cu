@@ -1133,10 +1133,9 @@ int check_timeouts(cg_ctx* c) {
     const unsigned long long align = c->hCounters[kCounterAlignTimeouts], mlp = c->hCounters[kCounterTimeouts];
     const unsigned long long moreAlign = align - c->alignTimeoutsSeen, moreMlp = mlp - c->timeoutsSeen;
     c->alignTimeoutsSeen = align;
+    c->timeoutsSeen = mlp;
     if (moreAlign)
         return fail(c, CG_ERR_TIMEOUT, "%llu alignment block(s) timed out waiting for the tensor cores", moreAlign);
-    if (c->params.correctionType != CG_CORR_LEARNED || c->collecting) return CG_OK;
-    c->timeoutsSeen = mlp;
     if (moreMlp)
         return fail(c, CG_ERR_TIMEOUT,
                     "%llu classifier block(s) timed out waiting for the tensor cores; their columns kept the "

@@ -230,3 +230,30 @@ def test_alignment_timeout_leaves_anchors_uncorrected(driver, polls):
     assert rc == capi.CG_OK
     same_results(r, (f2, o2), (flags, out))
     g.close()
+
+
+def test_timeouts_of_both_kinds_are_reported_once():
+    """Alignment timeouts that are still to be reported and classifier timeouts of one call: the call after it is
+    good."""
+    r = small_reads(76)
+    g = ctx(r, correction_type=capi.CG_CORR_LEARNED)
+    g.load_classifier(open(learned.DEFAULT_MODEL, "rb").read())
+    n, lmax = g.read_info()
+    rc, lf, lo = correct_into(g, n, lmax)
+    assert rc == capi.CG_OK
+    try:
+        g.set_alignment_wait_limit(0)
+        try:
+            g.columns()
+        except capi.CareError:
+            pass
+        g.set_alignment_wait_limit(-1)
+        capi.set_classifier_wait_limit(0)
+        rc, _, _ = correct_into(g, n, lmax)
+        assert rc == capi.CG_ERR_TIMEOUT
+    finally:
+        capi.set_classifier_wait_limit(-1)
+    rc, f2, o2 = correct_into(g, n, lmax)
+    assert rc == capi.CG_OK
+    same_results(r, (f2, o2), (lf, lo))
+    g.close()

@@ -250,8 +250,9 @@ int cg_build_tables(cg_ctx* ctx);
  * CG_RESULT_CORRECTED is set, out_sequences[j * out_pitch .. + length) gets the
  * corrected bases as 'A','C','G','T' (reference: TempCorrectedSequence::sequence).
  * In paired mode first_read and num_anchors must be even.
- * CG_ERR_TIMEOUT: alignment (or classifier) blocks gave up a bounded wait for
- * their tensor-core products; their anchors are not corrected.
+ * CG_ERR_TIMEOUT: blocks gave up a bounded wait for their tensor-core
+ * products.  The anchors of an alignment block that did are not corrected, the
+ * columns of a classifier block keep the fallback decision.
  */
 int cg_correct(cg_ctx* ctx, uint64_t first_read, uint64_t num_anchors,
                uint8_t* out_flags, char* out_sequences, size_t out_pitch);
@@ -381,7 +382,7 @@ int cg_load_classifier(cg_ctx* ctx, const void* data, size_t size);
  * features[count][32], the anchor id, the position in the anchor and the
  * consensus base of each.  *count = number of columns; at most `capacity` are
  * written (CG_ERR_INVALID_ARGUMENT if there are more).  The order of the
- * columns is unspecified.
+ * columns is unspecified.  CG_ERR_TIMEOUT as cg_correct, for the alignment.
  */
 int cg_get_columns(cg_ctx* ctx, uint64_t first, uint64_t num, float* features, uint64_t* anchors,
                    uint16_t* positions, char* consensus, uint64_t capacity, uint64_t* count);

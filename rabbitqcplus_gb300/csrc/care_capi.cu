@@ -1816,6 +1816,7 @@ int cg_get_columns(cg_ctx* c, uint64_t first, uint64_t num, float* features, uin
     for (uint64_t a = 0; a < num && rc == CG_OK; a += (uint64_t)B) {
         const int cnt = (int)std::min<uint64_t>((uint64_t)B, num - a);
         rc = run_plain(c, first + a, cnt, cnt, hFlags.data(), hOut.data(), (size_t)std::max(c->lmax, 1));
+        if (rc == CG_OK) rc = check_timeouts(c);
         if (rc != CG_OK) break;
         unsigned int k = 0;
         if (cudaMemcpy(&k, c->colCount.p, sizeof(k), cudaMemcpyDeviceToHost) != cudaSuccess) {

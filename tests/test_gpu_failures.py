@@ -257,3 +257,20 @@ def test_timeouts_of_both_kinds_are_reported_once():
     assert rc == capi.CG_OK
     same_results(r, (f2, o2), (lf, lo))
     g.close()
+
+
+def test_columns_report_alignment_timeouts():
+    """cg_get_columns does not pass off an incomplete list as whole; the context gives the whole one afterwards."""
+    r = small_reads(77)
+    g = ctx(r, correction_type=capi.CG_CORR_LEARNED, batch_anchors=4096)
+    want = g.columns()
+    assert len(want[0]) > 0
+    g.set_alignment_wait_limit(0)
+    with pytest.raises(capi.CareError, match="timeout"):
+        g.columns()
+    g.set_alignment_wait_limit(-1)
+    got = g.columns()
+    order = [np.lexsort((c[2], c[1])) for c in (want, got)]
+    for a, b in zip(want, got):
+        assert np.array_equal(a[order[0]], b[order[1]])
+    g.close()

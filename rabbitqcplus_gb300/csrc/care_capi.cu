@@ -18,6 +18,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <shared_mutex>
 #include <tuple>
 #include <new>
 #include <string>
@@ -35,8 +36,9 @@ namespace {
 // Device blocks released by the contexts of this process, kept for reuse
 // (like a caching allocator): a later context of the same shapes allocates
 // without cudaMalloc and frees without cudaFree.  A block is cached only after
-// the device has finished every queued kernel (the release synchronises, as
-// cudaFree would), and the cache is emptied before an allocation fails.
+// the work that uses it has finished (release waits for the device, as cudaFree
+// would; release_after for one stream), and the cache is emptied before an
+// allocation fails.
 // Simulated device out-of-memory (cg_set_allocation_fault): requests left
 // before every request fails; < 0 = off.
 std::atomic<long long> g_allocFault{-1};
@@ -48,6 +50,14 @@ bool simulated_out_of_memory() {
         if (g_allocFault.compare_exchange_weak(v, v - 1)) return false;
     }
     return false;
+}
+
+// Held shared while a stream of this library is captured, exclusively while the
+// device is waited for: waiting for a device fails, and breaks the capture, while
+// one of its streams is being captured, by whatever thread.
+std::shared_mutex& capture_mutex() {
+    static std::shared_mutex* m = new std::shared_mutex();  // as block_cache()
+    return *m;
 }
 
 class BlockCache {
@@ -94,11 +104,15 @@ public:
         return e;
     }
     void release(void* p, size_t bytes) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceSynchronize();
-        std::lock_guard<std::mutex> lock(mu_);
-        free_.emplace(bytes, std::make_pair(dev, p));
+        {
+            std::unique_lock<std::shared_mutex> noCapture(capture_mutex());
+            cudaDeviceSynchronize();
+        }
+        put(p, bytes);
+    }
+    void release_after(void* p, size_t bytes, cudaStream_t s) {
+        cudaStreamSynchronize(s);
+        put(p, bytes);
     }
     // frees the cached blocks of device dev (every device if dev < 0)
     void trim(int dev) {
@@ -118,6 +132,12 @@ public:
     }
 
 private:
+    void put(void* p, size_t bytes) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        std::lock_guard<std::mutex> lock(mu_);
+        free_.emplace(bytes, std::make_pair(dev, p));
+    }
     std::mutex mu_;
     std::multimap<size_t, std::pair<int, void*>> free_;
 };
@@ -889,12 +909,16 @@ int run_plain_batches(cg_ctx* c, uint64_t first, uint64_t num, int B, uint8_t* f
     return CG_OK;
 }
 
+// After an error nothing of the call is left in flight: the caller's buffers may
+// go away.
+void drain(cg_ctx* c) {
+    for (cudaStream_t s : {c->sets[0].stream, c->sets[1].stream, c->queryStream, c->copyStream, c->stream})
+        if (s) cudaStreamSynchronize(s);
+}
+
 int run_plain(cg_ctx* c, uint64_t first, uint64_t num, int B, uint8_t* flags, char* out, size_t pitch) {
     const int rc = run_plain_batches(c, first, num, B, flags, out, pitch);
-    if (rc != CG_OK) {  // nothing of the call is left in flight: the caller's buffers may go away
-        for (cudaStream_t s : {c->queryStream, c->copyStream, c->stream})
-            if (s) cudaStreamSynchronize(s);
-    }
+    if (rc != CG_OK) drain(c);
     return rc;
 }
 
@@ -1028,11 +1052,15 @@ int capture_set(cg_ctx* c, BatchSet& s, int count, unsigned long long stride, co
     if (s.exec && g == s.sig) return CG_OK;
     if (s.exec) cudaGraphExecDestroy(s.exec);
     s.exec = nullptr;
-    CG_CUDA(c, cudaStreamBeginCapture(s.stream, cudaStreamCaptureModeThreadLocal));
     int kernels = 0;
-    const cudaError_t e = enqueue_batch(c, s, count, stride, sh, tableRaw, &kernels);
     cudaGraph_t graph = nullptr;
-    const cudaError_t e2 = cudaStreamEndCapture(s.stream, &graph);
+    cudaError_t e, e2;
+    {
+        CaptureScope capture;
+        CG_CUDA(c, cudaStreamBeginCapture(s.stream, cudaStreamCaptureModeThreadLocal));
+        e = enqueue_batch(c, s, count, stride, sh, tableRaw, &kernels);
+        e2 = cudaStreamEndCapture(s.stream, &graph);
+    }
     if (e != cudaSuccess || e2 != cudaSuccess) {
         if (graph) cudaGraphDestroy(graph);
         cudaGetLastError();
@@ -1298,7 +1326,8 @@ int plan_for(cg_ctx* c, uint64_t first, uint64_t num, Plan* out) {
 // cg_correct with the batched driver: full batches as graph replays, the
 // remainder (fewer anchors than a batch) through the plain driver on the
 // context's own stream, concurrently.
-int correct_batched(cg_ctx* c, uint64_t first, uint64_t num, uint8_t* out_flags, char* out_seq, size_t out_pitch) {
+int correct_batched_range(cg_ctx* c, uint64_t first, uint64_t num, uint8_t* out_flags, char* out_seq,
+                          size_t out_pitch) {
     int rc = ensure_batched_state(c);
     if (rc != CG_OK) return rc;
     Plan pl;
@@ -1348,6 +1377,12 @@ int correct_batched(cg_ctx* c, uint64_t first, uint64_t num, uint8_t* out_flags,
     c->stats.seconds_correct = ms / 1000.0;
     c->stats.num_anchors_processed += num;
     return check_timeouts(c);
+}
+
+int correct_batched(cg_ctx* c, uint64_t first, uint64_t num, uint8_t* out_flags, char* out_seq, size_t out_pitch) {
+    const int rc = correct_batched_range(c, first, num, out_flags, out_seq, out_pitch);
+    if (rc != CG_OK) drain(c);
+    return rc;
 }
 
 }  // namespace
@@ -1988,7 +2023,9 @@ extern "C" int cg_get_candidates_noalloc(cg_ctx* c, uint64_t anchor, uint32_t* o
 namespace cg {
 
 cudaError_t cached_alloc(void** p, size_t n, size_t* got) { return block_cache().alloc(p, n, got); }
-void cached_release(void* p, size_t bytes) { block_cache().release(p, bytes); }
+void cached_release(void* p, size_t bytes, cudaStream_t s) { block_cache().release_after(p, bytes, s); }
+CaptureScope::CaptureScope() { capture_mutex().lock_shared(); }
+CaptureScope::~CaptureScope() { capture_mutex().unlock_shared(); }
 
 int append_device_chunk(cg_ctx* c, CachedMem& chars, CachedMem& offs, CachedMem& qual, uint64_t n, int lmax) {
     if (!c) return CG_ERR_INVALID_ARGUMENT;

@@ -13,28 +13,42 @@
 namespace cg {
 
 // Device memory from the process's block cache (cg_release_cached_memory): at
-// least n bytes, *got of them.  cached_release waits for the device, as cudaFree
-// does, and keeps the block of the current device for a later request.
+// least n bytes, *got of them.  cached_release waits for stream s and keeps the
+// block of the current device for a later request.  It does not wait for the whole
+// device: that fails, and breaks the capture, while another thread (of this
+// library or of the program) captures one of its streams.
 cudaError_t cached_alloc(void** p, size_t n, size_t* got);
-void cached_release(void* p, size_t bytes);
+void cached_release(void* p, size_t bytes, cudaStream_t s);
+
+// Held while a stream is captured: no thread of this library waits for the device
+// meanwhile.
+struct CaptureScope {
+    CaptureScope();
+    ~CaptureScope();
+    CaptureScope(const CaptureScope&) = delete;
+    CaptureScope& operator=(const CaptureScope&) = delete;
+};
 
 // A block of it, given back on scope exit.  Allocated and given back with the
-// same device current.
+// same device current.  Work of other streams than `stream` that uses it has ended
+// by then.
 struct CachedMem {
     void* p = nullptr;
     size_t bytes = 0;
+    cudaStream_t stream = nullptr;
     CachedMem() = default;
     CachedMem(const CachedMem&) = delete;
     CachedMem& operator=(const CachedMem&) = delete;
     ~CachedMem() { free(); }
-    cudaError_t alloc(size_t n) {
+    cudaError_t alloc(size_t n, cudaStream_t s) {
         free();
+        stream = s;
         const cudaError_t e = cached_alloc(&p, n < 16 ? 16 : n, &bytes);
         if (e != cudaSuccess) p = nullptr;
         return e;
     }
     void free() {
-        if (p) cached_release(p, bytes);
+        if (p) cached_release(p, bytes, stream);
         p = nullptr;
     }
     template <class T>

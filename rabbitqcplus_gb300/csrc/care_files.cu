@@ -346,7 +346,7 @@ int correct_fastq_on_device(const cg_options& options, const std::vector<ByteSpa
     const cudaStream_t s = st.s;
     const size_t nf = inputs.size();
     DMem flagsDev;  // bad-layout flags and the longest read
-    DCHECK(flagsDev.alloc(2 * sizeof(unsigned int)));
+    DCHECK(flagsDev.alloc(2 * sizeof(unsigned int), s));
     DCHECK(cudaMemsetAsync(flagsDev.p, 0, 2 * sizeof(unsigned int), s));
     unsigned int* bad = flagsDev.as<unsigned int>();
     unsigned int* maxLen = bad + 1;
@@ -358,13 +358,13 @@ int correct_fastq_on_device(const cg_options& options, const std::vector<ByteSpa
         const ByteSpan f = inputs[k];
         const bool needNl = f.size == 0 || f.data[f.size - 1] != '\n';
         const uint64_t size = f.size + (needNl ? 1 : 0);
-        DCHECK(fileDev[k].alloc(size));
+        DCHECK(fileDev[k].alloc(size, s));
         if (f.size) DCHECK(cudaMemcpyAsync(fileDev[k].p, f.data, f.size, cudaMemcpyHostToDevice, s));
         if (needNl) DCHECK(cudaMemsetAsync(fileDev[k].as<char>() + f.size, '\n', 1, s));
         const uint64_t blocks = (size + kIdxBlockBytes - 1) / kIdxBlockBytes;
         DMem counts, tmp;
-        DCHECK(counts.alloc((blocks + 1) * sizeof(unsigned long long)));
-        DCHECK(tmp.alloc(scan_tmp_bytes(blocks + 1)));
+        DCHECK(counts.alloc((blocks + 1) * sizeof(unsigned long long), s));
+        DCHECK(tmp.alloc(scan_tmp_bytes(blocks + 1), s));
         DCHECK(cudaMemsetAsync(counts.as<unsigned long long>() + blocks, 0, sizeof(unsigned long long), s));
         nl_count_kernel<<<(unsigned)blocks, kIdxThreads, 0, s>>>(fileDev[k].as<unsigned char>(), size,
                                                                  counts.as<unsigned long long>(), bad);
@@ -378,7 +378,7 @@ int correct_fastq_on_device(const cg_options& options, const std::vector<ByteSpa
         DCHECK(cudaStreamSynchronize(s));
         if (hbad || lines % 4 != 0) return failf(error, CG_ERR_UNSUPPORTED, "input %zu is not plain 4-line FASTQ", k);
         recs[k] = lines / 4;
-        DCHECK(nlDev[k].alloc(lines * sizeof(unsigned long long)));
+        DCHECK(nlDev[k].alloc(lines * sizeof(unsigned long long), s));
         nl_write_kernel<<<(unsigned)blocks, kIdxThreads, 0, s>>>(fileDev[k].as<unsigned char>(), size,
                                                                  counts.as<unsigned long long>(),
                                                                  nlDev[k].as<unsigned long long>());
@@ -400,8 +400,8 @@ int correct_fastq_on_device(const cg_options& options, const std::vector<ByteSpa
     groupStart.push_back(n);
     if (n == 0) return failf(error, CG_ERR_INVALID_ARGUMENT, "input contains no reads");
     DMem readsDev, readOut;
-    DCHECK(readsDev.alloc(n * sizeof(ReadIdx)));
-    DCHECK(readOut.alloc(n));
+    DCHECK(readsDev.alloc(n * sizeof(ReadIdx), s));
+    DCHECK(readOut.alloc(n, s));
     ReadIdx* reads = readsDev.as<ReadIdx>();
     for (size_t k = 0; k < nf; k++) {
         const uint64_t nrec = paired ? n / 2 : recs[k];
@@ -432,16 +432,16 @@ int correct_fastq_on_device(const cg_options& options, const std::vector<ByteSpa
         const uint64_t g0 = groupStart[g], m = groupStart[g + 1] - g0;
         if (m == 0) continue;
         DMem off, tmp, chars, qual;
-        DCHECK(off.alloc((m + 1) * sizeof(unsigned long long)));
-        DCHECK(tmp.alloc(scan_tmp_bytes(m + 1)));
+        DCHECK(off.alloc((m + 1) * sizeof(unsigned long long), s));
+        DCHECK(tmp.alloc(scan_tmp_bytes(m + 1), s));
         lengths_kernel<<<grid_for(m + 1, 256), 256, 0, s>>>(reads + g0, m, off.as<unsigned long long>());
         DCHECK(cudaGetLastError());
         DCHECK(scan_exclusive_u64(off.as<unsigned long long>(), m + 1, tmp.p, s));
         unsigned long long bytes = 0;
         DCHECK(cudaMemcpyAsync(&bytes, off.as<unsigned long long>() + m, sizeof(bytes), cudaMemcpyDeviceToHost, s));
         DCHECK(cudaStreamSynchronize(s));
-        DCHECK(chars.alloc(bytes));
-        if (quals) DCHECK(qual.alloc(bytes));
+        DCHECK(chars.alloc(bytes, s));
+        if (quals) DCHECK(qual.alloc(bytes, s));
         gather_kernel<<<grid_for(m * 32, 256), 256, 0, s>>>(reads + g0, m, off.as<unsigned long long>(),
                                                             chars.as<char>(), quals ? qual.as<char>() : nullptr);
         DCHECK(cudaGetLastError());
@@ -457,22 +457,22 @@ int correct_fastq_on_device(const cg_options& options, const std::vector<ByteSpa
     LCHECK(ctx.c, cg_get_read_info(ctx.c, &nr, &pitch));
     pitch = std::max(pitch, 1);
     DMem flagsOut, seqOut;
-    DCHECK(flagsOut.alloc(n));
-    DCHECK(seqOut.alloc(n * (uint64_t)pitch));
+    DCHECK(flagsOut.alloc(n, s));
+    DCHECK(seqOut.alloc(n * (uint64_t)pitch, s));
 
     // ---- STEP2 and STEP3 per range of reads (one range unless the caller
     // takes the output range by range): correction into device memory, then
     // the range's records of every output file
     DMem mode, status, size, recCount, lastRec, pos, tmp;
-    DCHECK(mode.alloc(n));
-    DCHECK(status.alloc(n));
-    DCHECK(size.alloc(n * sizeof(unsigned long long)));
-    DCHECK(recCount.alloc(sizeof(unsigned long long)));
+    DCHECK(mode.alloc(n, s));
+    DCHECK(status.alloc(n, s));
+    DCHECK(size.alloc(n * sizeof(unsigned long long), s));
+    DCHECK(recCount.alloc(sizeof(unsigned long long), s));
     DCHECK(cudaMemsetAsync(recCount.p, 0, sizeof(unsigned long long), s));
-    DCHECK(lastRec.alloc(sizeof(unsigned int)));
+    DCHECK(lastRec.alloc(sizeof(unsigned int), s));
     DCHECK(cudaMemsetAsync(lastRec.p, 0, sizeof(unsigned int), s));
-    DCHECK(pos.alloc((n + 1) * sizeof(unsigned long long)));
-    DCHECK(tmp.alloc(scan_tmp_bytes(n + 1)));
+    DCHECK(pos.alloc((n + 1) * sizeof(unsigned long long), s));
+    DCHECK(tmp.alloc(scan_tmp_bytes(n + 1), s));
     run->outputs.clear();
     run->outputs.resize((size_t)numOutputs);
     run->outputSizes.assign((size_t)numOutputs, 0);
@@ -517,7 +517,7 @@ int correct_fastq_on_device(const cg_options& options, const std::vector<ByteSpa
                 outDev = static_cast<char*>(raw);
                 run->deviceOutputs[(size_t)f].bytes = raw;  // freed with the run
             } else {
-                DCHECK(outMem.alloc(total));
+                DCHECK(outMem.alloc(total, s));
                 outDev = outMem.as<char>();
             }
             write_kernel<<<grid_for(m * 32, 256), 256, 0, s>>>(reads + r0, m, readOut.as<uint8_t>() + r0, (uint8_t)f,

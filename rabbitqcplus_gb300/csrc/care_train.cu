@@ -111,8 +111,8 @@ void serialize(const std::vector<unsigned char>& blob, void* out) {
 // features (FP32, host) -> BF16 on the device
 int upload_features(const float* features, uint64_t n, Dev& f32, Dev& bf, cudaStream_t s) {
     const uint64_t elems = n * kMlpFeatures;
-    TRY(f32.alloc(elems * sizeof(float)));
-    TRY(bf.alloc(elems * sizeof(__nv_bfloat16)));
+    TRY(f32.alloc(elems * sizeof(float), s));
+    TRY(bf.alloc(elems * sizeof(__nv_bfloat16), s));
     TRY(cudaMemcpyAsync(f32.p, features, elems * sizeof(float), cudaMemcpyHostToDevice, s));
     TRY(launch_to_bf16(f32.as<float>(), elems, bf.as<__nv_bfloat16>(), s));
     return CG_OK;
@@ -171,15 +171,15 @@ int cg_train_classifier(const cg_train_options* o, const float* features, const 
     if (rc != CG_OK) return rc;
     std::vector<float> hl(n);
     for (uint64_t i = 0; i < n; i++) hl[i] = labels[i] ? 1.0f : 0.0f;
-    TRY(lab.alloc(n * sizeof(float)));
+    TRY(lab.alloc(n * sizeof(float), s));
     TRY(cudaMemcpyAsync(lab.p, hl.data(), n * sizeof(float), cudaMemcpyHostToDevice, s));
-    TRY(perm.alloc(n * sizeof(uint32_t)));
-    TRY(model.alloc(kMlpBytes));
+    TRY(perm.alloc(n * sizeof(uint32_t), s));
+    TRY(model.alloc(kMlpBytes, s));
     TRY(cudaMemcpyAsync(model.p, blob.data(), kMlpBytes, cudaMemcpyHostToDevice, s));
     const unsigned parts = mlp_grad_parts((unsigned)B);
-    TRY(part.alloc((size_t)parts * kMlpPartStride * sizeof(float)));
+    TRY(part.alloc((size_t)parts * kMlpPartStride * sizeof(float), s));
     TRY(cudaMemsetAsync(part.p, 0, (size_t)parts * kMlpPartStride * sizeof(float), s));
-    TRY(failed.alloc(sizeof(unsigned long long)));
+    TRY(failed.alloc(sizeof(unsigned long long), s));
     TRY(cudaMemsetAsync(failed.p, 0, sizeof(unsigned long long), s));
     // optimiser state: master weights from the initial model
     auto hs = std::make_unique<MlpAdam>();
@@ -194,14 +194,15 @@ int cg_train_classifier(const cg_train_options* o, const float* features, const 
     hs->beta2Pow = 1.0f;
     hs->lr = o->learning_rate;
     hs->eps = 1e-8f;
-    TRY(adam.alloc(sizeof(MlpAdam)));
+    TRY(adam.alloc(sizeof(MlpAdam), s));
     TRY(cudaMemcpyAsync(adam.p, hs.get(), sizeof(MlpAdam), cudaMemcpyHostToDevice, s));
-    TRY(step.alloc(sizeof(unsigned long long)));
+    TRY(step.alloc(sizeof(unsigned long long), s));
     TRY(cudaMemsetAsync(step.p, 0, sizeof(unsigned long long), s));
-    TRY(loss.alloc(totalSteps * sizeof(float)));
+    TRY(loss.alloc(totalSteps * sizeof(float), s));
     // one training step, captured
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    auto capture = std::make_unique<CaptureScope>();
     TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaError_t e = launch_mlp_grad(model.as<unsigned char>(), bf.as<__nv_bfloat16>(), lab.as<float>(),
                                     perm.as<uint32_t>(), step.as<unsigned long long>(), stepsPerEpoch, (unsigned)B,
@@ -210,6 +211,7 @@ int cg_train_classifier(const cg_train_options* o, const float* features, const 
         e = launch_mlp_reduce(part.as<float>(), parts, nullptr, loss.as<float>(), adam.as<MlpAdam>(),
                               model.as<unsigned char>(), step.as<unsigned long long>(), s);
     const cudaError_t e2 = cudaStreamEndCapture(s, &graph);
+    capture.reset();
     if (e != cudaSuccess || e2 != cudaSuccess) {
         if (graph) cudaGraphDestroy(graph);
         return cuda_status(e != cudaSuccess ? e : e2);
@@ -259,15 +261,15 @@ int cg_classifier_gradients(int device, const void* model_data, size_t model_siz
     if (rc != CG_OK) return rc;
     std::vector<float> hl(n);
     for (uint32_t i = 0; i < n; i++) hl[i] = labels[i] ? 1.0f : 0.0f;
-    TRY(lab.alloc(n * sizeof(float)));
+    TRY(lab.alloc(n * sizeof(float), s));
     TRY(cudaMemcpyAsync(lab.p, hl.data(), n * sizeof(float), cudaMemcpyHostToDevice, s));
-    TRY(model.alloc(kMlpBytes));
+    TRY(model.alloc(kMlpBytes, s));
     TRY(cudaMemcpyAsync(model.p, blob.data(), kMlpBytes, cudaMemcpyHostToDevice, s));
     const unsigned parts = mlp_grad_parts(n);
-    TRY(part.alloc((size_t)parts * kMlpPartStride * sizeof(float)));
+    TRY(part.alloc((size_t)parts * kMlpPartStride * sizeof(float), s));
     TRY(cudaMemsetAsync(part.p, 0, (size_t)parts * kMlpPartStride * sizeof(float), s));
-    TRY(grad.alloc(kMlpParams * sizeof(float)));
-    TRY(failed.alloc(sizeof(unsigned long long)));
+    TRY(grad.alloc(kMlpParams * sizeof(float), s));
+    TRY(failed.alloc(sizeof(unsigned long long), s));
     TRY(cudaMemsetAsync(failed.p, 0, sizeof(unsigned long long), s));
     TRY(launch_mlp_grad(model.as<unsigned char>(), bf.as<__nv_bfloat16>(), lab.as<float>(), nullptr, nullptr, 1, n,
                         1.0f / (float)n, part.as<float>(), failed.as<unsigned long long>(), s));
@@ -295,12 +297,12 @@ int cg_classifier_logits(int device, const void* model_data, size_t model_size, 
     TRY(cudaStreamCreateWithFlags(&st.s, cudaStreamNonBlocking));
     cudaStream_t s = st.s;
     Dev f32, model, out, counters;
-    TRY(f32.alloc(n * kMlpFeatures * sizeof(float)));
+    TRY(f32.alloc(n * kMlpFeatures * sizeof(float), s));
     TRY(cudaMemcpyAsync(f32.p, features, n * kMlpFeatures * sizeof(float), cudaMemcpyHostToDevice, s));
-    TRY(model.alloc(kMlpBytes));
+    TRY(model.alloc(kMlpBytes, s));
     TRY(cudaMemcpyAsync(model.p, blob.data(), kMlpBytes, cudaMemcpyHostToDevice, s));
-    TRY(out.alloc(n * sizeof(float)));
-    TRY(counters.alloc(kNumCounters * sizeof(unsigned long long)));
+    TRY(out.alloc(n * sizeof(float), s));
+    TRY(counters.alloc(kNumCounters * sizeof(unsigned long long), s));
     TRY(cudaMemsetAsync(counters.p, 0, kNumCounters * sizeof(unsigned long long), s));
     int sms = 1;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) sms = 1;

@@ -94,6 +94,7 @@ struct Params {
     float hqMin[101];           // 1 - 3*percent/100
     int significantCount;       // int(int(cov) * 0.3f)
     uint32_t alignPolls;        // polls of an alignment block's wait for its products
+    float alignLift;            // added to the start values of its accumulators (set by launch_align)
     int useQuality;
     int excludeAmbiguous;
     int paired;

@@ -328,7 +328,6 @@ align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ raw
     Sm& sm = *static_cast<Sm*>(__cvta_shared_to_generic(smAt));
     const int tid = (int)threadIdx.x, lane = tid & 31, warp = (int)warp_uniform((uint32_t)tid >> 5);
     const float rate = p.maxErrorRate, slope = fmaxf(1.0f - 2.0f * rate, 0.0f);
-    const bool allPass = rate > 0.5f;
     unsigned int next = 0;  // thread 64: the unit after the one in work
     if (tid == 64) next = atomicAdd(b.unitCursor, 1u);
     if (tid == 0) {
@@ -449,8 +448,7 @@ align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ raw
         // n == 0: the first unit is still to be loaded
         const int n = (int)warp_uniform((uint32_t)sm.unit[u].n), La = (int)warp_uniform((uint32_t)sm.unit[u].len);
         if (tid == 64 && n) next = atomicAdd(b.unitCursor, 1u);  // arrives while this unit is in work
-        // (shifts without overlap have no mismatch limit to stay under: a negative minimum is none)
-        const int minov = max(max(p.minOverlap, (int)__fmul_rn((float)La, p.minOverlapRatio)), 0);
+        const int minov = max(p.minOverlap, (int)__fmul_rn((float)La, p.minOverlapRatio));
         const uint16_t* lens = sm.lens[u];
         const int lcMin = (int)warp_uniform(lens[0]), lcMax = (int)warp_uniform(lens[max(n - 1, 0)]);
         const int right = max(La - minov + 1, 0);  // the reference's shifts 0 .. right - 1, then the left ones
@@ -476,12 +474,11 @@ align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ raw
             }
         };
         // the accumulators' start values for this thread's row, shift sp
-        const float lift = allPass ? 0.25f + (float)La : 0.25f;  // no sum is below -La
         auto start = [&](int sp) {
             const int low = min(minov, La);
             auto value = [&](int lc) {
                 const int ov = sp >= 0 ? min(La - sp, lc) : min(La, lc + sp);
-                return lift - slope * (float)max(ov, min(low, lc));
+                return p.alignLift - slope * (float)max(ov, min(low, lc));
             };
             if (!varies) {
                 tc_fill(acc, value(lcMin), ncol, zero);
@@ -744,6 +741,9 @@ int align_occupancy(StoreArg st) {
 
 cudaError_t launch_align(StoreArg st, Params p, BatchArg b, bool varies, unsigned blocks, cudaStream_t s) {
     if (b.count <= 0 || blocks == 0) return cudaSuccess;
+    // a shift without overlap has no mismatch limit to stay under: a negative minimum is none
+    p.minOverlap = std::max(p.minOverlap, 0);
+    p.alignLift = p.maxErrorRate > 0.5f ? 0.25f + (float)st.lmax : 0.25f;  // no sum is below -lmax
     return with_instance(st, [&](auto k) { return k.launch(st, p, b, varies, blocks, s); });
 }
 

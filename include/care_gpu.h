@@ -184,7 +184,11 @@ void cg_default_options(cg_options* o);
 int cg_create(const cg_options* o, cg_ctx** out);
 
 /* Release the context.  Its device blocks go to a per-process cache that
- * later contexts allocate from; cg_release_cached_memory returns them. */
+ * later contexts allocate from; cg_release_cached_memory returns them.  The
+ * calls that need no context of the caller's (cg_correct_files, cg_train_classifier,
+ * cg_classifier_gradients, cg_classifier_logits) take their device memory from
+ * the same cache and leave up to 1 GiB of their own there, beside the blocks of
+ * the context that cg_correct_files makes. */
 void cg_destroy(cg_ctx* ctx);
 
 /* Free the device blocks cached for reuse on `device` (all devices if < 0);

@@ -38,7 +38,9 @@ namespace {
 // without cudaMalloc and frees without cudaFree.  A block is cached only after
 // the work that uses it has finished (release waits for the device, as cudaFree
 // would; release_after for one stream), and the cache is emptied before an
-// allocation fails.
+// allocation fails.  What release_after gives back -- blocks of calls without a
+// context, which a program does not expect to hold memory afterwards -- is kept up
+// to kKeptBytes per device, and freed beyond that.
 // Simulated device out-of-memory (cg_set_allocation_fault): requests left
 // before every request fails; < 0 = off.
 std::atomic<long long> g_allocFault{-1};
@@ -76,21 +78,21 @@ public:
             // it is at most twice as large and still a live allocation (a
             // cudaDeviceReset of the program's would have released it)
             for (auto it = free_.lower_bound(n); it != free_.end() && it->first <= 2 * n + 4096;) {
-                if (it->second.first != dev) {
+                if (it->second.device != dev) {
                     ++it;
                     continue;
                 }
                 cudaPointerAttributes attr{};
-                const bool live = cudaPointerGetAttributes(&attr, it->second.second) == cudaSuccess &&
+                const bool live = cudaPointerGetAttributes(&attr, it->second.p) == cudaSuccess &&
                                   attr.type == cudaMemoryTypeDevice && attr.device == dev;
                 if (!live) {
                     cudaGetLastError();
-                    it = free_.erase(it);
+                    it = drop(it);
                     continue;
                 }
-                *p = it->second.second;
+                *p = it->second.p;
                 *got = it->first;
-                free_.erase(it);
+                drop(it);
                 return cudaSuccess;
             }
         }
@@ -108,11 +110,11 @@ public:
             std::unique_lock<std::shared_mutex> noCapture(capture_mutex());
             cudaDeviceSynchronize();
         }
-        put(p, bytes);
+        put(p, bytes, false);
     }
     void release_after(void* p, size_t bytes, cudaStream_t s) {
         cudaStreamSynchronize(s);
-        put(p, bytes);
+        if (!put(p, bytes, true)) cudaFree(p);
     }
     // frees the cached blocks of device dev (every device if dev < 0)
     void trim(int dev) {
@@ -120,10 +122,10 @@ public:
         int cur = 0;
         cudaGetDevice(&cur);
         for (auto it = free_.begin(); it != free_.end();) {
-            if (dev < 0 || it->second.first == dev) {
-                cudaSetDevice(it->second.first);
-                cudaFree(it->second.second);
-                it = free_.erase(it);
+            if (dev < 0 || it->second.device == dev) {
+                cudaSetDevice(it->second.device);
+                cudaFree(it->second.p);
+                it = drop(it);
             } else {
                 ++it;
             }
@@ -132,14 +134,30 @@ public:
     }
 
 private:
-    void put(void* p, size_t bytes) {
+    static constexpr size_t kKeptBytes = 1ull << 30;
+    struct Block {
+        int device;
+        void* p;
+        bool counted;  // in kept_
+    };
+    using Blocks = std::multimap<size_t, Block>;
+    // false: counted blocks would exceed kKeptBytes with this one
+    bool put(void* p, size_t bytes, bool counted) {
         int dev = 0;
         cudaGetDevice(&dev);
         std::lock_guard<std::mutex> lock(mu_);
-        free_.emplace(bytes, std::make_pair(dev, p));
+        if (counted && kept_[dev] + bytes > kKeptBytes) return false;
+        if (counted) kept_[dev] += bytes;
+        free_.emplace(bytes, Block{dev, p, counted});
+        return true;
+    }
+    Blocks::iterator drop(Blocks::iterator it) {  // from the list; mu_ is held
+        if (it->second.counted) kept_[it->second.device] -= it->first;
+        return free_.erase(it);
     }
     std::mutex mu_;
-    std::multimap<size_t, std::pair<int, void*>> free_;
+    Blocks free_;
+    std::map<int, size_t> kept_;
 };
 
 BlockCache& block_cache() {

@@ -14,7 +14,8 @@ namespace cg {
 
 // Device memory from the process's block cache (cg_release_cached_memory): at
 // least n bytes, *got of them.  cached_release waits for stream s and keeps the
-// block of the current device for a later request.  It does not wait for the whole
+// block of the current device for a later request, or frees it where enough are
+// kept.  It does not wait for the whole
 // device: that fails, and breaks the capture, while another thread (of this
 // library or of the program) captures one of its streams.
 cudaError_t cached_alloc(void** p, size_t n, size_t* got);

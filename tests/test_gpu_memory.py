@@ -4,7 +4,7 @@ from."""
 import numpy as np
 import pytest
 
-from rabbitqcplus_gb300 import capi, sim
+from rabbitqcplus_gb300 import capi, learned, sim
 
 pytestmark = pytest.mark.gpu
 
@@ -40,3 +40,22 @@ def test_cached_blocks_reused_and_released():
     f3, o3 = correct_once(r)  # fresh allocations again
     assert np.array_equal(f1, f3) and np.array_equal(o1, o3)
     assert lib.cg_release_cached_memory(-1) == capi.CG_OK
+
+
+def test_calls_without_a_context_keep_a_bounded_amount():
+    torch = pytest.importorskip("torch")
+    model = open(learned.DEFAULT_MODEL, "rb").read()
+    small = np.zeros((1000, capi.CLASSIFIER_FEATURES), np.float32)
+    capi.classifier_logits(model, small)  # the kernel is loaded
+    assert capi.gpu_lib().cg_release_cached_memory(-1) == capi.CG_OK
+    free0, _ = torch.cuda.mem_get_info()
+    capi.classifier_logits(model, np.zeros((9_000_000, capi.CLASSIFIER_FEATURES), np.float32))  # 1.07 GiB of rows
+    free1, _ = torch.cuda.mem_get_info()
+    assert free0 - free1 <= 256 << 20  # the rows' block is not kept, the logits' (34 MiB) is
+    for rows in (5_000_000, 4_000_000, 2_000_000):  # 0.6, 0.48 and 0.24 GiB: not all of them fit
+        capi.classifier_logits(model, np.zeros((rows, capi.CLASSIFIER_FEATURES), np.float32))
+    free2, _ = torch.cuda.mem_get_info()
+    assert free0 - free2 <= (1 << 30) + (64 << 20)
+    assert capi.gpu_lib().cg_release_cached_memory(-1) == capi.CG_OK
+    free3, _ = torch.cuda.mem_get_info()
+    assert free3 >= free0 - (64 << 20)

@@ -52,6 +52,11 @@ struct CachedMem {
         if (p) cached_release(p, bytes, stream);
         p = nullptr;
     }
+    void* take() {  // the block is the caller's, to cudaFree
+        void* q = p;
+        p = nullptr;
+        return q;
+    }
     template <class T>
     T* as() const {
         return static_cast<T*>(p);

@@ -507,19 +507,12 @@ int correct_fastq_on_device(const cg_options& options, const std::vector<ByteSpa
                                    s));
             DCHECK(cudaStreamSynchronize(s));
             if (total == 0) continue;
-            // queue chunks outlive this call, on whatever thread and device: their bytes are not cached
             const bool keep = run->queueChunkBytes && !run->onChunk;
             DMem outMem;
-            char* outDev = nullptr;
-            if (keep) {
-                void* raw = nullptr;
-                DCHECK(cudaMalloc(&raw, total));
-                outDev = static_cast<char*>(raw);
-                run->deviceOutputs[(size_t)f].bytes = raw;  // freed with the run
-            } else {
-                DCHECK(outMem.alloc(total, s));
-                outDev = outMem.as<char>();
-            }
+            DCHECK(outMem.alloc(total, s));
+            char* const outDev = outMem.as<char>();
+            // queue chunks outlive this call, on whatever thread and device: their bytes are freed with the run
+            if (keep) run->deviceOutputs[(size_t)f].bytes = outMem.take();
             write_kernel<<<grid_for(m * 32, 256), 256, 0, s>>>(reads + r0, m, readOut.as<uint8_t>() + r0, (uint8_t)f,
                                                                pos.as<unsigned long long>(), mode.as<uint8_t>() + r0,
                                                                status.as<uint8_t>() + r0, sq, pitch,

@@ -152,7 +152,8 @@ typedef struct cg_stats {
     int32_t reserved;
     double seconds_build;             /* device time of the last cg_build_tables */
     double seconds_correct;           /* device time of the last cg_correct */
-    double seconds_candidates;        /* device time in candidate stages (query, unique), accumulated */
+    double seconds_candidates;        /* device time in candidate stages (query, unique), accumulated; of a
+                                       * query beside another batch, what it kept its own waiting */
     double seconds_align;             /* device time in the alignment/filter kernel, accumulated */
     double seconds_msa;               /* device time in the MSA/correction kernel, accumulated */
     uint64_t kernel_launches;         /* kernels this context launched, accumulated */

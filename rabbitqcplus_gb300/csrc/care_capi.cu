@@ -855,16 +855,38 @@ int enqueue_results(cg_ctx* c, int slot, int count, uint8_t* flags, char* out, s
     return CG_OK;
 }
 
-// stage times of the slot's batch, whose results have been copied
-void add_stage_times(cg_ctx* c, int slot) {
+// Time from event a to event b, both passed, added to a statistic.
+int add_time(cg_ctx* c, cudaEvent_t a, cudaEvent_t b, double* seconds) {
+    float ms = 0;
+    CG_CUDA(c, cudaEventElapsedTime(&ms, a, b));
+    *seconds += ms / 1000.0;
+    return CG_OK;
+}
+
+// The time batch j's bucket lookup, which has arrived, kept the batch waiting: the
+// first one's whole, that of a later one from the end of the batch before it, beside
+// which it ran.  (Its time there is mostly its wait for the other kernels.)  Taken
+// here since the slot's events are recorded again before the batch's results are out.
+int add_lookup_time(cg_ctx* c, uint64_t j) {
+    const PlainSlot& sl = c->slots[j & 1];
+    if (j == 0) return add_time(c, sl.q0, sl.q1, &c->stats.seconds_candidates);
+    const cudaEvent_t before = c->slots[(j + 1) & 1].s3;
+    const cudaError_t e = cudaEventQuery(before);
+    if (e == cudaErrorNotReady) return CG_OK;
+    CG_CUDA(c, e);
+    double wait = 0;
+    const int rc = add_time(c, before, sl.q1, &wait);
+    c->stats.seconds_candidates += std::max(wait, 0.0);
+    return rc;
+}
+
+// Stage times of the slot's batch, whose results have been copied.
+int add_stage_times(cg_ctx* c, int slot) {
     const PlainSlot& sl = c->slots[slot];
-    auto ms = [](cudaEvent_t a, cudaEvent_t b) {
-        float t = 0;
-        return cudaEventElapsedTime(&t, a, b) == cudaSuccess ? t / 1000.0 : 0.0;
-    };
-    c->stats.seconds_candidates += ms(sl.q0, sl.q1) + ms(sl.s0, sl.s1);
-    c->stats.seconds_align += ms(sl.s1, sl.s2);
-    c->stats.seconds_msa += ms(sl.s2, sl.s3);
+    int rc = add_time(c, sl.s0, sl.s1, &c->stats.seconds_candidates);
+    if (rc == CG_OK) rc = add_time(c, sl.s1, sl.s2, &c->stats.seconds_align);
+    if (rc == CG_OK) rc = add_time(c, sl.s2, sl.s3, &c->stats.seconds_msa);
+    return rc;
 }
 
 // The counters, read with a call's last results (before the event that ends
@@ -909,9 +931,12 @@ int run_plain_batches(cg_ctx* c, uint64_t first, uint64_t num, int B, uint8_t* f
         }
         if (j > 1) {  // the slot's results of batch j - 2 have left it
             CG_CUDA(c, cudaEventSynchronize(sl.copied));
-            add_stage_times(c, (int)(j & 1));
+            rc = add_stage_times(c, (int)(j & 1));
+            if (rc != CG_OK) return rc;
         }
         CG_CUDA(c, cudaEventSynchronize(sl.q1));
+        rc = add_lookup_time(c, j);
+        if (rc != CG_OK) return rc;
         if (several) CG_CUDA(c, cudaStreamWaitEvent(c->stream, sl.q1, 0));
         rc = enqueue_batch_plain(c, (int)(j & 1), first + at(j), size(j));
         if (rc == CG_OK && j > 0) rc = results(j - 1, cs);
@@ -923,8 +948,8 @@ int run_plain_batches(cg_ctx* c, uint64_t first, uint64_t num, int B, uint8_t* f
     CG_CUDA(c, read_counters(c));
     CG_CUDA(c, cudaEventRecord(c->ev1, c->stream));
     CG_CUDA(c, cudaEventSynchronize(c->ev1));
-    for (uint64_t j = nb < 2 ? 0 : nb - 2; j < nb; j++) add_stage_times(c, (int)(j & 1));
-    return CG_OK;
+    for (uint64_t j = nb < 2 ? 0 : nb - 2; j < nb && rc == CG_OK; j++) rc = add_stage_times(c, (int)(j & 1));
+    return rc;
 }
 
 // After an error nothing of the call is left in flight: the caller's buffers may

@@ -131,15 +131,26 @@ __device__ __forceinline__ ColInfo col_info(const uint2* wc, int cp, int c) {
 // that the anchor errs there.  A column's sum of a base thus receives the
 // reference's additions in the reference's order (anchor, then the kept candidates
 // in list order); sums of different bases are independent.
+// With quality scores, and for reads longer than 320 bp (msa_planes), the rows are
+// added one at a time in shared memory instead, each lane to its columns.
 // Measured, MSA stage: 2M anchors of 150 bp with repeats 12.9 ms (row by row in
 // shared memory 17.2 ms: 116 instructions per row); 60,000 anchors of 300 bp
-// 0.70 ms, 30,000 of 640 bp 1.60 ms, 20,000 of 1000 bp 4.6 ms (a block per anchor,
-// which reads longer than 256 bp used to take, 2.9, 3.1 and 4.2 ms).  It issues in
+// 0.70 ms, 30,000 of 640 bp 1.01 ms, 20,000 of 1000 bp 1.51 ms (a block per anchor,
+// which reads longer than 256 bp used to take, 2.9, 3.1 and 4.3 ms).  It issues in
 // 6 of 10 cycles: a warp's steps depend on one another, and registers and the sums
-// in shared memory leave room for 26 warps per SM (150 bp).
+// in shared memory leave room for 27 one-warp blocks per SM (150 bp; the occupancy
+// query's figure, as those below).
 //
 // `sm` is the warp's own slice of shared memory (MsaSlice), `qw` the block's
 // quality weights.
+
+// Whether a store without quality scores, of reads of up to lp bases (a multiple
+// of 32), adds its rows by planes or one at a time.  A row of many words holds more in
+// registers, and the few warps that its sums leave room for do not hide the steps from
+// word to word.  MSA stage, by planes and one row at a time: 60,000 anchors of 300 bp
+// 0.69 and 0.75 ms, 40,000 of 321 bp 1.00 and 0.62, of 500 bp 1.26 and 0.93, 30,000 of
+// 640 bp 1.64 and 1.01, 20,000 of 1000 bp 4.58 and 1.51.
+__host__ __device__ constexpr bool msa_planes(int lp) { return lp <= 320; }
 
 // Offsets in bytes of one warp's shared memory.  Its first 16 lp bytes hold the
 // weights and counts [4][lp].
@@ -152,7 +163,7 @@ struct MsaSlice {
         weight = stage + (size_t)32 * words * sizeof(uint32_t);  // [32]
         ref = weight + 32 * sizeof(float);                   // planes of the columns' bases [2][wp]
         meta = ref + (size_t)(2 * wp + 3) / 4 * 16;          // [32]: shift, len | orient << 16, weight, id
-        cons = meta + (p.useQuality || p.candidates ? 32 * sizeof(int4) : 0);
+        cons = meta + (p.useQuality || p.candidates || !msa_planes(lp) ? 32 * sizeof(int4) : 0);
         // candidate correction: the consensus codes of Lmax + 2 new_columns_to_correct columns
         const size_t cols = (size_t)lp + 2 * (size_t)p.newColumns;
         bytes = cons + (p.candidates ? (cols + 15) / 16 * 16 + 2 * ((cols + 31) / 32 + 1) * sizeof(uint64_t) : 0);
@@ -224,6 +235,7 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
     constexpr uint8_t kRm = 0x80;
 
     constexpr uint8_t kNew = 0x40;
+    constexpr bool kPlanes = !QUAL && msa_planes(32 * K);
     const int wp = st.wp;
     const uint32_t mine = 0x80000000u >> lane;  // the lane's column in a 32-column word
     const int listMax = 64 * wp;  // entries the staging area holds
@@ -427,11 +439,11 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
         return selected;
     };
 
-    // The same with quality scores: every base has its own weight, so the rows are
-    // added one at a time, with the lanes over the row's columns.  (The other pass
-    // needs a load per row and 32 columns for the matches' qualities as well, and
+    // The same a row at a time, with the lanes over the row's columns: for quality
+    // scores, where every base has its own weight, and for the longest reads
+    // (msa_planes).  (With qualities the other pass needs a load per row and 32 columns for the matches' qualities as well, and
     // then measured 6.5 ms where this one takes 5.5: 300,000 reads of 50 to 250 bp.)
-    auto qualityPass = [&](const bool add) -> int {
+    auto rowPass = [&](const bool add) -> int {
         int selected = 0;
         const uint32_t one = add ? 1u : ~0u;
 #pragma unroll 1
@@ -478,7 +490,9 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
                 const uint32_t flip = rc ? 3u : 0u;
                 // quality of position sp (row_quality; padding past the read's end is
                 // read as stored)
-                const uint8_t* q = st.qual + (uint64_t)(uint32_t)md.w * st.lmax + (rc ? st.lmax - rlen : 0);
+                const uint8_t* q = QUAL ? st.qual + (uint64_t)(uint32_t)md.w * st.lmax + (rc ? st.lmax - rlen : 0)
+                                        : nullptr;
+                auto weightAt = [&](int p) { return QUAL ? __fmul_rn(wr, qw[q[p]]) : wr; };
                 auto baseAt = [&](int w) -> uint32_t {
                     return (((h[w] << up) >> 31) * 2u + ((h[wp + w] << up) >> 31)) ^ flip;
                 };
@@ -492,7 +506,7 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
                 // distinct entries)
                 for (; c + 32 < c1; c += 64, wi += 2 * dwi, sp += 2 * dsp) {
                     const uint32_t b0 = baseAt(wi), b1 = baseAt(wi + dwi);
-                    const float w0 = __fmul_rn(wr, qw[q[sp]]), w1 = __fmul_rn(wr, qw[q[sp + dsp]]);
+                    const float w0 = weightAt(sp), w1 = weightAt(sp + dsp);
                     uint2* p0 = wc + b0 * lp + c;
                     uint2* p1 = wc + b1 * lp + (c + 32);
                     uint2 v0 = *p0, v1 = *p1;
@@ -504,7 +518,7 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
                 if (c < c1) {
                     uint2* p0 = wc + baseAt(wi) * lp + c;
                     uint2 v0 = *p0;
-                    upd(v0, __fmul_rn(wr, qw[q[sp]]));
+                    upd(v0, weightAt(sp));
                     *p0 = v0;
                 }
             }
@@ -519,7 +533,7 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
     auto rowsPass = [&](const bool add) -> int {
         if (add) {
             refBits = anchorBits;
-            if (!QUAL)
+            if (kPlanes)
                 for (int i = lane; i < 2 * wp; i += 32) ref[i] = st.hilo[aid * (2 * (uint64_t)wp) + i];
 #pragma unroll
             for (int k = 0; k < K; k++) {
@@ -530,10 +544,10 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
                 *ref_entry(k) = make_uint2(__float_as_uint(QUAL ? __fmul_rn(1.0f, qw[aq[c]]) : 1.0f), 1u);
             }
         }
-        if constexpr (QUAL)
-            return qualityPass(add);
-        else
+        if constexpr (kPlanes)
             return planePass(add);
+        else
+            return rowPass(add);
     };
 
     // Rounds of refinement.  A round begins with a build, or with the removal of
@@ -983,13 +997,19 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
 // blockIdx.x * warps + warp.  Persistent form (b.work set): warps take the
 // next anchor from the counter b.work[0] until the batch is done.
 // Registers: as many as the K-word arrays need without lowering the number of
-// resident warps, which shared memory bounds: 27 per SM at K = 5, which 72 registers
-// allow (MSA stage 12.9 ms for 2M anchors; 13.7 with 64, which spill, 13.8 with 88),
-// 16 at K = 8 (200,000 anchors of 250 bp 1.67 ms with 112, 1.94 with 80), 9 at K = 16
-// (40,000 of 500 bp 1.24 ms with 224, 1.76 with 128).  256 threads, the most a block
-// has, fit the register file in each case.
+// resident one-warp blocks much, which shared memory bounds: 27 per SM at K = 5 (23
+// with quality scores), 16 at K = 8, 14 at K = 10, 9, 7 and 4 at 16, 20 and 32.  MSA
+// stage: 2M anchors of 150 bp 12.9 ms with 72 (13.7 with 64, which spill, 13.8 with
+// 88), 300,000 with qualities 3.98 with 72 (4.02 with 64, 4.17 with 88); 200,000 of
+// 250 bp 2.57 with 112 (2.99 with 80, 2.49 with 96), 100,000 with qualities 2.22 (2.20
+// with 80, 2.25 with 96, 2.39 with 128); 60,000 of 300 bp 0.69 with 144 (0.71 with
+// 112, 0.75 with 168), with qualities 1.39 with any of them.  At K = 16 and above the
+// rows are added one at a time and need fewer: with qualities, 40,000 of 500 bp 2.08,
+// 30,000 of 640 bp 2.18 and 20,000 of 1000 bp 3.56 with 168 (2.14, 2.23 and 3.67 with
+// 128; 2.12, 2.35 and 3.64 with 224, 255 and 255).  256 threads, the most a block has,
+// fit the register file in each case.
 template <bool QUAL, int K>
-__global__ void __maxnreg__(K > 16 ? 255 : K > 10 ? 224 : K > 8 ? 144 : K > 5 ? 112 : 72)
+__global__ void __maxnreg__(K > 10 ? 168 : K > 8 ? 144 : K > 5 ? 112 : 72)
     msa_warp_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ rawOff, int lp) {
     extern __shared__ __align__(16) unsigned char sm[];
     const int warp = (int)(threadIdx.x >> 5), warps = (int)(blockDim.x >> 5);

@@ -65,6 +65,7 @@ std::shared_mutex& capture_mutex() {
 class BlockCache {
 public:
     cudaError_t alloc(void** p, size_t n, size_t* got) {
+        n = (n + 15) / 16 * 16;  // kernels read the last word of text or rows whole
         int dev = 0;
         cudaGetDevice(&dev);
         if (simulated_out_of_memory()) {

@@ -119,7 +119,8 @@ namespace {
 // Up to 16 characters of a read as a 2-bit word (first character highest, A C G T
 // = 0 1 2 3 in either case) and, per character, whether it is another one
 // (bad, same order, one bit each).  `have` >= 1 characters from p on.  The text is
-// read by aligned words that hold at least one of them.
+// read by aligned words that hold at least one of them: up to three bytes past the
+// text, within its block (blocks are multiples of 16 bytes).
 struct Chars16 {
     uint32_t word, bad;
 };

@@ -28,11 +28,6 @@ __device__ __forceinline__ uint32_t get2bit(const uint32_t* enc, int i) {
     return (enc[i >> 4] >> (30 - 2 * (i & 15))) & 3u;
 }
 
-// base at position p of a candidate read in its aligned orientation
-__device__ __forceinline__ uint32_t oriented_base(const uint32_t* enc, int len, bool rc, int p) {
-    return rc ? 3u - get2bit(enc, len - 1 - p) : get2bit(enc, p);
-}
-
 // reference: include/hostdevicefunctions.cuh:9-28
 __device__ __forceinline__ bool feq(float l, float r) {
     const float d = __fsub_rn(l, r) < 0.0f ? -__fsub_rn(l, r) : __fsub_rn(l, r);

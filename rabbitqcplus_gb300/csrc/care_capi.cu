@@ -250,7 +250,6 @@ struct Plan {
 };
 
 constexpr int kMaxSets = 2;
-constexpr uint32_t kDefaultPolls = 1u << 20;  // of a wait for tensor-core products
 
 // One of the plain driver's two batches in flight: the buffers that outlive
 // the batch's kernels (its bucket ranges are looked up while the batch before
@@ -334,7 +333,7 @@ struct cg_ctx {
     bool haveMlp = false;
     bool collecting = false;  // cg_get_columns: record the columns, do not score them
     float minLogit = 0.0f;    // logit of threshold_anchor
-    uint32_t alignPolls = kDefaultPolls;  // cg_set_alignment_wait_limit
+    uint32_t alignPolls = kWaitPolls;  // cg_set_alignment_wait_limit
     // alignment and classifier blocks whose tensor-core wait ran out, already reported
     unsigned long long alignTimeoutsSeen = 0, timeoutsSeen = 0;
 
@@ -379,7 +378,7 @@ uint64_t pow2_at_least(uint64_t x) {
 
 // polls of a wait as the cg_set_*_wait_limit calls take them
 uint32_t poll_limit(int64_t polls) {
-    return polls < 0 ? kDefaultPolls : (uint32_t)std::min<int64_t>(polls, 0xffffffffll);
+    return polls < 0 ? kWaitPolls : (uint32_t)std::min<int64_t>(polls, 0xffffffffll);
 }
 
 // Float constants in the reference's operand order (host, no contraction).

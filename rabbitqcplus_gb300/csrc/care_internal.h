@@ -42,6 +42,7 @@ constexpr int align_words(int lmax) {
 }
 constexpr int align_plane_words(int w) { return (w + 2) / 2 * 2; }
 constexpr int kAlignUnit = 64;
+constexpr uint32_t kWaitPolls = 1u << 20;  // polls of a wait for tensor-core products before it is declared failed
 
 struct Slot {
     unsigned long long key;

@@ -146,7 +146,6 @@ __device__ void filter_anchor(const StoreArg& st, const Params& p, const BatchAr
 constexpr int kAlignThreads = 128;         // a thread per TMEM lane
 constexpr uint32_t kAlignTmemCols = kAlignUnit;  // a column per candidate of a unit
 constexpr int kAlignQueue = 256;
-constexpr uint32_t kAlignSpins = 1u << 20;  // polls of the wait that drains a failed block's products
 constexpr uint32_t kOnes = 0x38383838u;    // four e4m3 +1 (the sign bit makes -1)
 
 // `keep` most significant bits (any keep: all from 32 up, none from 0 down)
@@ -295,7 +294,7 @@ constexpr int align_blocks_per_sm(int w) { return w <= 5 ? 8 : w <= 8 ? 6 : w <=
 // 32 columns, one instruction per element.  With a limit above half the overlap that
 // sum is negative and the test could rule out next to nothing: every shift passes to
 // the exact count.  (60,000 anchors of 150 bp, whole call: 1.2 ms with limits to 0.3,
-// 2.0 at 0.4, 3.4 at 0.45, 6.6 at 0.5, 8.7 at 0.7; the scan of every shift 1.9, 3.6, 3.7,
+// 2.1 at 0.4, 3.7 at 0.45, 7.1 at 0.5, 8.9 at 0.7; the scan of every shift 1.9, 3.6, 3.7,
 // 3.8 and 3.6.)
 //
 // With several read lengths the columns are in order of length, and the start
@@ -305,7 +304,7 @@ constexpr int align_blocks_per_sm(int w) { return w <= 5 ? 8 : w <= 8 ? 6 : w <=
 // The shifts that pass are queued and counted exactly: mismatches of both planes
 // over the overlap, the reference's limit and score, and the first smallest
 // score per candidate and orientation by an atomic minimum over (score, scan
-// position); the count of a shift ends where it can no longer win.  Then warps 0 and 1 choose the orientations and filter (an anchor of
+// position); a shift that can no longer win is not counted.  Then warps 0 and 1 choose the orientations and filter (an anchor of
 // several units: warp 0 of the last of them to finish) while warps 2 and 3 load
 // the next unit, whose chain of dependent loads would otherwise be the longest
 // part of a unit.
@@ -318,7 +317,10 @@ constexpr int align_blocks_per_sm(int w) { return w <= 5 ? 8 : w <= 8 ? 6 : w <=
 // products (about 7,800 warp instructions a unit, a quarter of them signs and start
 // values) and by waiting for the products in between.  The same test with mma.sync took 61 ms: e4m3 operands are unpacked to
 // FP16 there, at a quarter of this rate.
-template <int W>
+//
+// Limited: the waits end after p.alignPolls polls instead of kWaitPolls (an instance of
+// its own, since a limit that may be zero costs 0.5% of the time).
+template <int W, bool Limited>
 __global__ void __launch_bounds__(kAlignThreads, align_blocks_per_sm(W))
 align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ rawOff, int varies) {
     using Sm = AlignBlock<W>;
@@ -491,6 +493,9 @@ align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ raw
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         };
         // the exact count of the queued shifts
+        // unrolled where registers are to spare: 75 bp 3%, 640 and 1000 bp 1% of the
+        // alignment (150 to 300 bp lose up to 1% with it)
+        constexpr int kCountUnroll = W <= 4 || W > 10 ? 4 : 1;
         auto count = [&](int entries) {
             for (int e0 = tid; e0 < entries; e0 += kAlignThreads) {
                 uint4 e = sm.queue[e0];  // columns 0-31, columns 32-63 (first column highest), shift, orientation
@@ -517,7 +522,8 @@ align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ raw
                     const uint32_t* ot = sp >= 0 ? sm.planes[c] : ap;
                     uint32_t ch = sh[0], cl = sh[Sm::kPlane];
                     int m = 0;
-                    for (int i = 0; i < parts && m < out; i++) {
+#pragma unroll kCountUnroll
+                    for (int i = 0; i < parts; i++) {
                         const uint32_t nh = sh[i + 1], nl = sh[Sm::kPlane + i + 1];
                         const uint32_t x = (__funnelshift_l(nh, ch, bs) ^ ot[i]) |
                                            (__funnelshift_l(nl, cl, bs) ^ ot[Sm::kPlane + i]);
@@ -571,7 +577,7 @@ align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ raw
             }
             if (warp >= 2 && steps < 4) step();
             bool ok = true;
-            if (warp == 0) ok = mbar_wait(mb, phase, p.alignPolls);  // the other warps wait at the barrier
+            if (warp == 0) ok = mbar_wait(mb, phase, Limited ? p.alignPolls : kWaitPolls);  // the other warps wait at the barrier
             phase ^= 1u;
             if (__syncthreads_or(!ok)) {
                 failed = true;
@@ -695,7 +701,7 @@ align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ raw
     }
     if (failed) {
         if (tid == 0) atomicAdd(&b.counters[kCounterAlignTimeouts], 1ull);
-        mbar_wait(mb, phase ^ 1u, kAlignSpins);  // the products in flight, bounded again
+        mbar_wait(mb, phase ^ 1u, kWaitPolls);  // the products in flight, bounded again
     }
     tc_fence_before();
     __syncthreads();
@@ -707,15 +713,13 @@ align_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ raw
 
 template <int W>
 struct AlignInstance {
-    static cudaError_t prepare() {
-        return cudaFuncSetAttribute(align_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)sizeof(AlignBlock<W>));
-    }
     static cudaError_t launch(StoreArg st, const Params& p, const BatchArg& b, bool varies, unsigned blocks,
                               cudaStream_t s) {
-        const cudaError_t e = prepare();
+        const auto kernel = p.alignPolls == kWaitPolls ? align_kernel<W, false> : align_kernel<W, true>;
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)sizeof(AlignBlock<W>));
         if (e != cudaSuccess) return e;
-        align_kernel<W><<<blocks, kAlignThreads, sizeof(AlignBlock<W>), s>>>(st, p, b, b.rawCount, varies);
+        kernel<<<blocks, kAlignThreads, sizeof(AlignBlock<W>), s>>>(st, p, b, b.rawCount, varies);
         return cudaGetLastError();
     }
     static int occupancy() {

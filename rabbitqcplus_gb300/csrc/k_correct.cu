@@ -144,26 +144,28 @@ __device__ __forceinline__ ColInfo col_info(const uint2* wc, int cp, int c) {
 // `sm` is the warp's own slice of shared memory (MsaSlice), `qw` the block's
 // quality weights.
 
-// Whether a store without quality scores, of reads of up to lp bases (a multiple
-// of 32), adds its rows by planes or one at a time.  A row of many words holds more in
-// registers, and the few warps that its sums leave room for do not hide the steps from
-// word to word.  MSA stage, by planes and one row at a time: 60,000 anchors of 300 bp
-// 0.69 and 0.75 ms, 40,000 of 321 bp 1.00 and 0.62, of 500 bp 1.26 and 0.93, 30,000 of
-// 640 bp 1.64 and 1.01, 20,000 of 1000 bp 4.58 and 1.51.
-__host__ __device__ constexpr bool msa_planes(int lp) { return lp <= 320; }
+// Whether a store of reads of up to lp bases (a multiple of 32) adds its rows by
+// planes or one at a time.  With quality scores every base has its own weight: see
+// rowPass.  Without them, a row of many words holds more in registers, and the few
+// warps that its sums leave room for do not hide the steps from word to word.  MSA
+// stage, by planes and one row at a time: 60,000 anchors of 300 bp 0.70 and 0.75 ms,
+// 40,000 of 321 bp 1.00 and 0.62, of 500 bp 1.26 and 0.93, 30,000 of 640 bp 1.64 and
+// 1.01, 20,000 of 1000 bp 4.58 and 1.50.
+__host__ __device__ constexpr bool msa_planes(bool quality, int lp) { return !quality && lp <= 320; }
 
 // Offsets in bytes of one warp's shared memory.  Its first 16 lp bytes hold the
 // weights and counts [4][lp].
 struct MsaSlice {
     size_t sup, stage, weight, ref, meta, cons, bytes;
-    __host__ __device__ MsaSlice(int lp, int pitch, int wp, const Params& p) {
+    // rows: the rows are added one at a time
+    __host__ __device__ MsaSlice(int lp, int pitch, int wp, const Params& p, bool rows) {
         const int words = pitch > 2 * wp ? pitch : 2 * wp;
         sup = (size_t)lp * 4 * sizeof(uint2);
         stage = sup + (size_t)lp * sizeof(float);           // 32 rows' planes or 2-bit words; the mismatch list
         weight = stage + (size_t)32 * words * sizeof(uint32_t);  // [32]
         ref = weight + 32 * sizeof(float);                   // planes of the columns' bases [2][wp]
         meta = ref + (size_t)(2 * wp + 3) / 4 * 16;          // [32]: shift, len | orient << 16, weight, id
-        cons = meta + (p.useQuality || p.candidates || !msa_planes(lp) ? 32 * sizeof(int4) : 0);
+        cons = meta + (rows || p.candidates ? 32 * sizeof(int4) : 0);
         // candidate correction: the consensus codes of Lmax + 2 new_columns_to_correct columns
         const size_t cols = (size_t)lp + 2 * (size_t)p.newColumns;
         bytes = cons + (p.candidates ? (cols + 15) / 16 * 16 + 2 * ((cols + 31) / 32 + 1) * sizeof(uint64_t) : 0);
@@ -235,7 +237,7 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
     constexpr uint8_t kRm = 0x80;
 
     constexpr uint8_t kNew = 0x40;
-    constexpr bool kPlanes = !QUAL && msa_planes(32 * K);
+    constexpr bool kPlanes = msa_planes(QUAL, 32 * K);
     const int wp = st.wp;
     const uint32_t mine = 0x80000000u >> lane;  // the lane's column in a 32-column word
     const int listMax = 64 * wp;  // entries the staging area holds
@@ -1002,18 +1004,19 @@ __device__ __forceinline__ void msa_warp_anchor(const StoreArg& st, const Params
 // stage: 2M anchors of 150 bp 12.9 ms with 72 (13.7 with 64, which spill, 13.8 with
 // 88), 300,000 with qualities 3.98 with 72 (4.02 with 64, 4.17 with 88); 200,000 of
 // 250 bp 2.57 with 112 (2.99 with 80, 2.49 with 96), 100,000 with qualities 2.22 (2.20
-// with 80, 2.25 with 96, 2.39 with 128); 60,000 of 300 bp 0.69 with 144 (0.71 with
-// 112, 0.75 with 168), with qualities 1.39 with any of them.  At K = 16 and above the
+// with 80, 2.25 with 96, 2.39 with 128); 60,000 of 300 bp 0.70 with 128 (0.71 with
+// 112; 0.75 with 144 and 168, which leave room for 12 blocks), with qualities 1.39 with
+// any of them.  At K = 16 and above the
 // rows are added one at a time and need fewer: with qualities, 40,000 of 500 bp 2.08,
 // 30,000 of 640 bp 2.18 and 20,000 of 1000 bp 3.56 with 168 (2.14, 2.23 and 3.67 with
 // 128; 2.12, 2.35 and 3.64 with 224, 255 and 255).  256 threads, the most a block has,
 // fit the register file in each case.
 template <bool QUAL, int K>
-__global__ void __maxnreg__(K > 10 ? 168 : K > 8 ? 144 : K > 5 ? 112 : 72)
+__global__ void __maxnreg__(K > 10 ? 168 : K > 8 ? 128 : K > 5 ? 112 : 72)
     msa_warp_kernel(StoreArg st, Params p, BatchArg b, const uint32_t* __restrict__ rawOff, int lp) {
     extern __shared__ __align__(16) unsigned char sm[];
     const int warp = (int)(threadIdx.x >> 5), warps = (int)(blockDim.x >> 5);
-    const MsaSlice sl(lp, st.pitch, st.wp, p);
+    const MsaSlice sl(lp, st.pitch, st.wp, p, !msa_planes(QUAL, 32 * K));
     // The slice's address is kept in a register: left to itself the compiler builds
     // a shared address from the block's number in its cluster for every access.
     uint32_t at = (uint32_t)__cvta_generic_to_shared(sm + (QUAL ? 256 * sizeof(float) : 0) + (size_t)warp * sl.bytes);
@@ -1103,7 +1106,7 @@ struct MsaInstance {
 template <int K>
 MsaInstance msa_instance_of(StoreArg st, const Params& p) {
     return {p.useQuality ? msa_warp_kernel<true, K> : msa_warp_kernel<false, K>,
-            MsaSlice((st.lmax + 31) / 32 * 32, st.pitch, st.wp, p).bytes};
+            MsaSlice((st.lmax + 31) / 32 * 32, st.pitch, st.wp, p, !msa_planes(p.useQuality, 32 * K)).bytes};
 }
 MsaInstance msa_instance(StoreArg st, const Params& p) {
     const int words = (st.lmax + 31) / 32;

@@ -49,13 +49,12 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 
 constexpr int kTcRows = 128;
 constexpr uint32_t kTmemCols = 128;
-constexpr uint32_t kWaitSpins = 1u << 20;  // mbarrier polls before a wait is declared failed
 
 // Polls of the per-tile MMA waits (the waits whose failure ends a block);
 // set from the host by set_classifier_wait_limit.  The wait that drains a
 // failed block's MMAs before its tensor memory is released always uses
-// kWaitSpins.
-__device__ uint32_t g_tileWaitSpins = kWaitSpins;
+// kWaitPolls.
+__device__ uint32_t g_tileWaitSpins = kWaitPolls;
 
 // 32 consecutive FP32 accumulator columns of this thread's TMEM lane
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
@@ -242,7 +241,7 @@ __global__ void __launch_bounds__(kTcRows) mlp_infer_kernel(const unsigned char*
     }
     if (failed) {
         if (tid == 0 && counters) atomicAdd(&counters[kCounterTimeouts], 1ull);
-        mbar_wait(mb, phase ^ 1u, kWaitSpins);  // the MMAs in flight, bounded again at the full limit
+        mbar_wait(mb, phase ^ 1u, kWaitPolls);  // the MMAs in flight, bounded again at the full limit
     }
     __syncthreads();
     tc_fence_after();
@@ -398,7 +397,7 @@ __global__ void __launch_bounds__(kTrainRows, 1) mlp_grad_kernel(const unsigned 
     uint32_t phase = 0;
     bool ok = true;
     auto wait_mma = [&]() {
-        if (!mbar_wait(mb, phase, kWaitSpins)) ok = false;
+        if (!mbar_wait(mb, phase, kWaitPolls)) ok = false;
         phase ^= 1u;
         ok = !__syncthreads_or(!ok);
         tc_fence_after();
@@ -596,7 +595,7 @@ __global__ void __launch_bounds__(kTrainRows, 1) mlp_grad_kernel(const unsigned 
     } else {
         for (int i = tid; i < kMlpParams; i += kTrainRows) out[i] = 0.0f;
         if (tid == 0 && failed) atomicAdd(failed, 1ull);
-        mbar_wait(mb, phase ^ 1u, kWaitSpins);  // the MMAs in flight, bounded again
+        mbar_wait(mb, phase ^ 1u, kWaitPolls);  // the MMAs in flight, bounded again
     }
     __syncthreads();
     tc_fence_after();

@@ -72,16 +72,16 @@ WINDOW = 4_194_304  # anchors per step
 # DRAM bytes (read + write) of align_kernel per candidate, its warp instructions
 # per candidate and the pipes' activity, measured by ncu on one 65536-anchor
 # launch of the 100M-read workload's shape at 20 Mbp
-# (profiles/top_kernels_c4_shape_20mbp.md: 474.4 MB and 5.58698e8 warp
-# instructions for the launch's 3.3555M candidates, issue 64.4%, ALU pipe 54.6%,
-# tensor pipe 18.2% active).  On the 2M-read workload with repeats the DRAM
+# (profiles/top_kernels_c4_shape_20mbp.md: 475.6 MB and 5.56510e8 warp
+# instructions for the launch's 3.3555M candidates, issue 64.8%, ALU pipe 54.3%,
+# tensor pipe 18.4% active).  On the 2M-read workload with repeats the DRAM
 # bytes per candidate are far fewer (candidates shared by the anchors of a
 # batch hit in L2 there).
-ALIGN_DRAM_BYTES_PER_CANDIDATE = 474.4e6 / 3.3555e6
-ALIGN_WARP_INST_PER_CANDIDATE = 5.58698e8 / 3.3555e6
-ALIGN_ISSUE_ACTIVE = 0.644
-ALIGN_ALU_PIPE_ACTIVE = 0.546
-ALIGN_TENSOR_PIPE_ACTIVE = 0.182
+ALIGN_DRAM_BYTES_PER_CANDIDATE = 475.6e6 / 3.3555e6
+ALIGN_WARP_INST_PER_CANDIDATE = 5.56510e8 / 3.3555e6
+ALIGN_ISSUE_ACTIVE = 0.648
+ALIGN_ALU_PIPE_ACTIVE = 0.543
+ALIGN_TENSOR_PIPE_ACTIVE = 0.184
 # STEP2 speed of the oracle (the port) over the reference's own build, both on
 # 8 threads of an Intel Xeon @ 2.70 GHz, 2M-read 150 bp workload with repeats,
 # outputs byte-identical (python oracle/port_speed.py --threads 8): the port

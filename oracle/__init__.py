@@ -119,8 +119,8 @@ class Oracle:
 
     def check_orientation_shortcut(self, first: int, count: int, threads: int | None = None) -> dict:
         """(candidate, orientation scanned first) cases of anchors [first,
-        first + count), how many the device alignment's one-plane shortcut
-        decides, and how many of those the reference's rule decides otherwise
+        first + count), how many a one-plane shortcut, which no device kernel
+        takes, decides, and how many of those the reference's rule decides otherwise
         (oracle/care_oracle.cpp: orc_check_orientation_shortcut)."""
         out = np.zeros(3, dtype=np.uint64)
         assert self._L.orc_check_orientation_shortcut(self._h, first, count, threads or self.threads,

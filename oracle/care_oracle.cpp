@@ -1053,9 +1053,10 @@ int orc_candidates(void* h, uint64_t anchor, uint32_t* out, uint32_t cap, uint32
     return 0;
 }
 
-// Check of the device alignment's orientation shortcut (not part of the
-// reference: the GPU kernel align_lane_kernel scans one orientation first and
-// skips the other where a one-plane test rules out a tie).  For every
+// Check of a property of the orientation rule (not part of the reference, and
+// no device kernel relies on it: an earlier alignment kernel scanned one
+// orientation first and skipped the other where a one-plane test ruled out a
+// tie).  For every
 // candidate of the anchors [first, first + count) and for each orientation
 // taken as the one scanned first: the shortcut decides when that
 // orientation's result would be chosen on its own (choose it against an

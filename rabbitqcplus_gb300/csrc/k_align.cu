@@ -269,8 +269,8 @@ struct AlignBlock {
 
 // Blocks per SM: at most 8 (512 tensor-memory columns), as many as the shared
 // memory holds.  An instance for 640 bp gives those reads three blocks where the one
-// for 1024 has two: alignment of 30,000 anchors of 640 bp 2.47 ms, 6.05 with one block
-// of the largest instance; 20,000 of 1000 bp 4.05 ms with two, 7.37 with one; 60,000 of
+// for 1024 has two: alignment of 30,000 anchors of 640 bp 2.50 ms, 6.05 with one block
+// of the largest instance; 20,000 of 1000 bp 4.03 ms with two, 7.37 with one; 60,000 of
 // 300 bp 1.42 ms with five, 1.63 with four.
 constexpr int align_blocks_per_sm(int w) { return w <= 5 ? 8 : w <= 8 ? 6 : w <= 10 ? 5 : w <= 20 ? 3 : 2; }
 
@@ -310,13 +310,13 @@ constexpr int align_blocks_per_sm(int w) { return w <= 5 ? 8 : w <= 8 ? 6 : w <=
 // part of a unit.
 //
 // Measured, alignment and filter of 2M anchors of 150 bp (105M candidates, 10 Mbp
-// genome with repeats): 22.5 ms; the scan of every shift by XOR and popcount that
+// genome with repeats): 22.1 ms; the scan of every shift by XOR and popcount that
 // this replaces, 33.2 ms with its filter kernel (integer pipe 85% busy, popcounts at
-// a quarter of its rate).  60k anchors of 300 bp: 1.4 ms against 16.1.  Issue is 68%
+// a quarter of its rate).  60k anchors of 300 bp: 1.4 ms against 16.1.  Issue is 65%
 // busy, the tensor pipe 18%: what is left is bound by the instructions around the
 // products (about 7,800 warp instructions a unit, a quarter of them signs and start
-// values) and by waiting for the products in between.  The same test with mma.sync took 61 ms: e4m3 operands are unpacked to
-// FP16 there, at a quarter of this rate.
+// values) and by waiting for the products in between.  The same test with mma.sync
+// took 61 ms: e4m3 operands are unpacked to FP16 there, at a quarter of this rate.
 //
 // Limited: the waits end after p.alignPolls polls instead of kWaitPolls (an instance of
 // its own, since a limit that may be zero costs 0.5% of the time).

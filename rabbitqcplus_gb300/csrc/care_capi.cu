@@ -40,7 +40,7 @@ namespace {
 // would; release_after for one stream), and the cache is emptied before an
 // allocation fails.  What release_after gives back -- blocks of calls without a
 // context, which a program does not expect to hold memory afterwards -- is kept up
-// to kKeptBytes per device, and freed beyond that.
+// to kKeptBytes per device; beyond that the ones given back first are freed.
 // Simulated device out-of-memory (cg_set_allocation_fault): requests left
 // before every request fails; < 0 = off.
 std::atomic<long long> g_allocFault{-1};
@@ -115,7 +115,7 @@ public:
     }
     void release_after(void* p, size_t bytes, cudaStream_t s) {
         cudaStreamSynchronize(s);
-        if (!put(p, bytes, true)) cudaFree(p);
+        put(p, bytes, true);
     }
     // frees the cached blocks of device dev (every device if dev < 0)
     void trim(int dev) {
@@ -140,17 +140,29 @@ private:
         int device;
         void* p;
         bool counted;  // in kept_
+        uint64_t order;
     };
     using Blocks = std::multimap<size_t, Block>;
-    // false: counted blocks would exceed kKeptBytes with this one
-    bool put(void* p, size_t bytes, bool counted) {
+    void put(void* p, size_t bytes, bool counted) {
         int dev = 0;
         cudaGetDevice(&dev);
         std::lock_guard<std::mutex> lock(mu_);
-        if (counted && kept_[dev] + bytes > kKeptBytes) return false;
+        if (counted && bytes > kKeptBytes) {
+            cudaFree(p);
+            return;
+        }
+        while (counted && kept_[dev] + bytes > kKeptBytes) {
+            auto oldest = free_.end();
+            for (auto it = free_.begin(); it != free_.end(); ++it)
+                if (it->second.counted && it->second.device == dev &&
+                    (oldest == free_.end() || it->second.order < oldest->second.order))
+                    oldest = it;
+            if (oldest == free_.end()) break;
+            cudaFree(oldest->second.p);
+            drop(oldest);
+        }
         if (counted) kept_[dev] += bytes;
-        free_.emplace(bytes, Block{dev, p, counted});
-        return true;
+        free_.emplace(bytes, Block{dev, p, counted, order_++});
     }
     Blocks::iterator drop(Blocks::iterator it) {  // from the list; mu_ is held
         if (it->second.counted) kept_[it->second.device] -= it->first;
@@ -159,6 +171,7 @@ private:
     std::mutex mu_;
     Blocks free_;
     std::map<int, size_t> kept_;
+    uint64_t order_ = 0;
 };
 
 BlockCache& block_cache() {

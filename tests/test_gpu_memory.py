@@ -59,3 +59,16 @@ def test_calls_without_a_context_keep_a_bounded_amount():
     assert capi.gpu_lib().cg_release_cached_memory(-1) == capi.CG_OK
     free3, _ = torch.cuda.mem_get_info()
     assert free3 >= free0 - (64 << 20)
+
+
+def test_the_last_call_s_blocks_are_the_ones_kept():
+    torch = pytest.importorskip("torch")
+    model = open(learned.DEFAULT_MODEL, "rb").read()
+    capi.classifier_logits(model, np.zeros((1000, capi.CLASSIFIER_FEATURES), np.float32))
+    assert capi.gpu_lib().cg_release_cached_memory(-1) == capi.CG_OK
+    free0, _ = torch.cuda.mem_get_info()
+    for rows in (7_500_000, 2_000_000):  # 0.89 and 0.24 GiB: together above the bound
+        capi.classifier_logits(model, np.zeros((rows, capi.CLASSIFIER_FEATURES), np.float32))
+    free1, _ = torch.cuda.mem_get_info()
+    assert 200 << 20 <= free0 - free1 <= 512 << 20  # the second call's, not the first's
+    assert capi.gpu_lib().cg_release_cached_memory(-1) == capi.CG_OK
